@@ -1,7 +1,7 @@
 // Device-side state layout and kernel launchers of the SPH step engine.
 //
 // Layout in HBM (one scene, capacity N, stride Np = N rounded up to 32):
-//   pos   R4 {x,y,z,-}      integrated positions, permuted by the cell sort
+//   pos   R4 {x,y,z,key}    integrated positions with the bits of their bucket key, permuted by the cell sort
 //   vel   R4 {vx,vy,vz,m}   velocity with the particle mass in w
 //   xv    R4 {x,y,z,V}      sorted positions with the current volume in w
 //   acc   R4 {ax,ay,az,-}   total acceleration
@@ -12,7 +12,7 @@
 //                           `i/32` keeps neighbors 4g..4g+3 in one 8-byte
 //                           group; self is implicit, not stored
 //   halo  u32 [blocks][hcap] particle indices of each block's halo (the union
-//                           of its cells' stencil buckets), ascending
+//                           of its cells' stencil buckets), cell by cell
 //   ncnt  u32 [N]           neighbor counts
 //   bW, bG, bGu             per-particle boundary aggregates (see kernels)
 //   IISPH scratch: vstar R4, s R, aii R, accp R4, p R
@@ -69,6 +69,7 @@ struct StepParams {
   KernelConst<R> k;
   double range;          // kernel support radius (search range and cell size)
   R range2_lo, range2_hi;
+  R range2_out;          // range^2 widened past range2_hi and the rounding of a squared distance
   double spacing;        // rest density grid spacing
   R V0;                  // rest volume spacing^3
   R visc_f, visc_b;      // 10 * viscosity (= nu * 2 * (3 + 2))
@@ -87,7 +88,6 @@ struct StepParams {
   R omega, min_diag;
   double tde;            // IISPH target density error (%)
   int iteration_cap;     // 0 = unbounded (reference)
-  int sorted_lists;      // 1: neighbor lists in ascending index order
 };
 
 // Rigid body state, f64 (rigid_body_motion.rs:22-36).

@@ -25,6 +25,7 @@
 
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 
 #include "sph_engine.cuh"
 
@@ -122,17 +123,15 @@ __global__ void __launch_bounds__(kBlock) k_integrate_key(
       const R4<R> a = acc[i];
       v.x = v.x + dt * a.x; v.y = v.y + dt * a.y; v.z = v.z + dt * a.z;
       x.x = x.x + dt * v.x; x.y = x.y + dt * v.y; x.z = x.z + dt * v.z;
-      pos[i] = x;
       vel[i] = v;
     } else if (mode == 1) {
       const R m = v.w;
       x = xint[i];
       v = vint[i];
       v.w = m;
-      pos[i] = x;
       vel[i] = v;
     }
-    uint32_t k;
+    uint32_t k;  // also kept in the position's spare lane, which the sort carries along
     if ((double)x.z < P.disable_below) {
       k = P.T;
       atomicAdd(&sc->n_below, 1);
@@ -142,6 +141,8 @@ __global__ void __launch_bounds__(kBlock) k_integrate_key(
       const double vx = v.x, vy = v.y, vz = v.z;
       speed = sqrt((vx * vx + vy * vy) + vz * vz);
     }
+    x.w = key_lane<R>(k);
+    pos[i] = x;
     key[i] = k;
     slot[i] = atomicAdd(&count[k], 1u);
   }
@@ -387,8 +388,8 @@ __global__ void __launch_bounds__(kBlock) k_gather_samples(
 // The particles of one block (kBlock consecutive particles in bucket order)
 // find their neighbors in the union of the 27-bucket stencils of their
 // cells: the block's halo. Because buckets are contiguous in memory and the
-// halo is kept in ascending bucket key order, the halo is a short list of
-// runs of consecutive particle indices (halo_idx, ascending). Neighbor lists
+// halo is kept cell by cell, rows of cells along x one after the other, the
+// halo is a short list of runs of consecutive particle indices (halo_idx). Neighbor lists
 // hold 16-bit positions in the block's halo. The passes over neighbors copy
 // the halo's records into shared memory once per launch (ordered loads of
 // those runs) and gather from there; a block whose halo does not fit the
@@ -402,11 +403,6 @@ __device__ __forceinline__ size_t nbr_slot(int i, int k, int K) {
   const size_t t = (size_t)(i >> 5), lane = (size_t)(i & 31);
   return ((t * (size_t)(K >> 2) + (size_t)(k >> 2)) * 32 + lane) * 4 + (size_t)(k & 3);
 }
-
-constexpr int kHaloKeys = 8192;            // >= 27 * kBlock stencil keys, a power of two
-static_assert(kHaloKeys >= 27 * kBlock, "the sort buffer must hold the stencil keys of a full block");
-constexpr uint32_t kNoKey = 0xffffffffu;
-constexpr size_t kSearchSmem = kHaloKeys * (sizeof(uint32_t) + sizeof(uint16_t));
 
 // Neighbor lists of one step and the block halos they index.
 struct NbrArgs {
@@ -565,170 +561,446 @@ __device__ __forceinline__ void kahan_add(R& s, R& c, R t) {
   s = u;
 }
 
-// The 27 stencil bucket keys of cell (cx,cy,cz), ascending (= memory order)
-// when `sorted`, else in stencil order.
-__device__ __forceinline__ void stencil_keys(int cx, int cy, int cz, uint32_t mask, int sorted, uint32_t keys[27]) {
+// The 27 stencil bucket keys of cell (cx,cy,cz) in stencil order.
+__device__ __forceinline__ void stencil_keys(int cx, int cy, int cz, uint32_t mask, uint32_t keys[27]) {
 #pragma unroll
   for (int q = 0; q < 27; ++q) keys[q] = morton_key(cx + (q % 3) - 1, cy + (q / 3) % 3 - 1, cz + q / 9 - 1, mask);
-  if (sorted) {
+}
+
+// Shared memory of the neighbor search. Region X holds the halo's positions
+// (x, y and z each in an array of its own, so that a 16-byte load brings one
+// coordinate of four f32 candidates), region L the lists under construction
+// (entry k of thread t at [k * kBlock + t]) and, before them, the halo's
+// construction; region W the candidate runs of the block's cells. Four blocks
+// share an SM.
+constexpr size_t kSearchX = 24576;       // 2048 f32 / 1024 f64 positions
+constexpr int kListStage = 48;           // list entries per particle kept in shared memory
+constexpr size_t kSearchL = (size_t)kListStage * kBlock * sizeof(uint16_t);
+constexpr int kSearchCells = 184;        // cells of a block whose candidates are kept as runs
+constexpr size_t kSearchW = (size_t)9 * kSearchCells * sizeof(uint32_t);
+constexpr size_t kSearchSmem = kSearchX + kSearchL + kSearchW;
+constexpr int kBoxCells = 16384;         // cells of the block's bounding boxes (one bit each)
+constexpr int kBoxLevel = 12;            // key bit from which a block's cells get two boxes (16^3 cells)
+constexpr int kHaloCells = 3064;         // distinct halo cells
+constexpr int kHaloKeys = 8192;          // general path: >= 27 * kBlock stencil keys, a power of two
+constexpr uint32_t kNoKey = 0xffffffffu;
+static_assert(kHaloKeys >= 27 * kBlock, "the sort buffer must hold the stencil keys of a full block");
+static_assert(kHaloKeys * (sizeof(uint32_t) + sizeof(uint16_t)) <= kSearchX + kSearchL, "general path buffers");
+static_assert(kBoxCells / 32 * (sizeof(uint32_t) + sizeof(uint16_t)) + (kHaloCells + 2) * sizeof(uint16_t) +
+                      kHaloCells * sizeof(uint32_t) + kBlock * sizeof(int3) <= kSearchL, "halo construction buffers");
+
+// Two f32 operations in one instruction (each rounded like the scalar one).
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Distance tests of one particle against n staged candidates (n a multiple of
+// four, px/py/pz 16-byte aligned): the sign bit of r^2 - limit of candidate c
+// ends at bit n - 1 - c.
+struct RangeTest32 {
+  unsigned long long x, y, z, limit;
+  __device__ __forceinline__ RangeTest32(const R4<float>& xi, float lim)
+      : x(pack2(-xi.x, -xi.x)), y(pack2(-xi.y, -xi.y)), z(pack2(-xi.z, -xi.z)), limit(pack2(-lim, -lim)) {}
+  __device__ __forceinline__ unsigned long long two(unsigned long long a, unsigned long long b,
+                                                    unsigned long long c) const {
+    const unsigned long long dx = add2(a, x), dy = add2(b, y), dz = add2(c, z);
+    return fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, limit)));
+  }
+  __device__ __forceinline__ uint32_t run(const float* px, const float* py, const float* pz, int n) const {
+    uint32_t hits = 0;
+#pragma unroll 2
+    for (int c = 0; c < n; c += 4) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(px + c);
+      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(py + c);
+      const ulonglong2 d = *reinterpret_cast<const ulonglong2*>(pz + c);
+      const unsigned long long r0 = two(a.x, b.x, d.x), r1 = two(a.y, b.y, d.y);
+      hits = __funnelshift_l((uint32_t)r0, hits, 1);
+      hits = __funnelshift_l((uint32_t)(r0 >> 32), hits, 1);
+      hits = __funnelshift_l((uint32_t)r1, hits, 1);
+      hits = __funnelshift_l((uint32_t)(r1 >> 32), hits, 1);
+    }
+    return hits;
+  }
+};
+struct RangeTest64 {
+  double x, y, z, limit;
+  __device__ __forceinline__ RangeTest64(const R4<double>& xi, double lim) : x(xi.x), y(xi.y), z(xi.z), limit(lim) {}
+  __device__ __forceinline__ double one(double a, double b, double c) const {
+    const double dx = a - x, dy = b - y, dz = c - z;
+    return dz * dz + (dy * dy + (dx * dx - limit));
+  }
+  __device__ __forceinline__ uint32_t run(const double* px, const double* py, const double* pz, int n) const {
+    uint32_t hits = 0;
+    for (int c = 0; c < n; c += 2) {
+      const double2 a = *reinterpret_cast<const double2*>(px + c);
+      const double2 b = *reinterpret_cast<const double2*>(py + c);
+      const double2 d = *reinterpret_cast<const double2*>(pz + c);
+      hits = __funnelshift_l(sign_word(one(a.x, b.x, d.x)), hits, 1);
+      hits = __funnelshift_l(sign_word(one(a.y, b.y, d.y)), hits, 1);
+    }
+    return hits;
+  }
+};
+template <class R>
+using RangeTest = std::conditional_t<sizeof(R) == 4, RangeTest32, RangeTest64>;
+
+// Compensated (Kahan) sum of W over the neighbors in list order, on top of the
+// self term W(0) = alpha/h^3 / 2; add() takes the coordinates of four
+// neighbors, of which the first n count, and keeps the largest squared
+// distance. f32: two kernel values per packed instruction (the square root is r^2 rsqrt(r^2) with one Heron step, its
+// residual in one fma, which gives the rounded root).
+struct KernelSum32 {
+  unsigned long long x, y, z;
+  float ih, cw, s, c = 0.f, farthest = 0.f;
+  __device__ __forceinline__ KernelSum32(const R4<float>& xi, const KernelConst<float>& k)
+      : x(pack2(-xi.x, -xi.x)), y(pack2(-xi.y, -xi.y)), z(pack2(-xi.z, -xi.z)), ih(-k.inv_h),
+        cw(k.cw), s(k.cw * 0.5f) {}
+  __device__ __forceinline__ void one(float w) {
+    const float v = fmaf(cw, w, -c), n = s + v;
+    c = (n - s) - v;
+    s = n;
+  }
+  __device__ __forceinline__ void two(const R4<float>& a, const R4<float>& b, int n) {
+    const unsigned long long dx = add2(pack2(a.x, b.x), x), dy = add2(pack2(a.y, b.y), y),
+                             dz = add2(pack2(a.z, b.z), z);
+    // (2e-38 keeps the root of a coincident neighbor finite)
+    const unsigned long long d = fma2(dz, dz, fma2(dx, dx, fma2(dy, dy, pack2(2e-38f, 2e-38f))));
+    const float r0 = __uint_as_float((uint32_t)d), r1 = __uint_as_float((uint32_t)(d >> 32));
+    farthest = fmaxf(farthest, r0);
+    if (n > 1) farthest = fmaxf(farthest, r1);
+    float i0, i1;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i0) : "f"(r0));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i1) : "f"(r1));
+    const unsigned long long inv = pack2(i0, i1);
+    const unsigned long long minus = pack2(-1.f, -1.f), half = pack2(0.5f, 0.5f);
+    unsigned long long r = mul2(d, inv);
+    r = fma2(fma2(mul2(r, minus), r, d), mul2(inv, half), r);
+    // -|r|/h, in scalar form: a packed product and the packed sums behind it
+    // were measured to round once, and with them the volumes' last bits change
+    const unsigned long long q = pack2(__fmul_rn(__uint_as_float((uint32_t)r), ih),
+                                       __fmul_rn(__uint_as_float((uint32_t)(r >> 32)), ih));
+    // (a neighbor is within the support up to rounding: 1 - q needs no clamp)
+    const unsigned long long a1 = add2(pack2(1.f, 1.f), q), u = add2(half, q);
+    const unsigned long long b1 = pack2(fmaxf(__uint_as_float((uint32_t)u), 0.f),
+                                        fmaxf(__uint_as_float((uint32_t)(u >> 32)), 0.f));
+    const unsigned long long w = fma2(mul2(a1, a1), a1, mul2(mul2(mul2(b1, b1), b1), pack2(-4.f, -4.f)));
+    one(__uint_as_float((uint32_t)w));
+    if (n > 1) one(__uint_as_float((uint32_t)(w >> 32)));
+  }
+  __device__ __forceinline__ void add(const R4<float> p[4], int n) {
+    two(p[0], p[1], n);
+    if (n > 2) two(p[2], p[3], n - 2);
+  }
+};
+struct KernelSum64 {
+  R4<double> xi;
+  KernelConst<double> k;
+  double s, c = 0, farthest = 0;
+  __device__ __forceinline__ KernelSum64(const R4<double>& x, const KernelConst<double>& kc)
+      : xi(x), k(kc), s(kc.cw * 0.5) {}
+  __device__ __forceinline__ void add(const R4<double> p[4], int n) {
 #pragma unroll
-    for (int pass = 0; pass < 27; ++pass) {
-#pragma unroll
-      for (int q = pass & 1; q + 1 < 27; q += 2) {
-        const uint32_t a = keys[q], b = keys[q + 1];
-        keys[q] = min(a, b);
-        keys[q + 1] = max(a, b);
+    for (int u = 0; u < 4; ++u) {
+      if (u >= n) break;
+      const double rx = xi.x - p[u].x, ry = xi.y - p[u].y, rz = xi.z - p[u].z;
+      const double r2 = rx * rx + ry * ry + rz * rz;
+      farthest = fmax(farthest, r2);
+      kahan_add(s, c, kernel_w_r2(r2, k));
+    }
+  }
+};
+template <class R>
+using KernelSum = std::conditional_t<sizeof(R) == 4, KernelSum32, KernelSum64>;
+
+// The neighbors one particle has found, before they are written out: up to
+// kListStage halo positions in shared memory (entry k of thread t at
+// [k * kBlock + t]), a longer list in its place in global memory.
+struct FoundList {
+  uint16_t* s;       // shared memory, this thread's entry 0
+  uint16_t* list;    // global memory: entry k at list[(k >> 2) * 128 + (k & 3)]
+  int cap;           // capacity of the global list
+  int cnt = 0;
+  bool global = false;
+  __device__ __forceinline__ uint16_t& slot(int k) {
+    return global ? list[(size_t)(k >> 2) * 128 + (k & 3)] : s[k * kBlock];
+  }
+  // hits: candidate p + c at bit 31 - c
+  __device__ __forceinline__ void add(uint32_t hits, uint32_t p) {
+    const int n = __popc(hits);
+    if (!global && cnt + n > kListStage) {
+      for (int k = 0; k < min(cnt, cap); ++k) list[(size_t)(k >> 2) * 128 + (k & 3)] = s[k * kBlock];
+      global = true;
+    }
+    if (!global) {
+      uint16_t* dst = s + cnt * kBlock;
+      cnt += n;
+      while (hits) {
+        const int hb = __clz(hits);
+        hits ^= 0x80000000u >> hb;
+        *dst = (uint16_t)(p + (uint32_t)hb);
+        dst += kBlock;
+      }
+    } else {
+      while (hits) {
+        const int hb = __clz(hits);
+        hits ^= 0x80000000u >> hb;
+        if (cnt < cap) slot(cnt) = (uint16_t)(p + (uint32_t)hb);
+        ++cnt;
       }
     }
   }
-}
+};
 
-constexpr int kHashSlots = 4096;   // halo bucket set of a block (hash path)
-constexpr int kHashElems = 3072;   // stencil keys the hash path takes (27 per cell)
-__device__ __forceinline__ uint32_t hash_slot(uint32_t k) { return (k * 0x9E3779B1u) >> 20; }  // 12 bits
-
-// Writes a neighbor list in whole groups of four 16-bit halo positions (one
-// 8-byte store per group instead of one 2-byte store per neighbor); the last
-// group is completed with the particle's own position.
-struct ListWriter {
-  uint2* groups;  // this particle's group 0; group g sits 32 uint2 further
-  int cap;        // list capacity (a multiple of four)
-  uint32_t g0 = 0, g1 = 0;
-  __device__ __forceinline__ void add(int cnt, uint32_t l) {
-    const int q = cnt & 3;
-    if (q < 2) g0 = q == 0 ? l : (g0 | (l << 16));
-    else g1 = q == 2 ? l : (g1 | (l << 16));
-    if (q == 3 && cnt < cap) groups[(size_t)(cnt >> 2) * 32] = make_uint2(g0, g1);
+// Bank-aware list order: a particle's entries in one queue per halo position
+// modulo 8 (a full queue passes its entries on to the next); slot k of lane j
+// takes from queue (j + k) mod 8, or the next one that has entries left. A
+// 16-byte staged record at halo position l sits in shared-memory bank group
+// l mod 8, so the eight lanes of one 16-byte load phase of a neighbor pass
+// then mostly hit different groups.
+constexpr int kOrderQueue = kListStage / 8;
+struct OrderQueues {
+  uint16_t* s;                   // shared memory, this thread's entry 0
+  uint32_t fill = 0;             // entries per queue, four bits each
+  uint32_t cur = 0, avail = 0;   // entries taken per queue; queues with entries left (the mask twice)
+  __device__ __forceinline__ void push(uint32_t l) {
+    uint32_t q = 4u * (l & 7u), f = (fill >> q) & 15u;
+    while (f >= (uint32_t)kOrderQueue) {
+      q = (q + 4u) & 31u;
+      f = (fill >> q) & 15u;
+    }
+    fill += 1u << q;
+    avail |= 0x101u << (q >> 2);
+    s[((q >> 2) * kOrderQueue + f) * kBlock] = (uint16_t)l;
   }
-  __device__ __forceinline__ void finish(int cnt, uint32_t self) {
-    if (cnt >= cap || (cnt & 3) == 0) return;
-    for (int k = cnt; (k & 3) != 0; ++k) add(k, self);
+  __device__ __forceinline__ uint32_t pop(uint32_t want) {
+    const uint32_t r = (want + (uint32_t)__ffs((int)(avail >> want)) - 1u) & 7u, q = 4u * r;
+    const uint32_t c = (cur >> q) & 15u;
+    cur += 1u << q;
+    if (c + 1u == ((fill >> q) & 15u)) avail &= ~(0x101u << r);
+    return s[(r * kOrderQueue + c) * kBlock];
   }
 };
 
-template <class R>
-__global__ void __launch_bounds__(kBlock) k_neighbors_density(
+// Neighbor search and volume of one block of sorted particles.
+//
+// Halo: the block's cells are marked, each with its 26 neighbors, in a bitmap
+// over their bounding box (rows along x), so the rank of a set bit is the
+// cell's place in the halo and the three cells of a stencil row lie side by
+// side: a cell's candidates are nine runs of halo positions. A block whose
+// Morton keys cross a boundary of 16^3 cells, where the curve jumps, keeps
+// one box on either side of it (a cell that both hold is in the halo twice,
+// which only costs room). A block whose boxes or cells are too many (sparse
+// particles) sorts the stencil keys instead and visits 27 buckets per
+// particle.
+//
+// Candidates: each particle walks its cell's runs in pieces of up to 32
+// positions, four at a time, two per packed f32 instruction. A test is
+// branch-free: the sign bit of r^2 - h^2 (h^2 widened by the guard band) goes
+// into a mask, and the mask's set bits to the particle's list in shared
+// memory. A pass over the list sums the kernel; it decides the neighbors
+// inside the guard band by the exact f64 predicate, and a particle that loses
+// one there takes the pass again. The lists then go out in whole groups of
+// four, for the IISPH sweeps (ORDER) in bank-aware order.
+//
+// What bounds it: issue (about 216 candidates per particle; 73 % of the issue
+// slots used, 211 M warp instructions for one million particles at spacing
+// h/2). That scene took 470 us with a test-and-append loop per candidate over
+// 27 hashed buckets, and 78 us more in a kernel of its own for the bank-aware
+// order; in this form 270 us for both.
+template <class R, bool ORDER>
+__global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
     Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const uint32_t* __restrict__ start,
     R4<R>* __restrict__ xv, uint16_t* __restrict__ nbr, uint32_t* __restrict__ ncnt,
     uint32_t* __restrict__ halo_idx, uint32_t* __restrict__ halo_n, const R* __restrict__ bW,
     int has_boundary, int hcap, StepParams<R> P) {
   extern __shared__ __align__(32) unsigned char dsm[];
-  __shared__ int3 s_cell[kBlock];
-  __shared__ int s_own[kBlock];      // per cell: own bucket's halo offset - its first particle
+  __shared__ int s_own[kSearchCells];        // per cell: own bucket's halo offset - its first particle
+  __shared__ uint8_t s_head[kSearchCells];   // per cell: its first thread
   __shared__ uint32_t s_scan[32];
+  __shared__ int s_box[2][6];
+  __shared__ uint32_t s_ends[2];        // keys of the block's first and last particle
+  constexpr uint32_t kStage = (uint32_t)(kSearchX / (3 * sizeof(R)));
+  R* s_px = reinterpret_cast<R*>(dsm);
+  R* s_py = s_px + kStage;
+  R* s_pz = s_py + kStage;
+  int3* s_cell = reinterpret_cast<int3*>(dsm + kSearchX + kSearchL) - kBlock;  // the end of region L
+  uint16_t* s_list = reinterpret_cast<uint16_t*>(dsm + kSearchX);
+  uint32_t* s_row = reinterpret_cast<uint32_t*>(dsm + kSearchX + kSearchL);  // offset | length << 16, nine per cell
   const int tid = threadIdx.x;
   const int i = blockIdx.x * kBlock + tid;
   const bool active = i < sc->n_active;
   R4<R> xi = R4<R>{R(0), R(0), R(0), R(0)};
+  uint32_t key = 0;
   int cx = 0, cy = 0, cz = 0;
   if (active) {
     xi = pos[i];
-    cx = cell_coord((double)xi.x, P.range);
-    cy = cell_coord((double)xi.y, P.range);
-    cz = cell_coord((double)xi.z, P.range);
+    key = lane_key(xi.w);
+    // (the cell modulo the bucket grid, which is all that the stencil's buckets depend on)
+    cx = (int)gather3(key);
+    cy = (int)gather3(key >> 1);
+    cz = (int)gather3(key >> 2);
   }
   s_cell[tid] = make_int3(cx, cy, cz);
+  if (tid < 12) s_box[tid / 6][tid % 6] = tid % 6 < 3 ? 0x7fffffff : (int)0x80000000;
+  if (tid == 0) s_ends[0] = key;
+  if (i == min((int)(blockIdx.x + 1) * kBlock, sc->n_active) - 1) s_ends[1] = key;
   __syncthreads();
   // one head per run of particles in the same cell
   const int3 prev = tid > 0 ? s_cell[tid - 1] : make_int3(0, 0, 0);
   const bool head = active && (tid == 0 || prev.x != cx || prev.y != cy || prev.z != cz);
+  const int jump = 31 - __clz((int)((s_ends[0] ^ s_ends[1]) | 1u));  // highest key bit the block's cells differ in
+  const bool split = jump >= kBoxLevel;
+  const int side = split ? (int)((key >> jump) & 1u) : 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int c = d == 0 ? cx : (d == 1 ? cy : cz);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      if (e == 1 && !split) break;
+      const bool in = active && side == e;
+      const int lo = __reduce_min_sync(0xffffffffu, in ? c : 0x7fffffff);
+      const int hi = __reduce_max_sync(0xffffffffu, in ? c : (int)0x80000000);
+      if ((tid & 31) == 0 && lo <= hi) {
+        atomicMin(&s_box[e][d], lo);
+        atomicMax(&s_box[e][3 + d], hi);
+      }
+    }
+  }
   uint32_t nheads = 0;
   const uint32_t rank = block_excl_scan_u32(head ? 1u : 0u, s_scan, &nheads);
-  const int nk = 27 * (int)nheads;
+  const int hr = (int)rank - (head ? 0 : 1);  // this particle's cell
+  if (head && rank < (uint32_t)kSearchCells) s_head[rank] = (uint8_t)tid;
   uint32_t* hidx = halo_idx + (size_t)blockIdx.x * (size_t)hcap;
   uint32_t H = 0;
   bool miss = false;
-  // Per cell, the 27 stencil buckets as (halo offset << 16 | size) spans in
-  // ascending key order, in `span_tab` (27 words per cell) when the cells fit,
-  // else per particle in `span`.
-  const bool hashed = nk <= kHashElems;
-  uint32_t* span_tab = nullptr;
-  uint32_t span[27];
-  if (hashed) {
-    // hash path: the set of the cells' stencil buckets in a shared hash table,
-    // halo offsets in slot order
-    uint32_t* hkey = reinterpret_cast<uint32_t*>(dsm);            // kHashSlots
-    uint32_t* hval = hkey + kHashSlots;                            // kHashSlots: offset << 16 | size
-    span_tab = hval + kHashSlots;                                  // kHashElems: keys, then spans
-    for (int t = tid; t < kHashSlots; t += kBlock) hkey[t] = kNoKey;
+  int own_local = 0;
+  uint32_t span[27];  // general path: the particle's buckets as offset | length << 16
+  // the cells of each side and their neighbors as a box of nx x ny x nz cells,
+  // the second box's bits behind the first's
+  int nx[2] = {0, 0}, ny[2] = {0, 0}, bits[2] = {0, 0};
+  bool boxed = nheads > 0 && nheads <= (uint32_t)kSearchCells;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    if (s_box[e][0] > s_box[e][3]) continue;  // no cells on this side
+    const long long bx = (long long)s_box[e][3] - s_box[e][0] + 3, by = (long long)s_box[e][4] - s_box[e][1] + 3,
+                    bz = (long long)s_box[e][5] - s_box[e][2] + 3;
+    boxed = boxed && bx <= kBoxCells && by <= kBoxCells && bz <= kBoxCells && bx * by <= kBoxCells &&
+            bx * by * bz <= kBoxCells;
+    if (!boxed) break;
+    nx[e] = (int)bx; ny[e] = (int)by; bits[e] = (int)(bx * by * bz);
+  }
+  const int second = (bits[0] + 31) & ~31, nbits = bits[1] ? second + bits[1] : bits[0];
+  boxed = boxed && nbits <= kBoxCells;
+  if (boxed) {
+    uint32_t* s_bits = reinterpret_cast<uint32_t*>(dsm + kSearchX);
+    uint32_t* s_first = s_bits + kBoxCells / 32;                            // per halo cell: its bucket's first particle
+    uint16_t* s_off = reinterpret_cast<uint16_t*>(s_first + kHaloCells);    // per halo cell: length, then halo offset
+    uint16_t* s_pre = s_off + kHaloCells + 2;                               // set bits before each word
+    const int nw = (nbits + 31) >> 5;
+    for (int t = tid; t < nw; t += kBlock) s_bits[t] = 0u;
+    __syncthreads();
+    // bit of the cell at (-1, dy, dz) of the stencil around cell c of side e
+    auto bit_of = [&](const int3& c, int e, int dy, int dz) {
+      return (e ? second : 0) + ((c.z - s_box[e][2] + 1 + dz) * (e ? ny[1] : ny[0]) + (c.y - s_box[e][1] + 1 + dy)) *
+                                    (e ? nx[1] : nx[0]) + (c.x - s_box[e][0]);
+    };
     if (head) {
-      uint32_t keys[27];
-      stencil_keys(cx, cy, cz, P.mask, P.sorted_lists, keys);
 #pragma unroll
-      for (int q = 0; q < 27; ++q) span_tab[27 * rank + q] = keys[q];
-    }
-    __syncthreads();
-    // Ordered linear probing: a slot keeps the smaller of its key and the
-    // one being inserted, and the larger moves on. The table (and so the
-    // halo layout) then does not depend on the order the threads insert in
-    // (kNoKey, the empty mark, is the largest key).
-    for (int e = tid; e < nk; e += kBlock) {
-      uint32_t k = span_tab[e];
-      uint32_t h = hash_slot(k);
-      for (int probe = 0; probe < kHashSlots; ++probe, h = (h + 1) & (kHashSlots - 1)) {
-        const uint32_t old = atomicMin(&hkey[h], k);
-        if (old == kNoKey || old == k) break;
-        if (old > k) k = old;
+      for (int q = 0; q < 9; ++q) {
+        const int b = bit_of(make_int3(cx, cy, cz), side, q % 3 - 1, q / 3 - 1), w = b >> 5, sh = b & 31;
+        atomicOr(&s_bits[w], 7u << sh);
+        if (sh > 29) atomicOr(&s_bits[w + 1], 7u >> (32 - sh));
       }
     }
     __syncthreads();
-    // sizes of the distinct buckets, offsets by a block scan over the slots
-    constexpr int per = kHashSlots / kBlock;
-    uint32_t len[per], tot = 0;
-#pragma unroll
-    for (int u = 0; u < per; ++u) {
-      const uint32_t k = hkey[tid * per + u];
-      len[u] = k != kNoKey ? start[k + 1] - start[k] : 0u;
-      tot += len[u];
-    }
-    uint32_t run = block_excl_scan_u32(tot, s_scan, &H);
-#pragma unroll
-    for (int u = 0; u < per; ++u) {
-      const uint32_t k = hkey[tid * per + u];
-      miss |= len[u] > 0xffffu;
-      hval[tid * per + u] = (min(run, 65535u) << 16) | min(len[u], 65535u);
-      if (k != kNoKey) {
-        const uint32_t b = start[k];
-        for (uint32_t r = 0; r < len[u]; ++r)
-          if (run + r < (uint32_t)hcap) hidx[run + r] = b + r;
-      }
-      run += len[u];
-    }
+    uint32_t c0 = 0, c1 = 0, D = 0;
+    if (2 * tid < nw) c0 = __popc(s_bits[2 * tid]);
+    if (2 * tid + 1 < nw) c1 = __popc(s_bits[2 * tid + 1]);
+    const uint32_t before = block_excl_scan_u32(c0 + c1, s_scan, &D);
+    if (2 * tid < nw) s_pre[2 * tid] = (uint16_t)before;
+    if (2 * tid + 1 < nw) s_pre[2 * tid + 1] = (uint16_t)(before + c0);
     __syncthreads();
-    // each cell's spans: look its keys up in the table
-    for (int e = tid; e < nk; e += kBlock) {
-      const uint32_t k = span_tab[e];
-      uint32_t h = hash_slot(k), v = 0;
-      bool found = false;
-      for (int probe = 0; probe < kHashSlots; ++probe, h = (h + 1) & (kHashSlots - 1)) {
-        const uint32_t kk = hkey[h];
-        if (kk == k) { v = hval[h]; found = true; break; }
-        if (kk == kNoKey) break;
+    if (D > (uint32_t)kHaloCells) {
+      boxed = false;
+    } else {
+      auto cell_rank = [&](int b) { return (int)s_pre[b >> 5] + __popc(s_bits[b >> 5] & ((1u << (b & 31)) - 1u)); };
+      for (int b = tid; b < nbits; b += kBlock) {
+        if (!((s_bits[b >> 5] >> (b & 31)) & 1u)) continue;
+        const int r = cell_rank(b);
+        const int e = bits[1] && b >= second ? 1 : 0;
+        const int lx = e ? nx[1] : nx[0], lxy = lx * (e ? ny[1] : ny[0]), lb = e ? b - second : b;
+        const int z = lb / lxy, y = (lb - z * lxy) / lx, x = lb - z * lxy - y * lx;
+        const uint32_t k = morton_key(x + s_box[e][0] - 1, y + s_box[e][1] - 1, z + s_box[e][2] - 1, P.mask);
+        const uint32_t f = start[k], len = start[k + 1] - f;
+        miss |= len > 0xffffu;
+        s_first[r] = f;
+        s_off[r] = (uint16_t)min(len, 65535u);
       }
-      miss |= !found;
-      span_tab[e] = v;
-    }
-    if (head) {
-      // own bucket: its offset minus its first particle gives the halo position of i
-      const uint32_t own = morton_key(cx, cy, cz, P.mask);
-      uint32_t h = hash_slot(own), v = 0;
-      for (int probe = 0; probe < kHashSlots; ++probe, h = (h + 1) & (kHashSlots - 1)) {
-        const uint32_t kk = hkey[h];
-        if (kk == own) { v = hval[h]; break; }
-        if (kk == kNoKey) break;
+      __syncthreads();
+      for (uint32_t r0 = 0; r0 < D; r0 += kBlock) {  // lengths to offsets
+        const uint32_t r = r0 + tid;
+        uint32_t total = 0;
+        const uint32_t o = H + block_excl_scan_u32(r < D ? (uint32_t)s_off[r] : 0u, s_scan, &total);
+        if (r < D) s_off[r] = (uint16_t)min(o, 65535u);
+        H += total;
       }
-      s_own[rank] = (int)(v >> 16) - (int)start[own];
+      if (tid == 0) s_off[D] = (uint16_t)min(H, 65535u);
+      __syncthreads();
+      // the halo's particle indices, and its positions where they fit: eight lanes per cell
+      for (uint32_t r = tid >> 3; r < D; r += kBlock / 8) {
+        const uint32_t o = s_off[r], e = s_off[r + 1], f = s_first[r];
+        for (uint32_t l = o + (tid & 7); l < e; l += 8) {
+          if (l < (uint32_t)hcap) hidx[l] = f + (l - o);
+          if (l < kStage) {
+            const R4<R>* p = &pos[f + (l - o)];
+            async_copy(&s_px[l], &p->x);
+            async_copy(&s_py[l], &p->y);
+            async_copy(&s_pz[l], &p->z);
+          }
+        }
+      }
+      for (int e = tid; e < 9 * (int)nheads; e += kBlock) {
+        const int h = e / 9, q = e - 9 * h;
+        const int3 c = s_cell[s_head[h]];
+        const int e1 = split ? (int)((morton_key(c.x, c.y, c.z, P.mask) >> jump) & 1u) : 0;
+        const int r = cell_rank(bit_of(c, e1, q % 3 - 1, q / 3 - 1));
+        const uint32_t o = s_off[r];
+        s_row[e] = o | ((uint32_t)(s_off[r + 3] - o) << 16);
+        if (q == 4) s_own[h] = (int)s_off[r + 1] - (int)s_first[r + 1];
+      }
+      stage_done();  // the construction buffers become the lists
+      if (active) own_local = s_own[hr] + i;
     }
-  } else {
+  }
+  if (!boxed) {
     // general path: bitonic-sorted stencil keys, halo offsets in key order,
     // per-particle lookups by binary search
+    const int nk = 27 * (int)nheads;
     uint32_t* skey = reinterpret_cast<uint32_t*>(dsm);                 // sorted stencil keys
     uint16_t* soff = reinterpret_cast<uint16_t*>(skey + kHaloKeys);    // halo offset of each first key
     int S = 32;
     while (S < nk) S <<= 1;
+    __syncthreads();
     if (head) {
       uint32_t keys[27];
-      stencil_keys(cx, cy, cz, P.mask, 0, keys);
+      stencil_keys(cx, cy, cz, P.mask, keys);
 #pragma unroll
       for (int q = 0; q < 27; ++q) skey[27 * rank + q] = keys[q];
     }
@@ -771,7 +1043,7 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_density(
     __syncthreads();
     if (active) {
       uint32_t keys[27];
-      stencil_keys(cx, cy, cz, P.mask, P.sorted_lists, keys);
+      stencil_keys(cx, cy, cz, P.mask, keys);
       const uint32_t own = morton_key(cx, cy, cz, P.mask);
 #pragma unroll 1
       for (int q = 0; q < 27; ++q) {
@@ -786,200 +1058,141 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_density(
         const uint32_t b = start[k], len2 = start[k + 1] - b;
         miss |= !found || len2 > 0xffffu;
         const uint32_t off = found ? (uint32_t)soff[lo] : 0u;
-        span[q] = found && len2 <= 0xffffu ? (off << 16) | len2 : 0u;
-        if (k == own) s_own[tid] = (int)off - (int)b;
+        span[q] = off | (found && len2 <= 0xffffu ? len2 << 16 : 0u);
+        if (k == own) own_local = (int)off - (int)b + i;
       }
     }
+    __syncthreads();  // spans, offsets and halo_idx are complete; the sort buffers are free
+    if (H <= kStage && H <= (uint32_t)hcap)
+      for (uint32_t l = tid; l < H; l += kBlock) {
+        const R4<R> p = pos[hidx[l]];
+        s_px[l] = p.x;
+        s_py[l] = p.y;
+        s_pz[l] = p.z;
+      }
+    __syncthreads();
   }
   if (tid == 0) {
     halo_n[blockIdx.x] = H;
     atomicMax(&sc->max_halo, (int)min(H, 0x7fffffffu));
   }
-  __syncthreads();  // spans, offsets and halo_idx are complete; the sort / hash buffers are free
   const uint32_t usable = min(H, (uint32_t)hcap);
-  // The halo's positions move into the first 32 KB of shared memory when they
-  // fit (the cells' span table lies beyond them).
-  const bool staged = H <= usable && H <= (uint32_t)(2 * kHashSlots * sizeof(uint32_t) / sizeof(R4<R>));
-  R4<R>* s_x = reinterpret_cast<R4<R>*>(dsm);
-  if (staged)
-    for (uint32_t l = tid; l < H; l += kBlock) s_x[l] = pos[hidx[l]];
-  __syncthreads();
-  int cnt = 0;
+  const bool staged = H <= usable && H <= kStage;
+  FoundList found;
+  const uint32_t pad = (uint32_t)own_local < usable ? (uint32_t)own_local : 0u;  // the unused slots of a list's last group
   if (active) {
-    if (miss) atomicMax(&sc->max_halo, 0x7fffffff);  // cannot happen: every stencil bucket is in the halo
-    const int hr = head ? (int)rank : (int)rank - 1;  // this cell's row of the span table
-    const uint32_t* row = hashed ? span_tab + 27 * hr : nullptr;
-    const uint32_t own_local = (uint32_t)((hashed ? s_own[hr] : s_own[tid]) + i);
-    ListWriter lw;
-    lw.groups = reinterpret_cast<uint2*>(nbr + nbr_slot(i, 0, P.K));
-    lw.cap = P.K;
-    R sum = P.k.cw * R(0.5);  // self: W(0) = alpha/h^3 * 1/2
-    R comp = 0;
-    if (staged) {
-      // pass 1: the strict-range test over all candidates builds the list;
-      // in stencil order, a bucket whose cell lies entirely beyond the
-      // support radius (with a relative margin, so it only skips particles
-      // the test would reject) is passed over
-      const R h = (R)P.range;
-      const R cut2 = (R)(P.range * P.range * (1.0 + 1e-3));
-      const R lox = (R)cx * h, loy = (R)cy * h, loz = (R)cz * h;
-#pragma unroll 1
-      for (int q = 0; q < 27; ++q) {
-        const uint32_t sp = hashed ? row[q] : span[q];
-        const uint32_t off = sp >> 16;
-        uint32_t len = sp & 0xffffu;
-        if (!P.sorted_lists && len) {
-          const int ox = q % 3 - 1, oy = (q / 3) % 3 - 1, oz = q / 9 - 1;
-          const R ex = ox < 0 ? xi.x - lox : (ox > 0 ? lox + h - xi.x : R(0));
-          const R ey = oy < 0 ? xi.y - loy : (oy > 0 ? loy + h - xi.y : R(0));
-          const R ez = oz < 0 ? xi.z - loz : (oz > 0 ? loz + h - xi.z : R(0));
-          const R dx = fmax(ex, R(0)), dy = fmax(ey, R(0)), dz = fmax(ez, R(0));
-          if (dx * dx + dy * dy + dz * dz > cut2) len = 0;
-        }
-        for (uint32_t r = 0; r < len; ++r) {
-          const uint32_t local = off + r;
-          const R4<R> xj = s_x[local];
-          if (local != own_local && in_range(xi, xj, P.range, P.range2_lo, P.range2_hi)) {
-            lw.add(cnt, local);
-            ++cnt;
+    if (miss) atomicMax(&sc->max_halo, 0x7fffffff);  // a bucket beyond 65535 particles
+    found.s = s_list + tid;
+    found.list = nbr + nbr_slot(i, 0, P.K);
+    found.cap = P.K;
+    const RangeTest<R> range(xi, P.range2_out);
+    // (positions beyond a halo table that is too small are skipped: the update is redone with a larger one)
+    auto position = [&](uint32_t l) {
+      return staged ? R4<R>{s_px[l], s_py[l], s_pz[l], R(0)} : pos[hidx[l]];
+    };
+    auto test_run = [&](uint32_t row) {
+      const uint32_t o = row & 0xffffu, end = o + (row >> 16);
+      for (uint32_t p = o & ~3u; p < end; p += 32) {
+        const int n = min(32, (int)((end - p + 3u) & ~3u));
+        uint32_t hits;  // candidate p + c at bit 31 - c
+        if (staged) {
+          hits = range.run(s_px + p, s_py + p, s_pz + p, n) << (32 - n);
+        } else {
+          hits = 0;
+          for (int c = 0; c < n; ++c) {
+            const uint32_t l = p + c;
+            if (l >= o && l < end && l < usable) {
+              const R4<R> xj = pos[hidx[l]];
+              const R dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+              if (dx * dx + dy * dy + dz * dz < P.range2_out) hits |= 0x80000000u >> c;
+            }
           }
         }
+        if (p < o) hits &= 0xffffffffu >> (o - p);
+        if (end - p < 32u) hits &= ~(0xffffffffu >> (end - p));
+        const uint32_t self = (uint32_t)own_local - p;
+        if (self < 32u) hits &= ~(0x80000000u >> self);
+        found.add(hits, p);
       }
-      lw.finish(cnt, own_local);
-      // pass 2: the kernel sum over the neighbors, in list order
-      const int stored = min(cnt, P.K);
-      for (int k0 = 0; k0 < stored; k0 += 4) {
-        const uint2 w = lw.groups[(size_t)(k0 >> 2) * 32];
-        const uint32_t l[4] = {w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16};
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (k0 + u >= stored) break;
-          const R4<R> xj = s_x[l[u]];
-          const R rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-          kahan_add(sum, comp, kernel_w_r2(rx * rx + ry * ry + rz * rz, P.k));
-        }
-      }
+    };
+    if (boxed) {
+      const uint32_t* row = s_row + 9 * hr;
+#pragma unroll 1
+      for (int q = 0; q < 9; ++q) test_run(row[q]);
     } else {
 #pragma unroll 1
-      for (int q = 0; q < 27; ++q) {
-        const uint32_t sp = hashed ? row[q] : span[q];
-        const uint32_t off = sp >> 16, len = sp & 0xffffu;
-        const uint32_t b = len && off < usable ? hidx[off] : 0u;
-        for (uint32_t r = 0; r < len; ++r) {
-          const uint32_t j = b + r;
-          if ((int)j == i) continue;
-          const R4<R> xj = pos[j];
-          if (!in_range(xi, xj, P.range, P.range2_lo, P.range2_hi)) continue;
-          const uint32_t local = off + r;
-          lw.add(cnt, local < usable ? local : 0u);
-          ++cnt;
-          const R rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-          kahan_add(sum, comp, kernel_w_r2(rx * rx + ry * ry + rz * rz, P.k));
+      for (int q = 0; q < 27; ++q) test_run(span[q]);
+    }
+    // the kernel sum in list order
+    R sum;
+    for (;;) {
+      const int stored = min(found.cnt, P.K);
+      KernelSum<R> acc(xi, P.k);
+      if (staged && !found.global) {
+        const uint16_t* e = found.s;
+        int k = stored;
+        for (; k >= 4; k -= 4, e += 4 * kBlock) {
+          R4<R> xj[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t l = e[u * kBlock];
+            xj[u] = R4<R>{s_px[l], s_py[l], s_pz[l], R(0)};
+          }
+          acc.add(xj, 4);
+        }
+        for (; k > 0; --k, e += kBlock) {
+          const uint32_t l = e[0];
+          const R4<R> xj[4] = {R4<R>{s_px[l], s_py[l], s_pz[l], R(0)}};
+          acc.add(xj, 1);
+        }
+      } else {
+        for (int k = 0; k < stored; ++k) {
+          const R4<R> xj[4] = {position((uint32_t)found.slot(k))};
+          acc.add(xj, 1);
         }
       }
+      sum = acc.s;
+      if (!(acc.farthest >= P.range2_lo)) break;
+      // some neighbor lies inside the guard band: keep those the exact predicate keeps
+      int kept = 0;
+      for (int k = 0; k < stored; ++k) {
+        const uint32_t l = found.slot(k);
+        if (in_range(xi, position(l), P.range, P.range2_lo, P.range2_hi)) found.slot(kept++) = (uint16_t)l;
+      }
+      if (kept == stored) break;  // all of them
+      found.cnt -= stored - kept;
     }
-    // The unused slots of the last group of four hold the particle's own halo
-    // position: a sweep pass reads whole groups, and the self pair adds zero.
-    if (!staged) lw.finish(cnt, own_local < usable ? own_local : 0u);
     R denom = P.V0 * sum;
     if (has_boundary) denom += bW[i];
     const R V = P.V0 / denom;
     xv[i] = R4<R>{xi.x, xi.y, xi.z, V};
-    ncnt[i] = (uint32_t)cnt;
+    ncnt[i] = (uint32_t)found.cnt;
   }
+  // The lists in whole groups of four. The unused slots of the last group hold
+  // the particle's own halo position: the passes over neighbors read whole
+  // groups, and the self pair adds zero.
+  if (ORDER) __syncthreads();  // the queues take the place of the positions
+  if (active) {
+    const int stored = min(found.cnt, P.K);
+    uint2* groups = reinterpret_cast<uint2*>(found.list);
+    OrderQueues queue;
+    queue.s = reinterpret_cast<uint16_t*>(dsm) + tid;
+    if (ORDER && !found.global)
+      for (int k = 0; k < stored; ++k) queue.push(found.s[k * kBlock]);
+    for (int k0 = 0; k0 < stored; k0 += 4) {
+      uint32_t l[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        l[u] = k0 + u >= stored ? pad
+               : ORDER && !found.global ? queue.pop((uint32_t)(i + k0 + u) & 7u)
+                                        : (uint32_t)found.slot(k0 + u);
+      groups[(size_t)(k0 >> 2) * 32] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+    }
+  }
+  int cnt = found.cnt;
   // block max of the neighbor count
   for (int o = 16; o > 0; o >>= 1) cnt = max(cnt, __shfl_down_sync(0xffffffffu, cnt, o));
   if ((threadIdx.x & 31) == 0 && cnt > 0) atomicMax(&sc->max_nbrs, cnt);
-}
-
-// Reorders each particle's neighbor list so that, at one list slot, the lanes
-// of a warp tend to read different shared-memory banks in the neighbor
-// passes: lane j's slot k takes an entry whose halo position is j + k modulo
-// 8 when it has one left, else the next residue it has (cyclically). A 16-byte
-// staged record at halo position l sits in bank group l mod 8, so the eight
-// lanes of one 16-byte load phase then mostly hit eight different groups.
-// The list stays the same multiset; its padding slots keep the particle's own
-// position. Lists longer than KMAX keep their order.
-// RES residues (8: 16-byte records, eight lanes per shared-memory phase; 16:
-// also the 8-byte records of the second sweep pass, sixteen lanes per phase).
-// Dynamic shared memory: order_lists_smem(KMAX, RES) bytes.
-__host__ __device__ constexpr size_t order_lists_smem(int kmax, int res) {
-  return (size_t)kmax * kBlock * sizeof(uint16_t) + 2 * (size_t)res * kBlock * sizeof(uint32_t);
-}
-constexpr int kOrderResidues = 8;
-template <int KMAX, int RES>
-__global__ void __launch_bounds__(kBlock) k_order_lists(const Scalars* __restrict__ sc, uint16_t* __restrict__ nbr,
-                                                       const uint32_t* __restrict__ ncnt, int K) {
-  static_assert(RES == 8 || RES == 16, "8 or 16 residues");
-  extern __shared__ __align__(32) unsigned char dsm[];
-  uint32_t* s_cur = reinterpret_cast<uint32_t*>(dsm);  // per residue r of thread t, at [r * kBlock + t]:
-  uint32_t* s_end = s_cur + RES * kBlock;               //   the next slot to read and the end of its entries
-  uint16_t* ent = reinterpret_cast<uint16_t*>(s_end + RES * kBlock);  // entry e of thread t at [e * kBlock + t]
-  constexpr uint32_t M = RES - 1;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t = threadIdx.x;
-  if (i >= sc->n_active) return;
-  const int cnt = min((int)ncnt[i], K);
-  if (cnt < 2 || cnt > KMAX) return;
-  uint2* groups = reinterpret_cast<uint2*>(nbr + nbr_slot(i, 0, K));
-  const int ng = (cnt + 3) >> 2;
-#pragma unroll
-  for (int r = 0; r < RES; ++r) s_end[r * kBlock + t] = 0;
-  // entries per residue
-  uint2 last = make_uint2(0u, 0u);
-  for (int g = 0; g < ng; ++g) {
-    const uint2 w = groups[(size_t)g * 32];
-    last = w;
-    const uint32_t e[4] = {w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16};
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (4 * g + u < cnt) ++s_end[(e[u] & M) * kBlock + t];
-  }
-  // the entries grouped by residue (list order inside a residue); s_end
-  // advances from each residue's first slot to its end
-  uint32_t avail = 0, run = 0;
-#pragma unroll
-  for (int r = 0; r < RES; ++r) {
-    const uint32_t c = s_end[r * kBlock + t];
-    s_cur[r * kBlock + t] = run;
-    s_end[r * kBlock + t] = run;
-    if (c) avail |= ((1u << RES) + 1u) << r;  // the mask twice: a rotation is one shift
-    run += c;
-  }
-  for (int g = 0; g < ng; ++g) {
-    const uint2 w = groups[(size_t)g * 32];
-    const uint32_t e[4] = {w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16};
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (4 * g + u < cnt) {
-        uint32_t& f = s_end[(e[u] & M) * kBlock + t];
-        const uint32_t pos = f;
-        ent[pos * kBlock + t] = (uint16_t)e[u];
-        f = pos + 1;
-      }
-  }
-  const uint32_t pad[4] = {last.x & 0xffffu, last.x >> 16, last.y & 0xffffu, last.y >> 16};
-  uint32_t target = (uint32_t)i & M;  // lane j's slot k wants residue j + k (mod RES)
-  for (int g = 0; g < ng; ++g) {
-    uint32_t v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = 4 * g + u;
-      if (k >= cnt) {
-        v[u] = pad[u];
-        continue;
-      }
-      // the first residue at or after the target (cyclically) with entries left
-      const uint32_t r = (target + (uint32_t)(__ffs(avail >> target) - 1)) & M;
-      uint32_t& c = s_cur[r * kBlock + t];
-      const uint32_t pos = c;
-      v[u] = ent[pos * kBlock + t];
-      c = pos + 1;
-      if (pos + 1 == s_end[r * kBlock + t]) avail &= ~(((1u << RES) + 1u) << r);
-      target = (target + 1) & M;
-    }
-    groups[(size_t)g * 32] = make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
-  }
 }
 
 // ---------------------------------------------------------------------------

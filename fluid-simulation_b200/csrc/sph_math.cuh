@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <math_constants.h>
 
 namespace sph {
 
@@ -193,6 +194,10 @@ __device__ __forceinline__ bool in_range(const R4<R>& a, const R4<R>& b, double 
                         (double)b.z, range);
 }
 
+// The word of a number that holds its sign bit (bit 31; NaN results carry 0).
+__device__ __forceinline__ uint32_t sign_word(float v) { return (uint32_t)__float_as_int(v); }
+__device__ __forceinline__ uint32_t sign_word(double v) { return (uint32_t)__double2hiint(v); }
+
 // Cell of a position: floor(p / cell_size) in f64, saturated to i32 like
 // Rust's `as i32` (spatial_hashing.rs:40-46).
 __device__ __forceinline__ int cell_coord(double p, double cell_size) {
@@ -218,5 +223,25 @@ __device__ __forceinline__ uint32_t morton_key(int cx, int cy, int cz, uint32_t 
   return spread3((uint32_t)cx & mask) | (spread3((uint32_t)cy & mask) << 1) |
          (spread3((uint32_t)cz & mask) << 2);
 }
+
+// The inverse of spread3: every third bit of a key.
+__device__ __forceinline__ uint32_t gather3(uint32_t v) {
+  v &= 0x09249249;
+  v = (v | (v >> 2)) & 0x030C30C3;
+  v = (v | (v >> 4)) & 0x0300F00F;
+  v = (v | (v >> 8)) & 0x030000FF;
+  v = (v | (v >> 16)) & 0x3ff;
+  return v;
+}
+
+// A particle's key in the spare lane of its position.
+template <class R>
+__device__ __forceinline__ R key_lane(uint32_t k);
+template <>
+__device__ __forceinline__ float key_lane<float>(uint32_t k) { return __uint_as_float(k); }
+template <>
+__device__ __forceinline__ double key_lane<double>(uint32_t k) { return __hiloint2double(0, (int)k); }
+__device__ __forceinline__ uint32_t lane_key(float w) { return __float_as_uint(w); }
+__device__ __forceinline__ uint32_t lane_key(double w) { return (uint32_t)__double2loint(w); }
 
 }  // namespace sph

@@ -119,7 +119,8 @@ static void upload_serendipity_tables() {
 // Host-buffer state exchange in reference index order (sph_step_host).
 template <class R>
 __global__ void k_state_in(int n, const uint32_t* __restrict__ ref, const double* __restrict__ x,
-                           const double* __restrict__ v, R4<R>* __restrict__ pos, R4<R>* __restrict__ vel) {
+                           const double* __restrict__ v, R4<R>* __restrict__ pos, R4<R>* __restrict__ vel,
+                           R4<R>* __restrict__ xv) {
   const int d = blockIdx.x * blockDim.x + threadIdx.x;
   if (d >= n) return;
   const size_t r = ref[d];
@@ -127,6 +128,8 @@ __global__ void k_state_in(int n, const uint32_t* __restrict__ ref, const double
     R4<R> p = pos[d];
     p.x = (R)x[3 * r]; p.y = (R)x[3 * r + 1]; p.z = (R)x[3 * r + 2];
     pos[d] = p;
+    p.w = R(0);
+    xv[d] = p;  // the positions the step integrates from live here too
   }
   if (v) {
     R4<R> q = vel[d];
@@ -158,7 +161,6 @@ class System : public SystemBase {
  public:
   explicit System(const sph_config& c) : cfg_(c) {
     device = c.device;
-    if (const char* e = std::getenv("SPHGPU_SORTED_LISTS")) sorted_lists_ = std::atoi(e) != 0;
     if (const char* e = std::getenv("SPHGPU_DEPENDENT_LAUNCH")) pdl_ = std::atoi(e) != 0;
     if (const char* e = std::getenv("SPHGPU_SWEEP_PREFETCH")) prefetch_ = std::atoi(e) != 0;
     if (const char* e = std::getenv("SPHGPU_HALO_STAGE")) {
@@ -699,9 +701,8 @@ class System : public SystemBase {
         cuda_check(cudaStreamWaitEvent(stream_, io_ready_, 0), "event");
       }
       launch("state_io", k_state_in<R>, dim3(nb), dim3(kBlock), (int)n_, (const uint32_t*)ref_.p,
-             (const double*)(xi ? stage_x_.p : nullptr), (const double*)(vi ? stage_v_.p : nullptr), pos_.p, vel_.p);
-      // the positions the step integrates from live in xv too
-      if (xi) cuda_check(cudaMemcpyAsync(xv_.p, pos_.p, n_ * sizeof(R4<R>), cudaMemcpyDeviceToDevice, stream_), "D2D");
+             (const double*)(xi ? stage_x_.p : nullptr), (const double*)(vi ? stage_v_.p : nullptr), pos_.p, vel_.p,
+             xv_.p);
     }
     // The state a step returns is final once its update has sorted the
     // integrated particles, so the last step's readback is issued right
@@ -839,11 +840,6 @@ class System : public SystemBase {
   uint64_t time_offset_steps_ = 0;
   int last_iters_ = 3;
   int nb_ = 4;  // neighbor gather batch (prefetch width) of the neighbor passes
-  // Neighbor lists in ascending stencil-key order (1) or in stencil order (0,
-  // the default: neighbor records come from the block's staged halo, so list
-  // order no longer matters for memory locality, and stencil order lets the
-  // search skip buckets whose cell lies beyond the support radius).
-  bool sorted_lists_ = false;
   bool pdl_ = true;       // programmatic dependent launch between the sweep passes
   bool prefetch_ = true;  // sweep passes prefetch the next wave's streams into L2
   std::map<std::pair<const void*, size_t>, int> resident_;
@@ -1040,6 +1036,7 @@ class System : public SystemBase {
     const double band = sizeof(R) == 4 ? 1e-5 : 1e-12;
     P_.range2_lo = (R)(h * h * (1.0 - band));
     P_.range2_hi = (R)(h * h * (1.0 + band));
+    P_.range2_out = (R)(h * h * (1.0 + 1.1 * band));
     P_.spacing = sp;
     P_.V0 = (R)(sp * sp * sp);
     P_.visc_f = (R)(cfg_.fluid_viscosity * 2.0 * (3.0 + 2.0));
@@ -1062,7 +1059,6 @@ class System : public SystemBase {
     P_.min_diag = (R)cfg_.min_diagonal_element;
     P_.tde = cfg_.target_density_error;
     P_.iteration_cap = (int)cfg_.max_solver_iterations;
-    P_.sorted_lists = sorted_lists_ ? 1 : 0;
   }
 
   // ---- launches ---------------------------------------------------------------
@@ -1592,14 +1588,11 @@ class System : public SystemBase {
              (const R4<R>*)pos_.p, (const VMDesc*)vms_.p, (int)fields_.size(), (const Body*)bodies_d_.p, vmx_.p,
              vmv_.p, bW_.p, bG_.p, bGu_.p, P_);
     }
-    launch_s("neighbors_density", k_neighbors_density<R>, dim3(nb), dim3(kBlock), kSearchSmem, d_sc_.p,
-             (const R4<R>*)pos_.p, (const uint32_t*)start_.p, xv_.p, nbr_.p, ncnt_.p, halo_idx_.p, halo_n_.p,
-             (const R*)bW_.p, boundary_kind_ ? 1 : 0, hcap_, P_);
-    // IISPH in f32 re-reads the lists in every sweep pass: order them for
-    // shared-memory banks once per update
-    if (sizeof(R) == 4 && (cfg_.pressure_solver == SPH_IISPH || cfg_.pressure_solver == SPH_IISPH_W_OST))
-      launch_s("order_lists", k_order_lists<64, kOrderResidues>, dim3(nb), dim3(kBlock),
-               order_lists_smem(64, kOrderResidues), (const Scalars*)d_sc_.p, nbr_.p, (const uint32_t*)ncnt_.p, K_);
+    // IISPH in f32 re-reads the lists in every sweep pass: they come out ordered for shared-memory banks
+    const bool order = sizeof(R) == 4 && (cfg_.pressure_solver == SPH_IISPH || cfg_.pressure_solver == SPH_IISPH_W_OST);
+    launch_s("neighbors_density", order ? k_neighbors_density<R, sizeof(R) == 4> : k_neighbors_density<R, false>,
+             dim3(nb), dim3(kBlock), kSearchSmem, d_sc_.p, (const R4<R>*)pos_.p, (const uint32_t*)start_.p, xv_.p,
+             nbr_.p, ncnt_.p, halo_idx_.p, halo_n_.p, (const R*)bW_.p, boundary_kind_ ? 1 : 0, hcap_, P_);
     calc_acceleration();
     launch("avg_density", k_avg_density<R>, dim3(nb), dim3(kBlock), d_sc_.p, (const R4<R>*)xv_.p,
            (const R4<R>*)vel_.p, partials_.p, P_);
