@@ -14,7 +14,7 @@
 //   halo  u32 [blocks][hcap] particle indices of each block's halo (the union
 //                           of its cells' stencil buckets), cell by cell
 //   ncnt  u32 [N]           neighbor counts
-//   bW, bG, bGu             per-particle boundary aggregates (see kernels)
+//   bW, bG, bGu, bA         per-particle boundary aggregates (see kernels)
 //   IISPH scratch: vstar R4, s R, aii R, accp R4, p R
 // Cell grid: a Morton key of floor(x / h) modulo 2^(3m) buckets; a counting
 // sort orders particles by bucket and, inside a bucket, by reference index.
@@ -54,6 +54,7 @@ struct Scalars {
   int max_bnbrs;                   // largest boundary-sample neighbor count seen
   int max_halo;                    // largest block halo (particles) seen
   unsigned int vm_near;            // particles within the support radius of a volume map
+  unsigned int n_touch;            // particles with a neighbor on a dynamic body
   // graph-captured stepping (the host reads these once per chunk)
   double time_acc;                 // simulated time under CFL steps
   unsigned int trouble;            // bits: 1 neighbor overflow, 2 disabled particles, 4 unconverged

@@ -12,7 +12,8 @@
 //   k_sort_*             spatial_hashing.rs:27-37 (populate) as a counting sort
 //   k_neighbors_density  spatial_hashing.rs:75-158, neighbor_search/mod.rs:118-155,
 //                        sph/quantities.rs:14-61 (get_volume)
-//   k_sample_aggregate   boundary_handling/static_sample_boundary.rs:157-168
+//   k_sample_boundary    boundary_handling/static_sample_boundary.rs:157-168,
+//                        sph/non_pressure_accelerations.rs (boundary viscosity)
 //   k_vm_sample          boundary_handling/volume_map_boundary.rs:1259-1424,
 //                        utilities/discretization.rs:437-557
 //   k_accel              sph/non_pressure_accelerations.rs:19-185,
@@ -178,6 +179,7 @@ __global__ void k_prologue(Scalars* sc, StepParams<R> P, int accumulate_time) {
   sc->max_bnbrs = 0;
   sc->max_halo = 0;
   sc->vm_near = 0;
+  sc->n_touch = 0;
   sc->iterations = 0;
   sc->iterations_eqs1 = 0;
   sc->converged = 0;
@@ -680,9 +682,11 @@ struct KernelSum32 {
   __device__ __forceinline__ void two(const R4<float>& a, const R4<float>& b, int n) {
     const unsigned long long dx = add2(pack2(a.x, b.x), x), dy = add2(pack2(a.y, b.y), y),
                              dz = add2(pack2(a.z, b.z), z);
-    // (2e-38 keeps the root of a coincident neighbor finite)
-    const unsigned long long d = fma2(dz, dz, fma2(dx, dx, fma2(dy, dy, pack2(2e-38f, 2e-38f))));
-    const float r0 = __uint_as_float((uint32_t)d), r1 = __uint_as_float((uint32_t)(d >> 32));
+    const unsigned long long r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
+    // (a coincident neighbor keeps a finite root)
+    const float r0 = fmaxf(__uint_as_float((uint32_t)r2), 1e-35f);
+    const float r1 = fmaxf(__uint_as_float((uint32_t)(r2 >> 32)), 1e-35f);
+    const unsigned long long d = pack2(r0, r1);
     farthest = fmaxf(farthest, r0);
     if (n > 1) farthest = fmaxf(farthest, r1);
     float i0, i1;
@@ -1140,10 +1144,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
           }
           acc.add(xj, 4);
         }
-        for (; k > 0; --k, e += kBlock) {
-          const uint32_t l = e[0];
-          const R4<R> xj[4] = {R4<R>{s_px[l], s_py[l], s_pz[l], R(0)}};
-          acc.add(xj, 1);
+        if (k > 0) {
+          R4<R> xj[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t l = e[min(u, k - 1) * kBlock];
+            xj[u] = R4<R>{s_px[l], s_py[l], s_pz[l], R(0)};
+          }
+          acc.add(xj, k);
         }
       } else {
         for (int k = 0; k < stored; ++k) {
@@ -1198,50 +1206,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
 // ---------------------------------------------------------------------------
 // 5. boundary samples: sample boundaries (sorted sample grid) and volume maps
 // ---------------------------------------------------------------------------
-// Aggregates over a particle's boundary neighbors b (all boundaries):
-//   bW  = sum V_b W_ib                                  (volume)
-//   bG  = {sum V_b gradW_ib, sum V_b (v_b . gradW_ib)}  (pressure, source, a_ii)
-//   bGu = {sum gradW_ib, -}                             (SESPHwSplitting)
-template <class R>
-__global__ void __launch_bounds__(kBlock) k_sample_aggregate(
-    Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, SampleGrid<R> G,
-    R* __restrict__ bW, R4<R>* __restrict__ bG, R4<R>* __restrict__ bGu, StepParams<R> P) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int cnt = 0;
-  if (i < sc->n_active) {
-    const R4<R> xi = pos[i];
-    const int cx = cell_coord((double)xi.x, P.range), cy = cell_coord((double)xi.y, P.range),
-              cz = cell_coord((double)xi.z, P.range);
-    R w = 0, wc = 0;
-    R gx = 0, gy = 0, gz = 0, gv = 0, ux = 0, uy = 0, uz = 0;
-    for (int dz = -1; dz <= 1; ++dz)
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const uint32_t k = morton_key(cx + dx, cy + dy, cz + dz, G.mask);
-          const uint32_t b = G.start[k], e = G.start[k + 1];
-          for (uint32_t s = b; s < e; ++s) {
-            const R4<R> xs = G.xb[s];
-            if (!in_range(xi, xs, P.range, P.range2_lo, P.range2_hi)) continue;
-            ++cnt;
-            const R rx = xi.x - xs.x, ry = xi.y - xs.y, rz = xi.z - xs.z;
-            R kw, f;
-            kernel_w_and_grad(rx * rx + ry * ry + rz * rz, P.k, kw, f);
-            kahan_add(w, wc, xs.w * kw);
-            const R vf = xs.w * f;
-            gx += vf * rx; gy += vf * ry; gz += vf * rz;
-            const R4<R> vs = G.vb[s];
-            gv += vf * (vs.x * rx + vs.y * ry + vs.z * rz);
-            ux += f * rx; uy += f * ry; uz += f * rz;
-          }
-        }
-    bW[i] = w;
-    bG[i] = R4<R>{gx, gy, gz, gv};
-    bGu[i] = R4<R>{ux, uy, uz, R(0)};
-  }
-  for (int o = 16; o > 0; o >>= 1) cnt = max(cnt, __shfl_down_sync(0xffffffffu, cnt, o));
-  if ((threadIdx.x & 31) == 0 && cnt > 0) atomicMax(&sc->max_bnbrs, cnt);
-}
-
 // Serendipity reference nodes (discretization.rs:267-300): lattice offsets and
 // node kind (0 corner, 1/2/3 edge along x/y/z) with reference coordinates.
 __constant__ double c_ser_ref[32][3];
@@ -1331,7 +1295,7 @@ __global__ void __launch_bounds__(kBlock) k_vm_near(
     Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const VMDesc* __restrict__ vms, int nvm,
     const Body* __restrict__ bodies, uint32_t* __restrict__ near_list, R4<R>* __restrict__ vmx,
     R4<R>* __restrict__ vmv, R* __restrict__ bW, R4<R>* __restrict__ bG, R4<R>* __restrict__ bGu,
-    StepParams<R> P) {
+    R4<R>* __restrict__ bA, StepParams<R> P) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= sc->n_active) return;
   const R4<R> xr = pos[i];
@@ -1348,14 +1312,11 @@ __global__ void __launch_bounds__(kBlock) k_vm_near(
     near_list[atomicAdd(&sc->vm_near, 1u)] = (uint32_t)i;
     return;
   }
-  for (int b = 0; b < nvm; ++b) {
-    const size_t o = (size_t)b * P.Np + i;
-    vmx[o] = R4<R>{R(0), R(0), R(0), R(0)};
-    vmv[o] = R4<R>{R(0), R(0), R(0), R(0)};
-  }
+  for (int b = 0; b < nvm; ++b) vmv[(size_t)b * P.Np + i] = R4<R>{R(0), R(0), R(0), R(0)};  // kind 0: vmx is not read
   bW[i] = R(0);
   bG[i] = R4<R>{R(0), R(0), R(0), R(0)};
-  bGu[i] = R4<R>{R(0), R(0), R(0), R(0)};
+  if (bGu) bGu[i] = R4<R>{R(0), R(0), R(0), R(0)};
+  bA[i] = R4<R>{R(0), R(0), R(0), R(0)};
 }
 
 // Normal-mode sample of volume map D for the world-frame point p
@@ -1389,16 +1350,57 @@ __device__ __forceinline__ bool vm_normal_sample(const VMDesc& D, const Body* bo
   return true;
 }
 
+// The four tangential viscosity samples of a volume-map sample x_b of particle
+// position xi: x_b +- r/2 t1, x_b +- r/2 t2 (volume_map_boundary.rs:1344-1377);
+// kind as in vmv.w.
+template <class R>
+struct TangentSamples {
+  V3<R> xb, d1, d2;
+  __device__ __forceinline__ TangentSamples(const R4<R>& xi, const R4<R>& x, R kind, double range)
+      : xb{x.x, x.y, x.z} {
+    const V3<R> u = xb - V3<R>{xi.x, xi.y, xi.z};
+    const V3<R> tmp = kind == R(1) ? V3<R>{1, 0, 0} : V3<R>{0, 1, 0};
+    V3<R> t1 = cross(u, tmp);
+    V3<R> t2 = cross(u, t1);
+    t1 = (R(1) / sqrt(dot(t1, t1))) * t1;
+    t2 = (R(1) / sqrt(dot(t2, t2))) * t2;
+    const R d = R(0.5) * (R)range;
+    d1 = d * t1;
+    d2 = d * t2;
+  }
+  __device__ __forceinline__ V3<R> at(int k) const {
+    return k == 0 ? xb + d1 : k == 1 ? xb - d1 : k == 2 ? xb + d2 : xb - d2;
+  }
+};
+template <class R>
+__device__ __forceinline__ V3<R> body_velocity_r(const Body* bodies, int body, const V3<R>& q) {
+  if (body < 0) return V3<R>{0, 0, 0};
+  const double p[3] = {(double)q.x, (double)q.y, (double)q.z};
+  double v[3];
+  body_velocity_at(bodies[body], p, v);
+  return V3<R>{(R)v[0], (R)v[1], (R)v[2]};
+}
+// Boundary viscosity acceleration from one sample: its factor along r = xi - x.
+template <class R>
+__device__ __forceinline__ R boundary_viscosity(const V3<R>& r, const V3<R>& dv, R V, const StepParams<R>& P) {
+  const R r2 = r.x * r.x + r.y * r.y + r.z * r.z;
+  const R f = kernel_grad_factor(r2, P.k);
+  const R vr = dv.x * r.x + dv.y * r.y + dv.z * r.z;
+  return P.visc_b * V * vr / (r2 + P.eps_visc) * f;
+}
+
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_vm_sample(
     Scalars* __restrict__ sc, const uint32_t* __restrict__ near_list, const R4<R>* __restrict__ pos,
-    const VMDesc* __restrict__ vms, int nvm, const Body* __restrict__ bodies, R4<R>* __restrict__ vmx,
-    R4<R>* __restrict__ vmv, R* __restrict__ bW, R4<R>* __restrict__ bG, R4<R>* __restrict__ bGu,
-    StepParams<R> P) {
+    const R4<R>* __restrict__ vel, const VMDesc* __restrict__ vms, int nvm, const Body* __restrict__ bodies,
+    R4<R>* __restrict__ vmx, R4<R>* __restrict__ vmv, R* __restrict__ bW, R4<R>* __restrict__ bG,
+    R4<R>* __restrict__ bGu, R4<R>* __restrict__ bA, uint32_t* __restrict__ touch, StepParams<R> P) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int)sc->vm_near) return;
   const int i = (int)near_list[t];
-  const R4<R> xr = pos[i];
+  const R4<R> xr = pos[i], vi = vel[i];
+  bool dyn = false;
+  R sx = 0, sy = 0, sz = 0;  // viscosity
   const double p[3] = {(double)xr.x, (double)xr.y, (double)xr.z};
   const double range = P.range;
   const double ball = 4.0 / 3.0 * 3.14159265358979323846 * (range * range * range);
@@ -1429,12 +1431,28 @@ __global__ void __launch_bounds__(kBlock) k_vm_sample(
       ux += (R)(f * rx); uy += (R)(f * ry); uz += (R)(f * rz);
     }
     const size_t o = (size_t)b * P.Np + i;
-    vmx[o] = R4<R>{(R)xb[0], (R)xb[1], (R)xb[2], (R)vol};
+    const R4<R> xx{(R)xb[0], (R)xb[1], (R)xb[2], (R)vol};
+    vmx[o] = xx;
     vmv[o] = R4<R>{(R)vb[0], (R)vb[1], (R)vb[2], (R)kind};
+    if (kind == 0) continue;
+    // viscosity: four tangential samples of a quarter of the volume each
+    const TangentSamples<R> ts(xr, xx, (R)kind, range);
+    const bool moves = D.body >= 0 && bodies[D.body].dynamic;
+    dyn |= moves;
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      const V3<R> q = ts.at(k);
+      const V3<R> vq = body_velocity_r(bodies, D.body, q);
+      const V3<R> r{xr.x - q.x, xr.y - q.y, xr.z - q.z};
+      const R s = boundary_viscosity(r, V3<R>{vi.x - vq.x, vi.y - vq.y, vi.z - vq.z}, R(0.25) * xx.w, P);
+      sx += s * r.x; sy += s * r.y; sz += s * r.z;
+    }
   }
   bW[i] = w;
   bG[i] = R4<R>{gx, gy, gz, gv};
-  bGu[i] = R4<R>{ux, uy, uz, R(0)};
+  if (bGu) bGu[i] = R4<R>{ux, uy, uz, R(0)};
+  bA[i] = R4<R>{sx, sy, sz, R(0)};
+  if (dyn) touch[atomicAdd(&sc->n_touch, 1u)] = (uint32_t)i;
 }
 
 // ScalarQuantity at evaluation positions (sph/mod.rs:241-341 with the sums
@@ -1549,102 +1567,36 @@ struct BoundaryArgs {
   const R* bW;
   const R4<R>* bG;
   const R4<R>* bGu;
+  const R4<R>* bA;
   double* body_partials;  // [gridDim][kMaxBodies][6] reaction force/torque partials
+  const uint32_t* touch;  // particles with a neighbor on a dynamic body (sc->n_touch of them)
   int nbodies;
 };
 
-// Calls fn(xb, vb, Vb, body) for every boundary neighbor of the viscosity
-// request mode: sample-boundary neighbors, or the 4 tangential volume-map
-// samples at x_b +- r/2 t1, x_b +- r/2 t2 (volume_map_boundary.rs:1344-1377).
-template <class R, class Fn>
-__device__ __forceinline__ void for_each_visc_sample(const BoundaryArgs<R>& B, const R4<R>& xi,
-                                                     int i, const StepParams<R>& P, Fn&& fn) {
-  if (B.kind == 1) {
-    const int cx = cell_coord((double)xi.x, P.range), cy = cell_coord((double)xi.y, P.range),
-              cz = cell_coord((double)xi.z, P.range);
-    for (int dz = -1; dz <= 1; ++dz)
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const uint32_t k = morton_key(cx + dx, cy + dy, cz + dz, B.grid.mask);
-          const uint32_t b = B.grid.start[k], e = B.grid.start[k + 1];
-          for (uint32_t s = b; s < e; ++s) {
-            const R4<R> xs = B.grid.xb[s];
-            if (!in_range(xi, xs, P.range, P.range2_lo, P.range2_hi)) continue;
-            const R4<R> vs = B.grid.vb[s];
-            fn(V3<R>{xs.x, xs.y, xs.z}, V3<R>{vs.x, vs.y, vs.z}, xs.w, (int)B.grid.bid[s]);
-          }
-        }
-  } else if (B.kind == 2) {
-    for (int b = 0; b < B.nvm; ++b) {
-      const size_t o = (size_t)b * P.Np + i;
-      const R4<R> vv = B.vmv[o];
-      if (vv.w == R(0)) continue;
-      const R4<R> xx = B.vmx[o];
-      const V3<R> xb{xx.x, xx.y, xx.z};
-      const V3<R> u = xb - V3<R>{xi.x, xi.y, xi.z};
-      const V3<R> tmp = vv.w == R(1) ? V3<R>{1, 0, 0} : V3<R>{0, 1, 0};
-      V3<R> t1 = cross(u, tmp);
-      V3<R> t2 = cross(u, t1);
-      t1 = (R(1) / sqrt(dot(t1, t1))) * t1;
-      t2 = (R(1) / sqrt(dot(t2, t2))) * t2;
-      const R d = R(0.5) * (R)P.range;
-      const V3<R> q[4] = {xb + d * t1, xb - d * t1, xb + d * t2, xb - d * t2};
-      const int body = B.vms[b].body;
-      for (int k = 0; k < 4; ++k) {
-        V3<R> vq{0, 0, 0};
-        if (body >= 0) {
-          const double pq[3] = {(double)q[k].x, (double)q[k].y, (double)q[k].z};
-          double vo[3];
-          body_velocity_at(B.bodies[body], pq, vo);
-          vq = V3<R>{(R)vo[0], (R)vo[1], (R)vo[2]};
-        }
-        fn(q[k], vq, R(0.25) * xx.w, body);
-      }
-    }
-  }
-}
-
-// Calls fn(xb, Vb, body) for every boundary neighbor of the Normal mode.
-template <class R, class Fn>
-__device__ __forceinline__ void for_each_normal_sample(const BoundaryArgs<R>& B, const R4<R>& xi,
-                                                       int i, const StepParams<R>& P, Fn&& fn) {
-  if (B.kind == 1) {
-    const int cx = cell_coord((double)xi.x, P.range), cy = cell_coord((double)xi.y, P.range),
-              cz = cell_coord((double)xi.z, P.range);
-    for (int dz = -1; dz <= 1; ++dz)
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const uint32_t k = morton_key(cx + dx, cy + dy, cz + dz, B.grid.mask);
-          const uint32_t b = B.grid.start[k], e = B.grid.start[k + 1];
-          for (uint32_t s = b; s < e; ++s) {
-            const R4<R> xs = B.grid.xb[s];
-            if (!in_range(xi, xs, P.range, P.range2_lo, P.range2_hi)) continue;
-            fn(V3<R>{xs.x, xs.y, xs.z}, xs.w, (int)B.grid.bid[s]);
-          }
-        }
-  } else if (B.kind == 2) {
-    for (int b = 0; b < B.nvm; ++b) {
-      const size_t o = (size_t)b * P.Np + i;
-      if (B.vmv[o].w == R(0)) continue;
-      const R4<R> xx = B.vmx[o];
-      fn(V3<R>{xx.x, xx.y, xx.z}, xx.w, B.vms[b].body);
-    }
-  }
-}
-
 // Per-block rigid-body force/torque accumulation in f64 (shared memory),
 // flushed to per-block partials that a fixed-order kernel reduces.
+// A thread sums for one body at a time and adds to the block's sums when the
+// next force is another body's, and at the end.
 struct BodyAccum {
   double* sh;  // [kMaxBodies][6]
-  __device__ void add(const Body* bodies, int body, const double F[3], const double x[3]) {
-    const Body& b = bodies[body];
-    const double r[3] = {x[0] - b.com[0], x[1] - b.com[1], x[2] - b.com[2]};
-    atomicAdd(&sh[body * 6 + 0], F[0]);
-    atomicAdd(&sh[body * 6 + 1], F[1]);
-    atomicAdd(&sh[body * 6 + 2], F[2]);
-    atomicAdd(&sh[body * 6 + 3], r[1] * F[2] - r[2] * F[1]);
-    atomicAdd(&sh[body * 6 + 4], r[2] * F[0] - r[0] * F[2]);
-    atomicAdd(&sh[body * 6 + 5], r[0] * F[1] - r[1] * F[0]);
+  int body = -1;
+  double a[6] = {0, 0, 0, 0, 0, 0};
+  __device__ __forceinline__ void add(const Body* bodies, int b, const double F[3], const double x[3]) {
+    if (b != body) flush();
+    body = b;
+    const double* com = bodies[b].com;
+    const double r[3] = {x[0] - com[0], x[1] - com[1], x[2] - com[2]};
+    a[0] += F[0]; a[1] += F[1]; a[2] += F[2];
+    a[3] += r[1] * F[2] - r[2] * F[1];
+    a[4] += r[2] * F[0] - r[0] * F[2];
+    a[5] += r[0] * F[1] - r[1] * F[0];
+  }
+  __device__ __forceinline__ void flush() {
+    for (int k = 0; k < 6; ++k) {
+      if (body >= 0) atomicAdd(&sh[body * 6 + k], a[k]);
+      a[k] = 0.0;
+    }
+    body = -1;
   }
 };
 
@@ -1656,6 +1608,245 @@ __device__ __forceinline__ void body_accum_flush(double* sh, int nbodies, double
   __syncthreads();
   for (int t = threadIdx.x; t < nbodies * 6; t += blockDim.x)
     partials[(size_t)blockIdx.x * kMaxBodies * 6 + t] = sh[t];
+}
+
+// ---------------------------------------------------------------------------
+// 5a. sample boundaries: everything a particle takes from its boundary
+// samples, in one pass over them (all boundaries):
+//   bW  = sum V_b W_ib                                  (volume)
+//   bG  = {sum V_b gradW_ib, sum V_b (v_b . gradW_ib)}  (pressure, source, a_ii)
+//   bGu = {sum gradW_ib, -}                             (SESPHwSplitting only)
+//   bA  = {boundary viscosity acceleration, -}
+// and the list of the particles with a neighbor on a dynamic body.
+//
+// A warp takes one cell at a time (a block holds eight warps for the cells of
+// kSampleBlock particles, about as many): 27 lanes read the stencil's bucket
+// bounds at once, and a cell without samples around it (most of them) is
+// done. Otherwise its candidates are staged in shared memory, and 4 or 8 lanes
+// share them for every particle of the cell. A lane first tests its
+// candidates into a mask, then sums over the set bits. The kernel values go
+// through shared memory to one lane, which sums them in sample order (the
+// volume's compensated sum keeps its bits whatever the split).
+//
+// What bounds it: latency. With one thread per particle walking 27 buckets,
+// in this pass and again for the viscosity, scenes of 5 to 195 thousand
+// particles took 63-72 us here and 75-105 us more in the acceleration pass;
+// in this form 23-36 us here and 11-36 us there.
+// ---------------------------------------------------------------------------
+constexpr int kSampleBlock = 64;   // particles per block of kBlock threads
+constexpr int kSampleChunk = 96;   // candidates staged at a time
+template <class R>
+struct SampleStage {  // per warp
+  R4<R> x[kSampleChunk], v[kSampleChunk];
+  uint32_t s[kSampleChunk];
+  R w[8][kSampleChunk];  // per particle: kernel values, -1 out of range
+};
+
+template <class R, bool SPLIT>
+__global__ void __launch_bounds__(kBlock) k_sample_boundary(
+    Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const R4<R>* __restrict__ vel, SampleGrid<R> G,
+    const Body* __restrict__ bodies, int any_dynamic, R* __restrict__ bW, R4<R>* __restrict__ bG,
+    R4<R>* __restrict__ bGu, R4<R>* __restrict__ bA, uint32_t* __restrict__ touch, StepParams<R> P) {
+  extern __shared__ __align__(32) unsigned char dsm[];
+  __shared__ uint32_t s_key[kSampleBlock], s_heads[kSampleBlock / 32];
+  __shared__ uint8_t s_head[kSampleBlock + 1], s_near[kSampleBlock];  // per cell: first particle; it has candidates
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i0 = blockIdx.x * kSampleBlock, i = i0 + tid;
+  const int m = min(kSampleBlock, sc->n_active - i0);  // this block's particles
+  if (m <= 0) return;
+  if (tid < kSampleBlock) s_key[tid] = tid < m ? lane_key(pos[i].w) : 0u;
+  __syncthreads();
+  const bool head = tid < m && (tid == 0 || s_key[tid - 1] != s_key[tid]);
+  const uint32_t heads = __ballot_sync(0xffffffffu, head);
+  if (lane == 0 && warp < kSampleBlock / 32) s_heads[warp] = heads;
+  __syncthreads();
+  const int nheads = __popc(s_heads[0]) + __popc(s_heads[1]);
+  const int rank = (warp == 1 ? __popc(s_heads[0]) : 0) + __popc(heads & ((2u << lane) - 1u)) - 1;  // this particle's cell
+  if (head) s_head[rank] = (uint8_t)tid;
+  if (tid == 0) s_head[nheads] = (uint8_t)m;
+  __syncthreads();
+  SampleStage<R>& T = reinterpret_cast<SampleStage<R>*>(dsm)[warp];
+  int most = 0;
+  for (int h = warp; h < nheads; h += kBlock / 32) {
+    const int p0 = s_head[h], np = s_head[h + 1] - p0;
+    const uint32_t ck = s_key[p0];
+    uint32_t first = 0, len = 0;
+    if (lane < 27) {
+      const uint32_t k = morton_key((int)gather3(ck) + lane % 3 - 1, (int)gather3(ck >> 1) + (lane / 3) % 3 - 1,
+                                    (int)gather3(ck >> 2) + lane / 9 - 1, G.mask);
+      first = G.start[k];
+      len = G.start[k + 1] - first;
+    }
+    const bool near = __any_sync(0xffffffffu, len != 0);
+    if (lane == 0) s_near[h] = near;
+    if (!near) continue;
+    uint32_t end = len;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += y;
+    }
+    const uint32_t C = __shfl_sync(0xffffffffu, end, 31), begin = end - len;
+    const int S = np <= 4 ? 8 : 4;  // lanes per particle
+    const int sub = lane & (S - 1), row = lane / S;
+    for (int g = 0; g < np; g += 32 / S) {
+      const int p = g + row;
+      const bool mine = p < np;
+      const int ip = i0 + p0 + (mine ? p : 0);
+      const R4<R> xi = pos[ip], vi = vel[ip];
+      R w = 0, wc = 0;
+      R gx = 0, gy = 0, gz = 0, gv = 0, ux = 0, uy = 0, uz = 0, sx = 0, sy = 0, sz = 0;
+      int cnt = 0;
+      bool dyn = false;
+      for (uint32_t c0 = 0; c0 < C; c0 += kSampleChunk) {
+        const int nc = (int)min(C - c0, (uint32_t)kSampleChunk);
+        __syncwarp();
+        for (uint32_t c = max(begin, c0); c < min(end, c0 + (uint32_t)nc); ++c) T.s[c - c0] = first + (c - begin);
+        __syncwarp();
+        for (int c = lane; c < nc; c += 32) {
+          const uint32_t s = T.s[c];
+          T.x[c] = G.xb[s];
+          T.v[c] = G.vb[s];
+        }
+        __syncwarp();
+        uint32_t in = 0;  // candidate sub + S q at bit q
+        for (int c = sub, q = 0; c < nc; c += S, ++q) {
+          const bool hit = mine && in_range(xi, T.x[c], P.range, P.range2_lo, P.range2_hi);
+          if (hit) in |= 1u << q;
+          else T.w[row][c] = R(-1);
+        }
+        cnt += __popc(in);
+        while (in) {
+          const int q = __ffs((int)in) - 1;
+          in &= in - 1;
+          const int c = sub + S * q;
+          const R4<R> xs = T.x[c], vs = T.v[c];
+          const R rx = xi.x - xs.x, ry = xi.y - xs.y, rz = xi.z - xs.z;
+          const R r2 = rx * rx + ry * ry + rz * rz;
+          R kw, f;
+          kernel_w_and_grad(r2, P.k, kw, f);
+          T.w[row][c] = kw;
+          const R vf = xs.w * f;
+          gx += vf * rx; gy += vf * ry; gz += vf * rz;
+          gv += vf * (vs.x * rx + vs.y * ry + vs.z * rz);
+          if (SPLIT) { ux += f * rx; uy += f * ry; uz += f * rz; }
+          const R vr = (vi.x - vs.x) * rx + (vi.y - vs.y) * ry + (vi.z - vs.z) * rz;
+          const R s = P.visc_b * xs.w * vr / (r2 + P.eps_visc) * f;
+          sx += s * rx; sy += s * ry; sz += s * rz;
+          if (any_dynamic) dyn |= bodies[G.bid[T.s[c]]].dynamic != 0;
+        }
+        __syncwarp();
+        if (sub == 0) {
+#pragma unroll 8
+          for (int c = 0; c < nc; ++c) {
+            const R kw = T.w[row][c], V = T.x[c].w;
+            R w2 = w, c2 = wc;
+            kahan_add(w2, c2, V * kw);
+            w = kw >= R(0) ? w2 : w;
+            wc = kw >= R(0) ? c2 : wc;
+          }
+        }
+      }
+      for (int o = S >> 1; o > 0; o >>= 1) {
+        gx += __shfl_xor_sync(0xffffffffu, gx, o); gy += __shfl_xor_sync(0xffffffffu, gy, o);
+        gz += __shfl_xor_sync(0xffffffffu, gz, o); gv += __shfl_xor_sync(0xffffffffu, gv, o);
+        if (SPLIT) {
+          ux += __shfl_xor_sync(0xffffffffu, ux, o); uy += __shfl_xor_sync(0xffffffffu, uy, o);
+          uz += __shfl_xor_sync(0xffffffffu, uz, o);
+        }
+        sx += __shfl_xor_sync(0xffffffffu, sx, o); sy += __shfl_xor_sync(0xffffffffu, sy, o);
+        sz += __shfl_xor_sync(0xffffffffu, sz, o);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+        if (any_dynamic) dyn |= __shfl_xor_sync(0xffffffffu, (int)dyn, o) != 0;
+      }
+      most = max(most, cnt);
+      if (mine && sub == 0) {
+        bW[ip] = w;
+        bG[ip] = R4<R>{gx, gy, gz, gv};
+        if (SPLIT) bGu[ip] = R4<R>{ux, uy, uz, R(0)};
+        bA[ip] = R4<R>{sx, sy, sz, R(0)};
+        if (dyn) touch[atomicAdd(&sc->n_touch, 1u)] = (uint32_t)ip;
+      }
+    }
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 0 && most > 0) atomicMax(&sc->max_bnbrs, most);
+  __syncthreads();
+  if (tid < m && !s_near[rank]) {
+    bW[i] = R(0);
+    bG[i] = R4<R>{R(0), R(0), R(0), R(0)};
+    if (SPLIT) bGu[i] = R4<R>{R(0), R(0), R(0), R(0)};
+    bA[i] = R4<R>{R(0), R(0), R(0), R(0)};
+  }
+}
+
+// Reactions on dynamic bodies, once the pressures are known: for every
+// particle of the touch list and each of its boundary neighbors on a dynamic
+// body, the viscosity's F = -m_i a_ib (non_pressure_accelerations.rs) and the
+// pressure's F = 2 gamma_p V_i V_b p_i gradW_ib (pressure_solver/mod.rs:
+// 160-195). A warp per particle: its lanes take the stencil's buckets (sample
+// boundaries) or the volume maps. (Inside the acceleration passes, which
+// walked every particle's samples twice for it, a tank of 276 thousand
+// particles with eight bodies took 591 us there, now 56 us and 21 us here.)
+template <class R>
+__global__ void __launch_bounds__(kBlock) k_body_react(const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv,
+                                                      const R4<R>* __restrict__ vel, const R* __restrict__ press,
+                                                      BoundaryArgs<R> B, StepParams<R> P) {
+  __shared__ double sh_body[kMaxBodies * 6];
+  body_accum_init(sh_body, B.nbodies);
+  BodyAccum acc_b{sh_body};
+  const int lane = threadIdx.x & 31;
+  const uint32_t warps = gridDim.x * (kBlock / 32);
+  for (uint32_t t = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); t < sc->n_touch; t += warps) {
+    const int i = (int)B.touch[t];
+    const R4<R> xi = xv[i], vi = vel[i];
+    const R pi = press[i];
+    auto viscous = [&](const V3<R>& x, const V3<R>& v, R V, int body) {
+      const V3<R> r{xi.x - x.x, xi.y - x.y, xi.z - x.z};
+      const R s = boundary_viscosity(r, V3<R>{vi.x - v.x, vi.y - v.y, vi.z - v.z}, V, P);
+      const double mi = (double)vi.w;
+      const double F[3] = {-mi * (double)(s * r.x), -mi * (double)(s * r.y), -mi * (double)(s * r.z)};
+      const double xl[3] = {(double)x.x, (double)x.y, (double)x.z};
+      acc_b.add(B.bodies, body, F, xl);
+    };
+    auto pressure = [&](const V3<R>& x, R V, int body) {
+      const R rx = xi.x - x.x, ry = xi.y - x.y, rz = xi.z - x.z;
+      const R f = kernel_grad_factor(rx * rx + ry * ry + rz * rz, P.k);
+      const double c2 = 2.0 * (double)P.gamma_p * (double)xi.w * (double)V * (double)pi * (double)f;
+      const double F[3] = {c2 * rx, c2 * ry, c2 * rz};
+      const double xl[3] = {(double)x.x, (double)x.y, (double)x.z};
+      acc_b.add(B.bodies, body, F, xl);
+    };
+    if (B.kind == 1 && lane < 27) {
+      const uint32_t k = morton_key(cell_coord((double)xi.x, P.range) + lane % 3 - 1,
+                                    cell_coord((double)xi.y, P.range) + (lane / 3) % 3 - 1,
+                                    cell_coord((double)xi.z, P.range) + lane / 9 - 1, B.grid.mask);
+      const uint32_t e = B.grid.start[k + 1];
+      for (uint32_t s = B.grid.start[k]; s < e; ++s) {
+        const int body = (int)B.grid.bid[s];
+        if (!B.bodies[body].dynamic) continue;
+        const R4<R> xs = B.grid.xb[s], vs = B.grid.vb[s];
+        if (!in_range(xi, xs, P.range, P.range2_lo, P.range2_hi)) continue;
+        const V3<R> x{xs.x, xs.y, xs.z};
+        viscous(x, V3<R>{vs.x, vs.y, vs.z}, xs.w, body);
+        pressure(x, xs.w, body);
+      }
+    } else if (B.kind == 2 && lane < B.nvm) {
+      const size_t o = (size_t)lane * P.Np + i;
+      const int body = B.vms[lane].body;
+      const R kind = B.vmv[o].w;
+      if (body >= 0 && B.bodies[body].dynamic && kind != R(0)) {
+        const R4<R> xs = B.vmx[o];
+        const TangentSamples<R> ts(xi, xs, kind, P.range);
+        for (int k = 0; k < 4; ++k) {
+          const V3<R> q = ts.at(k);
+          viscous(q, body_velocity_r(B.bodies, body, q), R(0.25) * xs.w, body);
+        }
+        pressure(V3<R>{xs.x, xs.y, xs.z}, xs.w, body);
+      }
+    }
+  }
+  acc_b.flush();
+  body_accum_flush(sh_body, B.nbodies, B.body_partials);
 }
 
 // ---------------------------------------------------------------------------
@@ -1802,10 +1993,7 @@ __global__ void __launch_bounds__(kBlock) k_accel(
     const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv, const R4<R>* __restrict__ vel,
     NbrArgs N, BoundaryArgs<R> B, R4<R>* __restrict__ acc, R4<R>* __restrict__ vstar,
     R* __restrict__ press, int write_vstar, StepParams<R> P) {
-  __shared__ double sh_body[kMaxBodies * 6];
   extern __shared__ __align__(32) unsigned char dsm[];
-  const bool bodies = B.any_dynamic != 0;
-  if (bodies) body_accum_init(sh_body, B.nbodies);
   const HaloView H = halo_view(N);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool act = i < sc->n_active;
@@ -1856,36 +2044,12 @@ __global__ void __launch_bounds__(kBlock) k_accel(
     else
       sweep_groups(L, [&](uint32_t l) { const uint32_t g = H.idx[l]; return XV<R>{xv[g], vel[g]}; }, pair);
     if (B.kind != 0) {
-      BodyAccum acc_b{sh_body};
-      for_each_visc_sample<R>(B, xi, i, P, [&](V3<R> xb, V3<R> vb, R Vb, int body) {
-        const R rx = xi.x - xb.x, ry = xi.y - xb.y, rz = xi.z - xb.z;
-        const R r2 = rx * rx + ry * ry + rz * rz;
-        const R f = kernel_grad_factor(r2, P.k);
-        const R vr = (vi.x - vb.x) * rx + (vi.y - vb.y) * ry + (vi.z - vb.z) * rz;
-        const R s = P.visc_b * Vb * vr / (r2 + P.eps_visc) * f;
-        sx += s * rx; sy += s * ry; sz += s * rz;
-        if (bodies && body >= 0 && B.bodies[body].dynamic) {
-          const double F[3] = {-(double)mi * (double)(s * rx), -(double)mi * (double)(s * ry),
-                               -(double)mi * (double)(s * rz)};
-          const double xl[3] = {(double)xb.x, (double)xb.y, (double)xb.z};
-          acc_b.add(B.bodies, body, F, xl);
-        }
-      });
+      const R4<R> bv = B.bA[i];
+      sx += bv.x; sy += bv.y; sz += bv.z;
       if (PRESS == 1) {
         const R4<R> g = B.bG[i];
         const R c = R(2) * P.gamma_p * pi;  // boundary: 2 gamma V_i V_b p_i gradW / m_i
         px += c * g.x; py += c * g.y; pz += c * g.z;
-        if (bodies) {
-          for_each_normal_sample<R>(B, xi, i, P, [&](V3<R> xb, R Vb, int body) {
-            if (body < 0 || !B.bodies[body].dynamic) return;
-            const R rx = xi.x - xb.x, ry = xi.y - xb.y, rz = xi.z - xb.z;
-            const R f = kernel_grad_factor(rx * rx + ry * ry + rz * rz, P.k);
-            const double c2 = 2.0 * (double)P.gamma_p * (double)Vi * (double)Vb * (double)pi * (double)f;
-            const double F[3] = {c2 * rx, c2 * ry, c2 * rz};
-            const double xl[3] = {(double)xb.x, (double)xb.y, (double)xb.z};
-            acc_b.add(B.bodies, body, F, xl);
-          });
-        }
       }
     }
     const R vm = Vi / mi;
@@ -1899,24 +2063,17 @@ __global__ void __launch_bounds__(kBlock) k_accel(
     }
     if (PRESS == 1) press[i] = pi;
   }
-  if (bodies) body_accum_flush(sh_body, B.nbodies, B.body_partials);
 }
 
 // ---------------------------------------------------------------------------
 // 7. pressure acceleration from stored pressures (pressure_solver/mod.rs:121-195)
 // ---------------------------------------------------------------------------
-// MODE: 1 -> acc += accel (reaction forces if mirror)
-//       2 -> acc  = accel (reaction forces if mirror)
-// (the Jacobi sweep's own pressure accelerations are k_sweep_accel)
-template <class R, int MODE>
+// acc += accel (the solvers with Jacobi sweeps take it from k_sweep_accel)
+template <class R>
 __global__ void __launch_bounds__(kBlock) k_pressure_accel(
     const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv, const R4<R>* __restrict__ vel,
-    const R* __restrict__ press, NbrArgs N, BoundaryArgs<R> B, R4<R>* __restrict__ out, int mirror,
-    StepParams<R> P) {
-  __shared__ double sh_body[kMaxBodies * 6];
+    const R* __restrict__ press, NbrArgs N, BoundaryArgs<R> B, R4<R>* __restrict__ out, StepParams<R> P) {
   extern __shared__ __align__(32) unsigned char dsm[];
-  const bool bodies = mirror && B.any_dynamic != 0;
-  if (bodies) body_accum_init(sh_body, B.nbodies);
   const HaloView H = halo_view(N);
   // this particle's own data and first list batch travel while the halo stages
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1955,30 +2112,12 @@ __global__ void __launch_bounds__(kBlock) k_pressure_accel(
       const R4<R> g = B.bG[i];
       const R c = R(2) * P.gamma_p * pi;
       px += c * g.x; py += c * g.y; pz += c * g.z;
-      if (bodies) {
-        BodyAccum acc_b{sh_body};
-        for_each_normal_sample<R>(B, xi, i, P, [&](V3<R> xb, R Vb, int body) {
-          if (body < 0 || !B.bodies[body].dynamic) return;
-          const R rx = xi.x - xb.x, ry = xi.y - xb.y, rz = xi.z - xb.z;
-          const R f = kernel_grad_factor(rx * rx + ry * ry + rz * rz, P.k);
-          const double c2 = 2.0 * (double)P.gamma_p * (double)Vi * (double)Vb * (double)pi * (double)f;
-          const double F[3] = {c2 * rx, c2 * ry, c2 * rz};
-          const double xl[3] = {(double)xb.x, (double)xb.y, (double)xb.z};
-          acc_b.add(B.bodies, body, F, xl);
-        });
-      }
     }
     const R vm = Vi / mi;
-    const R4<R> a = R4<R>{-vm * px, -vm * py, -vm * pz, R(0)};
-    if (MODE == 1) {
-      R4<R> o = out[i];
-      o.x += a.x; o.y += a.y; o.z += a.z;
-      out[i] = o;
-    } else {
-      out[i] = a;
-    }
+    R4<R> o = out[i];
+    o.x += -vm * px; o.y += -vm * py; o.z += -vm * pz;
+    out[i] = o;
   }
-  if (bodies) body_accum_flush(sh_body, B.nbodies, B.body_partials);
 }
 
 // ---------------------------------------------------------------------------
@@ -2081,8 +2220,8 @@ __global__ void __launch_bounds__(kBlock) k_iisph_source_diag(
 // (f32: at most 48 registers, so five blocks share an SM; the records are
 // gathered two at a time to fit)
 // OUT 0: the records of pass B; OUT 1: acc += a_i, OUT 2: acc = a_i (the
-// final pressure acceleration of a solve, pressure_solver/mod.rs:121-195,
-// when no boundary takes reaction forces).
+// final pressure acceleration of a solve, pressure_solver/mod.rs:121-195; the
+// reaction on dynamic bodies is k_body_react).
 template <class R, int OUT = 0>
 __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_accel(
     const Scalars* __restrict__ sc, const R* __restrict__ press, const R4<R>* __restrict__ TA,

@@ -79,6 +79,7 @@ static void allow_smem(const void* fn, size_t bytes) {
 // the staging passes keep aside for their static arrays.
 constexpr size_t kMaxSmemPerBlock = 232448;
 constexpr size_t kStaticSmemReserve = 4096;
+constexpr int kReactBlocks = 2 * 148;  // most blocks of the body reaction pass
 static int blocks_for(long long n) { return (int)std::max(1LL, (n + kBlock - 1) / kBlock); }
 static size_t round_up(size_t n, size_t m) { return (n + m - 1) / m * m; }
 
@@ -295,7 +296,8 @@ class System : public SystemBase {
     any_dynamic_ = has_dyn;
     bodies_d_.alloc(std::max(1, nbodies_));
     if (nbodies_) copy_h2d(bodies_d_.p, bodies_.data(), (size_t)nbodies_);
-    body_partials_.alloc((size_t)blocks_for((long long)cap_) * kMaxBodies * 6);
+    if (any_dynamic_) body_partials_.alloc((size_t)kReactBlocks * kMaxBodies * 6);
+    if (any_dynamic_) touch_.alloc(cap_);
     // boundaries
     if (cfg_.boundary_handling == SPH_STATIC_SAMPLE_BOUNDARY && !h_sample_bid_.empty())
       init_sample_boundaries();
@@ -779,14 +781,14 @@ class System : public SystemBase {
   }
   size_t device_bytes() const override {
     size_t b = d_sc_.bytes() + d_meas_.bytes();
-    for (const auto* d : {&pos_, &pos2_, &vel_, &vel2_, &xv_, &acc_, &vstar_, &xq_, &xu_, &TA_, &TB_, &xint_, &vint_, &bG_, &bGu_,
+    for (const auto* d : {&pos_, &pos2_, &vel_, &vel2_, &xv_, &acc_, &vstar_, &xq_, &xu_, &TA_, &TB_, &xint_, &vint_, &bG_, &bGu_, &bA_,
                           &xb_, &xb2_, &vb_, &vb2_, &xbody_, &vmx_, &vmv_, &snap_pos_, &snap_vel_, &snap_acc_,
                           &snap_xint_, &snap_vint_})
       b += d->bytes();
     for (const auto* d : {&press_, &s_, &aii_, &bW_, &rho_pred_}) b += d->bytes();
     b += uu_.bytes() + SA_.bytes();
     b += nbr_.bytes();
-    for (const auto* d : {&ref_, &ref2_, &fid_, &fid2_, &key_, &slot_, &perm_, &halo_idx_, &halo_n_, &vm_near_, &ncnt_,
+    for (const auto* d : {&ref_, &ref2_, &fid_, &fid2_, &key_, &slot_, &perm_, &halo_idx_, &halo_n_, &vm_near_, &touch_, &ncnt_,
                           &count_, &start_,
                           &tile_sums_, &sbid_, &sbid2_, &sorig_, &sorig2_, &skey_, &sslot_, &sperm_, &scount_,
                           &sstart_, &snap_ref_, &snap_fid_})
@@ -850,7 +852,7 @@ class System : public SystemBase {
   std::vector<Pending> pending_;
 
   // particle state
-  DBuf<R4<R>> pos_, pos2_, vel_, vel2_, xv_, acc_, vstar_, xint_, vint_, bG_, bGu_;
+  DBuf<R4<R>> pos_, pos2_, vel_, vel2_, xv_, acc_, vstar_, xint_, vint_, bG_, bGu_, bA_;
   DBuf<R4<R>> xq_, xu_;      // IISPH sweep records {x, V p}, {x, V a_x}
   DBuf<R4<R>> TA_, TB_;      // IISPH per-solve constants of the two sweep passes
   DBuf<R2<R>> uu_, SA_;      // IISPH sweep records {V a_y, V a_z}; {s, a_ii}
@@ -890,6 +892,7 @@ class System : public SystemBase {
   DBuf<ContactScalars> contact_scalars_;
   DBuf<R4<R>> vmx_, vmv_;
   DBuf<uint32_t> vm_near_;  // particles near a volume map this step
+  DBuf<uint32_t> touch_;    // particles with a neighbor on a dynamic body this step
   DBuf<float> eval_pos_, eval_out_;  // quantity evaluation positions and values
   // surface reconstruction scratch (grown on demand, render frames only)
   DBuf<double> surf_vol_, surf_phi_, surf_vtx_;
@@ -993,7 +996,8 @@ class System : public SystemBase {
     ref_.alloc(c); ref2_.alloc(c); fid_.alloc(c); fid2_.alloc(c);
     key_.alloc(c); slot_.alloc(c); perm_.alloc(c); ncnt_.alloc(c);
     press_.alloc(c);
-    bW_.alloc(c); bG_.alloc(c); bGu_.alloc(c);
+    bW_.alloc(c); bG_.alloc(c); bA_.alloc(c);
+    if (cfg_.pressure_solver == SPH_SESPH_W_SPLITTING) bGu_.alloc(c);
     const bool needs_vstar = cfg_.pressure_solver != SPH_SESPH;
     if (needs_vstar) vstar_.alloc(c);
     if (cfg_.pressure_solver == SPH_IISPH || cfg_.pressure_solver == SPH_IISPH_W_OST) {
@@ -1007,7 +1011,7 @@ class System : public SystemBase {
     halo_idx_.alloc((size_t)blocks_for((long long)c) * (size_t)hcap_);
     ensure_partials(2 * (size_t)blocks_for((long long)c));
     press_.zero(stream_);
-    bW_.zero(stream_); bG_.zero(stream_); bGu_.zero(stream_);
+    bW_.zero(stream_); bG_.zero(stream_); bGu_.zero(stream_); bA_.zero(stream_);
   }
 
   void choose_grid() {
@@ -1385,15 +1389,21 @@ class System : public SystemBase {
     B.bW = bW_.p;
     B.bG = bG_.p;
     B.bGu = bGu_.p;
+    B.bA = bA_.p;
+    B.touch = touch_.p;
     B.body_partials = body_partials_.p;
     B.nbodies = nbodies_;
     return B;
   }
 
-  void body_reduce(int producer_blocks) {
+  // Boundary viscosity's and pressure's reactions on dynamic bodies.
+  void body_react() {
     if (!any_dynamic_) return;
+    const int nb = std::min(blocks_for((long long)cap_), kReactBlocks);
+    launch("body_react", k_body_react<R>, dim3(nb), dim3(kBlock), (const Scalars*)d_sc_.p, (const R4<R>*)xv_.p,
+           (const R4<R>*)vel_.p, (const R*)press_.p, bargs(), P_);
     launch("body_reduce", k_body_reduce, dim3(nbodies_), dim3(kBlock), bodies_d_.p, nbodies_,
-           (const double*)body_partials_.p, producer_blocks);
+           (const double*)body_partials_.p, nb);
   }
 
   // One Jacobi iteration: pressure accelerations of the current pressures, then
@@ -1435,7 +1445,6 @@ class System : public SystemBase {
   // The pressure acceleration after a solve (a13 with the solved pressures;
   // OUT 1: +=, OUT 2: overwrite) as one more sweep pass A: the per-solve
   // constants and the {x, V p} records of the last sweep are still current.
-  // Only without reaction forces onto dynamic bodies.
   template <int OUT>
   void final_pressure_accel() {
     const int nb = blocks_for((long long)n_);
@@ -1489,32 +1498,25 @@ class System : public SystemBase {
       case SPH_SESPH:
         launch_s("accel_sesph", k_accel<R, 1>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(), acc_.p,
                vstar_.p, press_.p, 0, P_);
-        body_reduce(nb);
+        body_react();
         break;
       case SPH_SESPH_W_SPLITTING:
         launch_s("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
                acc_.p, vstar_.p, press_.p, 1, P_);
-        body_reduce(nb);
         launch_s("split_density", k_split_density<R, NB>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
                (const R4<R>*)vstar_.p, nbr, bargs(), press_.p, rho_pred_.p, P_);
-        launch_s("pressure_accel", k_pressure_accel<R, 1>, dim3(nb), dim3(kBlock), sm_xp, csc, xv, vel,
-               (const R*)press_.p, nbr, bargs(), acc_.p, 1, P_);
-        body_reduce(nb);
+        launch_s("pressure_accel", k_pressure_accel<R>, dim3(nb), dim3(kBlock), sm_xp, csc, xv, vel,
+               (const R*)press_.p, nbr, bargs(), acc_.p, P_);
+        body_react();
         break;
       case SPH_IISPH:
         launch_s("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
                acc_.p, vstar_.p, press_.p, 1, P_);
-        body_reduce(nb);
         launch_s("iisph_source_diag", k_iisph_source_diag<R, 1>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
                (const R4<R>*)vstar_.p, nbr, bargs(), s_.p, aii_.p, press_.p, TA_.p, TB_.p, SA_.p, xq_.p, P_);
         solve_loop(-1);
-        if (any_dynamic_) {
-          launch_s("pressure_accel", k_pressure_accel<R, 1>, dim3(nb), dim3(kBlock), sm_xp, csc, xv, vel,
-                 (const R*)press_.p, nbr, bargs(), acc_.p, 1, P_);
-          body_reduce(nb);
-        } else {
-          final_pressure_accel<1>();
-        }
+        final_pressure_accel<1>();
+        body_react();
         break;
       case SPH_IISPH_W_OST:
         launch_s("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
@@ -1577,16 +1579,19 @@ class System : public SystemBase {
              (const uint32_t*)sbid_.p, xb_.p, vb_.p);
       sort_samples();
     }
-    if (boundary_kind_ == 1)
-      launch("boundary_samples", k_sample_aggregate<R>, dim3(nb), dim3(kBlock), d_sc_.p, (const R4<R>*)pos_.p,
-             sample_grid(), bW_.p, bG_.p, bGu_.p, P_);
-    else if (boundary_kind_ == 2) {
+    if (boundary_kind_ == 1) {
+      const bool split = cfg_.pressure_solver == SPH_SESPH_W_SPLITTING;
+      launch_s("boundary_samples", split ? k_sample_boundary<R, true> : k_sample_boundary<R, false>,
+               dim3((unsigned)((n_ + kSampleBlock - 1) / kSampleBlock) + (n_ == 0)), dim3(kBlock),
+               sizeof(SampleStage<R>) * (kBlock / 32), d_sc_.p, (const R4<R>*)pos_.p, (const R4<R>*)vel_.p,
+               sample_grid(), (const Body*)bodies_d_.p, any_dynamic_ ? 1 : 0, bW_.p, bG_.p, bGu_.p, bA_.p, touch_.p, P_);
+    } else if (boundary_kind_ == 2) {
       launch("vm_near", k_vm_near<R>, dim3(nb), dim3(kBlock), d_sc_.p, (const R4<R>*)pos_.p,
              (const VMDesc*)vms_.p, (int)fields_.size(), (const Body*)bodies_d_.p, vm_near_.p, vmx_.p, vmv_.p,
-             bW_.p, bG_.p, bGu_.p, P_);
+             bW_.p, bG_.p, bGu_.p, bA_.p, P_);
       launch("boundary_samples", k_vm_sample<R>, dim3(nb), dim3(kBlock), d_sc_.p, (const uint32_t*)vm_near_.p,
-             (const R4<R>*)pos_.p, (const VMDesc*)vms_.p, (int)fields_.size(), (const Body*)bodies_d_.p, vmx_.p,
-             vmv_.p, bW_.p, bG_.p, bGu_.p, P_);
+             (const R4<R>*)pos_.p, (const R4<R>*)vel_.p, (const VMDesc*)vms_.p, (int)fields_.size(),
+             (const Body*)bodies_d_.p, vmx_.p, vmv_.p, bW_.p, bG_.p, bGu_.p, bA_.p, touch_.p, P_);
     }
     // IISPH in f32 re-reads the lists in every sweep pass: they come out ordered for shared-memory banks
     const bool order = sizeof(R) == 4 && (cfg_.pressure_solver == SPH_IISPH || cfg_.pressure_solver == SPH_IISPH_W_OST);
