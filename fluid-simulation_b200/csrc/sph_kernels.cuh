@@ -2255,7 +2255,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_accel(
   R px = 0, py = 0, pz = 0;
   auto pair = [&](const R4<R>& r) {
     const R rx = xi.x - r.x, ry = xi.y - r.y, rz = xi.z - r.z;
-    const R t = r.w * grad_piecewise(rx * rx + ry * ry + rz * rz, ih);
+    const R t = r.w * grad_third(rx, ry, rz, ih);
     px += t * rx; py += t * ry; pz += t * rz;
   };
   if (H.staged) {
@@ -2278,7 +2278,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_accel(
       pair(r0); pair(r1); pair(r2); pair(r3);
     }
   }
-  const R cg = R(-3) * P.k.cg;  // grad_piecewise is grad_core divided by -3
+  const R cg = R(-3) * P.k.cg;  // gradW = -3 cg grad_third r
   const R fx = pi * Ti.x + cg * px, fy = pi * Ti.y + cg * py, fz = pi * Ti.z + cg * pz;
   const R c = Ti.w;  // V_i a_i = -(V_i^2 / m_i) F
   if (OUT == 0) {
@@ -2342,7 +2342,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_jacobi
     R sum = 0;
     auto pair = [&](const R4<R>& a, const R2<R>& b) {
       const R rx = xi.x - a.x, ry = xi.y - a.y, rz = xi.z - a.z;
-      sum += grad_core(rx * rx + ry * ry + rz * rz, ih) * (a.w * rx + b.x * ry + b.y * rz);
+      sum += grad_third(rx, ry, rz, ih) * (a.w * rx + b.x * ry + b.y * rz);
     };
     if (H.staged) {
       for (int g = 0; g < L.ng; ++g) {
@@ -2365,7 +2365,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_jacobi
     const R dt = (R)sc->dt;
     const R iV = R(1) / xi.w;
     const R ax = u4.w * iV, ay = u2.x * iV, az = u2.y * iV;
-    const R tot = ax * Ti.x + ay * Ti.y + az * Ti.z - P.k.cg * sum;
+    const R tot = ax * Ti.x + ay * Ti.y + az * Ti.z + R(3) * P.k.cg * sum;  // gradW = -3 cg grad_third r
     const R A = dt * dt * tot;
     const R s = sa.x, aii = sa.y;
     R pn = p0;

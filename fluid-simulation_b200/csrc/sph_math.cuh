@@ -94,65 +94,38 @@ __device__ __forceinline__ R kernel_grad_factor(R r2, const KernelConst<R>& k) {
   return k.cg * dw / rn;
 }
 
-// f32: reciprocal square root instead of IEEE sqrt + division (relative
-// error ~1e-7, far inside the f32 state's tolerance); f64 keeps the exact form.
+// f32: w'(q) / |r| = 3 ((1-2q)_+^2 - (1-q)_+^2) / |r| from one approximate
+// reciprocal square root (relative error ~1e-7, far inside the f32 state's
+// tolerance); the clamps ride in saturating FMAs, and the squared distance is
+// kept away from 0, where the factor is exactly 0, so that there is no compare
+// and no select. f64 keeps the exact form.
+__device__ __forceinline__ float grad_third_r2(float r2, float inv_h) {  // -1/3 w'(q) / |r|, r2 > 0
+  float inv, t, b;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(r2));
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(t) : "f"(r2 * inv), "f"(-inv_h), "f"(1.f));  // (1-q)_+
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(b) : "f"(t), "f"(2.f), "f"(-1.f));           // (1-2q)_+
+  return fmaf(-b, b, t * t) * inv;
+}
 template <>
 __device__ __forceinline__ float kernel_grad_factor<float>(float r2, const KernelConst<float>& k) {
-  if (!(r2 > 0.f)) return 0.f;
-  const float inv = rsqrtf(r2);
-  const float q = r2 * inv * k.inv_h;
-  const float a = q < 1.f ? 1.f - q : 0.f;
-  const float b = q < 0.5f ? 0.5f - q : 0.f;
-  return k.cg * (-3.f * (a * a) + 12.f * (b * b)) * inv;
+  return -3.f * k.cg * grad_third_r2(fmaxf(r2, 1e-30f), k.inv_h);
 }
 
-// The gradient factor without its constant: gradW(r) = cg * grad_core(r2) * r,
-// grad_core = w'(q) / |r| with w'(q) = 12 (1/2-q)_+^2 - 3 (1-q)_+^2 (zero at
-// r = 0 and outside the support). Sums of grad_core terms are scaled by cg
-// once, after the loop.
+// The gradient factor without its constant, from the pair's offset: gradW(r) =
+// -3 cg * grad_third * r. In f64 in its piecewise form, (2 - 3q) / h for
+// q < 1/2 and (1-q)^2 / |r| beyond. The caller scales its sums by -3 cg once.
 template <class R>
-__device__ __forceinline__ R grad_core(R r2, R inv_h) {
-  const R rn = sqrt(r2);
-  const R q = rn * inv_h;
-  const R a = q < R(1) ? R(1) - q : R(0);
-  const R b = q < R(0.5) ? R(0.5) - q : R(0);
-  return r2 > R(0) ? (R(12) * (b * b) - R(3) * (a * a)) / rn : R(0);
-}
-// f32: one approximate reciprocal square root (relative error ~2^-23, far
-// inside the f32 state's tolerance) and no branch.
-template <>
-__device__ __forceinline__ float grad_core<float>(float r2, float inv_h) {
-  float inv;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(r2));
-  inv = r2 > 0.f ? inv : 0.f;
-  const float q = r2 * inv * inv_h;
-  const float a = fmaxf(1.f - q, 0.f), b = fmaxf(0.5f - q, 0.f);
-  return fmaf(12.f * b, b, -3.f * a * a) * inv;
-}
-
-// The same factor in its piecewise form, divided by -3: with q = |r|/h,
-// w'(q) = 9q^2 - 6q for q < 1/2 and -3 (1-q)^2 for 1/2 <= q < 1, so
-// grad_core / -3 = (2 - 3q) / h, resp. (1-q)^2 / |r| (no division in f32;
-// the caller scales its sums by -3 cg once). Its product with r is zero at
-// r = 0.
-template <class R>
-__device__ __forceinline__ R grad_piecewise(R r2, R inv_h) {
-  const R rn = sqrt(r2);
+__device__ __forceinline__ R grad_third(R rx, R ry, R rz, R inv_h) {
+  const R rn = sqrt(rx * rx + ry * ry + rz * rz);
   const R q = rn * inv_h;
   if (q < R(0.5)) return (R(2) - R(3) * q) * inv_h;
   const R t = R(1) - q;
   return q < R(1) ? t * t / rn : R(0);
 }
-// f32: r2 is clamped away from 0 so that the self pair (r = 0) gives a finite
-// factor; one approximate reciprocal square root.
+// (1e-30 has no effect on any pair but the self pair)
 template <>
-__device__ __forceinline__ float grad_piecewise<float>(float r2, float inv_h) {
-  const float r2c = fmaxf(r2, 1e-30f);
-  float inv;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(r2c));
-  const float q = r2c * inv * inv_h;
-  const float t = fmaxf(1.f - q, 0.f);
-  return q < 0.5f ? fmaf(-3.f * inv_h, q, 2.f * inv_h) : t * t * inv;
+__device__ __forceinline__ float grad_third<float>(float rx, float ry, float rz, float inv_h) {
+  return grad_third_r2(fmaf(rz, rz, fmaf(ry, ry, fmaf(rx, rx, 1e-30f))), inv_h);
 }
 
 // Both W and the gradient factor from one square root.
