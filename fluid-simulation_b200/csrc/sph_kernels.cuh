@@ -1206,11 +1206,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
 // ---------------------------------------------------------------------------
 // 5. boundary samples: sample boundaries (sorted sample grid) and volume maps
 // ---------------------------------------------------------------------------
-// Serendipity reference nodes (discretization.rs:267-300): lattice offsets and
-// node kind (0 corner, 1/2/3 edge along x/y/z) with reference coordinates.
-__constant__ double c_ser_ref[32][3];
+// Serendipity reference nodes (discretization.rs:267-300): lattice offsets in
+// the reference's order.
 __constant__ int c_ser_off[32][3];
-__constant__ int c_ser_kind[32];
 
 // f64 arithmetic that the compiler may not contract into FMAs, so that the
 // field evaluation rounds exactly like the reference's (discretization.rs:
@@ -1221,52 +1219,78 @@ __device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double sub_(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double div_(double a, double b) { return __ddiv_rn(a, b); }
 
-__device__ bool ser_function(const DevField& F, double px, double py, double pz, double& out) {
+// The 32 nodes in the reference's order (discretization.rs:267-300): 8 corners,
+// 8 nodes each on the edges along x, y and z. The partial products that nodes
+// share are formed once, in the reference's order of multiplication, so every
+// term keeps its bits. The nodes of a group are loaded together.
+__device__ __forceinline__ bool ser_eval(const DevField& F, double px, double py, double pz, double& out) {
   const double p[3] = {px, py, pz};
   long long c[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const double fi = floor(div_(sub_(p[d], F.xmin[d]), F.dx));
     if (p[d] < F.xmin[d] || p[d] > F.xmax[d]) return false;
-    long long idx = (long long)fi;
+    const long long idx = (long long)fi;
     c[d] = idx < (long long)F.n[d] - 1 ? idx : (long long)F.n[d] - 1;
   }
-  const double o0 = add_(F.xmin[0], mul_((double)c[0], F.dx));
-  const double o1 = add_(F.xmin[1], mul_((double)c[1], F.dx));
-  const double o2 = add_(F.xmin[2], mul_((double)c[2], F.dx));
-  const double xi = sub_(div_(mul_(2.0, sub_(p[0], o0)), F.dx), 1.0);
-  const double eta = sub_(div_(mul_(2.0, sub_(p[1], o1)), F.dx), 1.0);
-  const double zeta = sub_(div_(mul_(2.0, sub_(p[2], o2)), F.dx), 1.0);
-  const double r2 = add_(add_(mul_(xi, xi), mul_(eta, eta)), mul_(zeta, zeta));
-  const double e19 = sub_(mul_(9.0, r2), 19.0);
-  const long long bx = 3 * c[0], by = 3 * c[1], bz = 3 * c[2];
+  const double xi = sub_(div_(mul_(2.0, sub_(p[0], add_(F.xmin[0], mul_((double)c[0], F.dx)))), F.dx), 1.0);
+  const double eta = sub_(div_(mul_(2.0, sub_(p[1], add_(F.xmin[1], mul_((double)c[1], F.dx)))), F.dx), 1.0);
+  const double zeta = sub_(div_(mul_(2.0, sub_(p[2], add_(F.xmin[2], mul_((double)c[2], F.dx)))), F.dx), 1.0);
+  const long long ny = F.NX, nz = F.NX * F.NY;  // one step along y and z
+  const double* base = F.nodes + ((3 * c[2] * F.NY + 3 * c[1]) * F.NX + 3 * c[0]);
+  const double lx[2] = {sub_(1.0, xi), add_(1.0, xi)};
+  const double ly[2] = {sub_(1.0, eta), add_(1.0, eta)};
+  const double lz[2] = {sub_(1.0, zeta), add_(1.0, zeta)};
+  const double third = 1.0 / 3.0;
   double s = 0.0;
-  for (int a = 0; a < 32; ++a) {
-    const long long idx =
-        ((bz + c_ser_off[a][2]) * F.NY + (by + c_ser_off[a][1])) * F.NX + (bx + c_ser_off[a][0]);
-    const double v = __ldg(F.nodes + idx);
-    if (v != v) return false;  // pruned cell
-    const double ax = c_ser_ref[a][0], ay = c_ser_ref[a][1], az = c_ser_ref[a][2];
-    const double lx = add_(1.0, mul_(xi, ax)), ly = add_(1.0, mul_(eta, ay)), lz = add_(1.0, mul_(zeta, az));
-    double N;
-    switch (c_ser_kind[a]) {
-      case 0:  // (1/64)(1+xi a)(1+eta b)(1+zeta c)(9 r^2 - 19)
-        N = mul_(mul_(mul_(mul_(1.0 / 64.0, lx), ly), lz), e19);
-        break;
-      case 1:  // (9/64)(1-xi^2)(1+9 xi a)(1+eta b)(1+zeta c)
-        N = mul_(mul_(mul_(mul_(9.0 / 64.0, sub_(1.0, mul_(xi, xi))), add_(1.0, mul_(mul_(9.0, xi), ax))), ly), lz);
-        break;
-      case 2:  // (9/64)(1-eta^2)(1+9 eta b)(1+xi a)(1+zeta c)
-        N = mul_(mul_(mul_(mul_(9.0 / 64.0, sub_(1.0, mul_(eta, eta))), add_(1.0, mul_(mul_(9.0, eta), ay))), lx), lz);
-        break;
-      default:  // (9/64)(1-zeta^2)(1+9 zeta c)(1+xi a)(1+eta b)
-        N = mul_(mul_(mul_(mul_(9.0 / 64.0, sub_(1.0, mul_(zeta, zeta))), add_(1.0, mul_(mul_(9.0, zeta), az))), lx), ly);
-        break;
-    }
-    s = add_(s, mul_(v, N));
-  }
+  double v[8], w[4];
+  auto load = [&](auto offset) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = __ldg(base + offset(k));
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) ok = ok && v[k] == v[k];
+    return ok;  // no pruned node
+  };
+  // corners: (1/64)(1+xi a)(1+eta b)(1+zeta c)(9 r^2 - 19)
+  if (!load([&](int k) { return 3 * (k & 1) + 3 * ((k >> 1) & 1) * ny + 3 * (k >> 2) * nz; })) return false;
+  const double e19 = sub_(mul_(9.0, add_(add_(mul_(xi, xi), mul_(eta, eta)), mul_(zeta, zeta))), 19.0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w[k] = mul_(mul_(1.0 / 64.0, lx[k & 1]), ly[k >> 1]);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s = add_(s, mul_(v[k], mul_(mul_(w[k & 3], lz[k >> 2]), e19)));
+  // edges along x: (9/64)(1-xi^2)(1+9 xi a)(1+eta b)(1+zeta c), a = -1/3, 1/3
+  auto along = [&](double u, double e[2]) {
+    const double f = mul_(9.0 / 64.0, sub_(1.0, mul_(u, u))), g = mul_(mul_(9.0, u), third);
+    e[0] = mul_(f, sub_(1.0, g));
+    e[1] = mul_(f, add_(1.0, g));
+  };
+  double e[2];
+  if (!load([&](int k) { return 1 + (k & 1) + 3 * ((k >> 1) & 1) * ny + 3 * (k >> 2) * nz; })) return false;
+  along(xi, e);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w[k] = mul_(e[k & 1], ly[k >> 1]);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s = add_(s, mul_(v[k], mul_(w[k & 3], lz[k >> 2])));
+  // along y: z outer, x, then the node on the edge
+  if (!load([&](int k) { return (1 + (k & 1)) * ny + 3 * ((k >> 1) & 1) + 3 * (k >> 2) * nz; })) return false;
+  along(eta, e);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w[k] = mul_(e[k & 1], lx[k >> 1]);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s = add_(s, mul_(v[k], mul_(w[k & 3], lz[k >> 2])));
+  // along z: y outer, x, then the node on the edge
+  if (!load([&](int k) { return (1 + (k & 1)) * nz + 3 * ((k >> 1) & 1) + 3 * (k >> 2) * ny; })) return false;
+  along(zeta, e);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w[k] = mul_(e[k & 1], lx[k >> 1]);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s = add_(s, mul_(v[k], mul_(w[k & 3], ly[k >> 2])));
   out = s;
   return true;
+}
+__device__ __noinline__ bool ser_function(const DevField& F, double px, double py, double pz, double& out) {
+  return ser_eval(F, px, py, pz, out);
 }
 
 __device__ bool ser_gradient(const DevField& F, double px, double py, double pz, double g[3]) {
@@ -1289,7 +1313,10 @@ __device__ bool ser_gradient(const DevField& F, double px, double py, double pz,
 // signed distance (the cheap, light first test of find_boundary_samples) and
 // lists the particles within the support radius of some boundary, writing
 // the empty result for all others; k_vm_sample then does the full sampling
-// for the listed particles only.
+// for the listed particles only, eight lanes each, which evaluate the eight
+// field values of a sample at once (one lane after the other took 77-87 us per
+// update for scenes of 133 thousand to one million particles, 15-56 us now; both
+// passes are bound by f64 issue and the latency of the node loads).
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_vm_near(
     Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const VMDesc* __restrict__ vms, int nvm,
@@ -1306,7 +1333,7 @@ __global__ void __launch_bounds__(kBlock) k_vm_near(
     double pl[3] = {p[0], p[1], p[2]};
     if (D.body >= 0) body_world_to_local(bodies[D.body], p, pl);
     double sd;
-    near = ser_function(D.sdf, pl[0], pl[1], pl[2], sd) && sd < P.range;
+    near = ser_eval(D.sdf, pl[0], pl[1], pl[2], sd) && sd < P.range;
   }
   if (near) {
     near_list[atomicAdd(&sc->vm_near, 1u)] = (uint32_t)i;
@@ -1326,28 +1353,31 @@ __global__ void __launch_bounds__(kBlock) k_vm_near(
 // the support ball); the sample sits at max(sd + spacing/4, spacing) against
 // the normalized gradient, moving with the body's velocity there. Returns
 // false, leaving the outputs untouched, when the point has no sample.
-__device__ __forceinline__ bool vm_normal_sample(const VMDesc& D, const Body* body, const double p[3],
-                                                 double range, double ball, double spacing,
-                                                 double xb[3], double vb[3], double& vol) {
-  double pl[3] = {p[0], p[1], p[2]};
-  if (body) body_world_to_local(*body, p, pl);
-  double sd;
-  if (!ser_function(D.sdf, pl[0], pl[1], pl[2], sd) || !(sd < range)) return false;
-  double g[3];
-  if (!ser_gradient(D.sdf, pl[0], pl[1], pl[2], g)) return false;
-  if (body) {
-    double gw[3];
-    qrot(body->q, g, gw);
-    g[0] = gw[0]; g[1] = gw[1]; g[2] = gw[2];
-  }
+// vm_sample_from takes the field values: the signed distance, its gradient in
+// the body frame, and the volume map.
+__device__ __forceinline__ bool vm_sample_from(double sd, const double gl[3], double vm, const Body* body,
+                                               const double p[3], double ball, double spacing, double xb[3],
+                                               double vb[3], double& vol) {
+  double g[3] = {gl[0], gl[1], gl[2]};
+  if (body) qrot(body->q, gl, g);
   const double gn = __dsqrt_rn(add_(add_(mul_(g[0], g[0]), mul_(g[1], g[1])), mul_(g[2], g[2])));
-  double vm;
-  if (!(gn > 0.5 && gn < 2.0) || !ser_function(D.vm, pl[0], pl[1], pl[2], vm) || !(vm > 0.0)) return false;
+  if (!(gn > 0.5 && gn < 2.0) || !(vm > 0.0)) return false;
   vol = vm < ball ? vm : ball;
   const double d = fmax(add_(sd, mul_(0.25, spacing)), spacing);
   for (int c = 0; c < 3; ++c) xb[c] = sub_(p[c], mul_(div_(g[c], gn), d));
   if (body) body_velocity_at(*body, xb, vb);
   return true;
+}
+__device__ __forceinline__ bool vm_normal_sample(const VMDesc& D, const Body* body, const double p[3],
+                                                 double range, double ball, double spacing,
+                                                 double xb[3], double vb[3], double& vol) {
+  double pl[3] = {p[0], p[1], p[2]};
+  if (body) body_world_to_local(*body, p, pl);
+  double sd, g[3], vm;
+  if (!ser_function(D.sdf, pl[0], pl[1], pl[2], sd) || !(sd < range)) return false;
+  if (!ser_gradient(D.sdf, pl[0], pl[1], pl[2], g)) return false;
+  if (!ser_function(D.vm, pl[0], pl[1], pl[2], vm)) return false;
+  return vm_sample_from(sd, g, vm, body, p, ball, spacing, xb, vb, vol);
 }
 
 // The four tangential viscosity samples of a volume-map sample x_b of particle
@@ -1390,13 +1420,15 @@ __device__ __forceinline__ R boundary_viscosity(const V3<R>& r, const V3<R>& dv,
 }
 
 template <class R>
-__global__ void __launch_bounds__(kBlock) k_vm_sample(
+__global__ void __launch_bounds__(kBlock, 3) k_vm_sample(
     Scalars* __restrict__ sc, const uint32_t* __restrict__ near_list, const R4<R>* __restrict__ pos,
     const R4<R>* __restrict__ vel, const VMDesc* __restrict__ vms, int nvm, const Body* __restrict__ bodies,
     R4<R>* __restrict__ vmx, R4<R>* __restrict__ vmv, R* __restrict__ bW, R4<R>* __restrict__ bG,
     R4<R>* __restrict__ bGu, R4<R>* __restrict__ bA, uint32_t* __restrict__ touch, StepParams<R> P) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int)sc->vm_near) return;
+  const int lane = threadIdx.x & 31, e = lane & 7;
+  const unsigned group = 0xffu << (lane & ~7);
+  const int t = (blockIdx.x * kBlock + threadIdx.x) >> 3;
+  if (t >= (int)sc->vm_near) return;  // (a group of eight lanes stays together)
   const int i = (int)near_list[t];
   const R4<R> xr = pos[i], vi = vel[i];
   bool dyn = false;
@@ -1410,7 +1442,25 @@ __global__ void __launch_bounds__(kBlock) k_vm_sample(
     const Body* body = D.body >= 0 ? &bodies[D.body] : nullptr;
     int kind = 0;
     double xb[3] = {0, 0, 0}, vb[3] = {0, 0, 0}, vol = 0;
-    if (vm_normal_sample(D, body, p, range, ball, P.spacing, xb, vb, vol)) {
+    double pl[3] = {p[0], p[1], p[2]};
+    if (body) body_world_to_local(*body, p, pl);
+    // lanes 0 to 5: the distance half a node step to either side along x, y
+    // and z (ser_gradient); lane 6: the distance; lane 7: the volume map
+    const double step = div_(D.sdf.dx, 6.0);
+    const double off = e & 1 ? -step : step;
+    double q[3] = {pl[0], pl[1], pl[2]};
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      if (e >> 1 == d) q[d] = add_(q[d], off);
+    double f = 0.0;
+    const bool ok = ser_eval(e == 7 ? D.vm : D.sdf, q[0], q[1], q[2], f);
+    const bool all = __all_sync(group, ok);
+    const double sd = __shfl_sync(group, f, 6, 8), vm = __shfl_sync(group, f, 7, 8);
+    double g[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      g[d] = div_(sub_(__shfl_sync(group, f, 2 * d, 8), __shfl_sync(group, f, 2 * d + 1, 8)), mul_(2.0, step));
+    if (all && sd < range && vm_sample_from(sd, g, vm, body, p, ball, P.spacing, xb, vb, vol)) {
       const double u[3] = {xb[0] - p[0], xb[1] - p[1], xb[2] - p[2]};
       const double un = sqrt((u[0] * u[0] + u[1] * u[1]) + u[2] * u[2]);
       kind = fabs(u[0] / un) > 0.9 ? 2 : 1;
@@ -1432,22 +1482,27 @@ __global__ void __launch_bounds__(kBlock) k_vm_sample(
     }
     const size_t o = (size_t)b * P.Np + i;
     const R4<R> xx{(R)xb[0], (R)xb[1], (R)xb[2], (R)vol};
-    vmx[o] = xx;
-    vmv[o] = R4<R>{(R)vb[0], (R)vb[1], (R)vb[2], (R)kind};
+    if (e == 0) {
+      vmx[o] = xx;
+      vmv[o] = R4<R>{(R)vb[0], (R)vb[1], (R)vb[2], (R)kind};
+    }
     if (kind == 0) continue;
-    // viscosity: four tangential samples of a quarter of the volume each
+    // viscosity: four tangential samples of a quarter of the volume each, one per lane
     const TangentSamples<R> ts(xr, xx, (R)kind, range);
-    const bool moves = D.body >= 0 && bodies[D.body].dynamic;
-    dyn |= moves;
-#pragma unroll 1
+    dyn |= D.body >= 0 && bodies[D.body].dynamic;
+    const V3<R> qt = ts.at(e & 3);
+    const V3<R> vq = body_velocity_r(bodies, D.body, qt);
+    const V3<R> r{xr.x - qt.x, xr.y - qt.y, xr.z - qt.z};
+    const R c = boundary_viscosity(r, V3<R>{vi.x - vq.x, vi.y - vq.y, vi.z - vq.z}, R(0.25) * xx.w, P);
+    const R tx = c * r.x, ty = c * r.y, tz = c * r.z;
+#pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const V3<R> q = ts.at(k);
-      const V3<R> vq = body_velocity_r(bodies, D.body, q);
-      const V3<R> r{xr.x - q.x, xr.y - q.y, xr.z - q.z};
-      const R s = boundary_viscosity(r, V3<R>{vi.x - vq.x, vi.y - vq.y, vi.z - vq.z}, R(0.25) * xx.w, P);
-      sx += s * r.x; sy += s * r.y; sz += s * r.z;
+      sx += __shfl_sync(group, tx, k, 8);
+      sy += __shfl_sync(group, ty, k, 8);
+      sz += __shfl_sync(group, tz, k, 8);
     }
   }
+  if (e != 0) return;
   bW[i] = w;
   bG[i] = R4<R>{gx, gy, gz, gv};
   if (bGu) bGu[i] = R4<R>{ux, uy, uz, R(0)};
@@ -1999,6 +2054,11 @@ __global__ void __launch_bounds__(kBlock) k_accel(
   const bool act = i < sc->n_active;
   SweepList<R> L;  // the list head travels while the halo stages
   L.begin(N, act ? i : 0, act ? min((int)N.ncnt[i], N.K) : 0);
+  R4<R> xi{}, vi{};
+  if (act) {
+    xi = xv[i];
+    vi = vel[i];
+  }
   R4<R>* s_x = staged_vec<R>(dsm, N.hs, 0);
   R4<R>* s_v = staged_vec<R>(dsm, N.hs, 1);
   if (H.staged)
@@ -2008,8 +2068,6 @@ __global__ void __launch_bounds__(kBlock) k_accel(
     });
   stage_done();
   if (act) {
-    const R4<R> xi = xv[i];
-    const R4<R> vi = vel[i];
     const R mi = vi.w, Vi = xi.w;
     R ax, ay, az;
     if (P.gravity_mode == 0) {
@@ -2031,10 +2089,10 @@ __global__ void __launch_bounds__(kBlock) k_accel(
           const R r2 = rx * rx + ry * ry + rz * rz;
           const R f = kernel_grad_factor(r2, P.k);
           const R vr = (vi.x - vj.x) * rx + (vi.y - vj.y) * ry + (vi.z - vj.z) * rz;
-          const R s = P.visc_f * xj.w * vr / (r2 + P.eps_visc) * f;
+          const R s = quotient(P.visc_f * xj.w * vr, r2 + P.eps_visc) * f;
           sx += s * rx; sy += s * ry; sz += s * rz;
           if (PRESS == 1) {
-            const R pj = P.stiffness * fmax(P.V0 / xj.w - R(1), R(0));
+            const R pj = P.stiffness * fmax(quotient(P.V0, xj.w) - R(1), R(0));
             const R t = xj.w * (pi + pj) * f;
             px += t * rx; py += t * ry; pz += t * rz;
           }
@@ -2059,7 +2117,8 @@ __global__ void __launch_bounds__(kBlock) k_accel(
     acc[i] = R4<R>{ax, ay, az, R(0)};
     if (write_vstar) {
       const R dt = (R)sc->dt;
-      vstar[i] = R4<R>{vi.x + dt * ax, vi.y + dt * ay, vi.z + dt * az, mi};  // the mass rides along
+      // (the lane that the next pass needs rides along: the mass, or V^2 / m)
+      vstar[i] = R4<R>{vi.x + dt * ax, vi.y + dt * ay, vi.z + dt * az, write_vstar == 2 ? Vi * Vi / mi : mi};
     }
     if (PRESS == 1) press[i] = pi;
   }
@@ -2137,7 +2196,14 @@ __global__ void __launch_bounds__(kBlock) k_iisph_source_diag(
   const bool act = i < sc->n_active;
   SweepList<R> L;  // the list head travels while the halo stages
   L.begin(N, act ? i : 0, act ? min((int)N.ncnt[i], N.K) : 0);
-  // records {x, V} and {v*, m} (the acceleration pass stores m in v*.w)
+  R4<R> xi{}, vsi{};
+  R mi = 1;
+  if (act) {
+    xi = xv[i];
+    vsi = vstar[i];
+    mi = vel[i].w;
+  }
+  // records {x, V} and {v*, V^2/m} (the acceleration pass stores V^2/m in v*.w)
   R4<R>* s_x = staged_vec<R>(dsm, N.hs, 0);
   R4<R>* s_v = staged_vec<R>(dsm, N.hs, 1);
   if (H.staged)
@@ -2148,9 +2214,7 @@ __global__ void __launch_bounds__(kBlock) k_iisph_source_diag(
   stage_done();
   if (!act) return;
   const R dt = (R)sc->dt;
-  const R4<R> xi = xv[i];
-  const R4<R> vsi = vstar[i];
-  const R Vi = xi.w, mi = vsi.w;
+  const R Vi = xi.w;
   R div = 0;                       // sum V_j (v*_i - v*_j) . gradW
   R sfx = 0, sfy = 0, sfz = 0;     // S_f = sum V_j gradW
   R s2 = 0;                        // sum V_j^2 / m_j |gradW|^2
@@ -2163,7 +2227,7 @@ __global__ void __launch_bounds__(kBlock) k_iisph_source_diag(
     const R Vf = xj.w * f;
     div += Vf * ((vsi.x - vsj.x) * rx + (vsi.y - vsj.y) * ry + (vsi.z - vsj.z) * rz);
     sfx += Vf * rx; sfy += Vf * ry; sfz += Vf * rz;
-    s2 += xj.w * xj.w / vsj.w * (f * f * r2);
+    s2 += vsj.w * (f * f * r2);
   };
   if (H.staged)
     sweep_groups(L, [&](uint32_t l) { return XV<R>{s_x[l], s_v[l]}; }, pair);

@@ -73,6 +73,16 @@ __host__ KernelConst<R> make_kernel_const(double h) {
 template <class R>
 __device__ __forceinline__ R sq(R x) { return x * x; }
 
+// a / b. f32: the approximate reciprocal and one Newton step on the quotient
+// (its residual in one fma), within an ulp for the b > 0 of the pair loops.
+__device__ __forceinline__ double quotient(double a, double b) { return a / b; }
+__device__ __forceinline__ float quotient(float a, float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  const float q = a * r;
+  return fmaf(fmaf(-b, q, a), r, q);
+}
+
 // W from the squared distance; zero outside the support.
 template <class R>
 __device__ __forceinline__ R kernel_w_r2(R r2, const KernelConst<R>& k) {

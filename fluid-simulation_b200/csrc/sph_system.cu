@@ -93,27 +93,19 @@ static void upload_serendipity_tables() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && done_for[dev]) return;
-  double ref[32][3];
   int off[32][3];
-  int kind[32];
   int a = 0;
   const double s[2] = {-1.0, 1.0}, t[2] = {-1.0 / 3.0, 1.0 / 3.0};
   auto push = [&](double x, double y, double z) {
-    ref[a][0] = x; ref[a][1] = y; ref[a][2] = z;
     const double r[3] = {x, y, z};
     for (int d = 0; d < 3; ++d) off[a][d] = (int)std::llround((r[d] + 1.0) * 1.5);
-    auto corner = [](double c) { return std::fabs(std::fabs(c) - 1.0) < 1e-9; };
-    const bool cx = corner(x), cy = corner(y), cz = corner(z);
-    kind[a] = (cx && cy && cz) ? 0 : (!cx ? 1 : (!cy ? 2 : 3));
     ++a;
   };
   for (double z : s) for (double y : s) for (double x : s) push(x, y, z);
   for (double z : s) for (double y : s) for (double q : t) push(q, y, z);
   for (double z : s) for (double x : s) for (double q : t) push(x, q, z);
   for (double y : s) for (double x : s) for (double q : t) push(x, y, q);
-  cuda_check(cudaMemcpyToSymbol(c_ser_ref, ref, sizeof ref), "serendipity tables");
   cuda_check(cudaMemcpyToSymbol(c_ser_off, off, sizeof off), "serendipity tables");
-  cuda_check(cudaMemcpyToSymbol(c_ser_kind, kind, sizeof kind), "serendipity tables");
   if (dev >= 0 && dev < 64) done_for[dev] = true;
 }
 
@@ -860,7 +852,11 @@ class System : public SystemBase {
   DBuf<uint32_t> ref_, ref2_, fid_, fid2_, key_, slot_, perm_, ncnt_, halo_idx_, halo_n_;
   DBuf<uint16_t> nbr_;
   int hcap_ = 8192;   // halo table capacity per block (grows on overflow, at most 65535)
-  int hs_ = sizeof(R) == 4 ? 1536 : 1024;  // halo records staged in shared memory per block
+  // halo records staged in shared memory per block (f32: 1792 x 32 B lets four
+  // blocks of the widest pass share an SM; halos of a flowing scene reach 1700
+  // records, and with 1536 the acceleration and source passes of 133 thousand
+  // particles took 26 and 27 us, now 19 each)
+  int hs_ = sizeof(R) == 4 ? 1792 : 1024;
   // the same for the IISPH sweep passes (f32: 1792 x 24 B lets five pass-B
   // blocks share an SM's shared memory)
   int sweep_hs_ = sizeof(R) == 4 ? 1792 : 1024;
@@ -1511,7 +1507,7 @@ class System : public SystemBase {
         break;
       case SPH_IISPH:
         launch_s("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
-               acc_.p, vstar_.p, press_.p, 1, P_);
+               acc_.p, vstar_.p, press_.p, 2, P_);
         launch_s("iisph_source_diag", k_iisph_source_diag<R, 1>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
                (const R4<R>*)vstar_.p, nbr, bargs(), s_.p, aii_.p, press_.p, TA_.p, TB_.p, SA_.p, xq_.p, P_);
         solve_loop(-1);
@@ -1520,7 +1516,7 @@ class System : public SystemBase {
         break;
       case SPH_IISPH_W_OST:
         launch_s("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
-               acc_.p, vstar_.p, press_.p, 1, P_);
+               acc_.p, vstar_.p, press_.p, 2, P_);
         launch_s("iisph_source_diag", k_iisph_source_diag<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
                (const R4<R>*)vstar_.p, nbr, bargs(), s_.p, aii_.p, press_.p, TA_.p, TB_.p, SA_.p, xq_.p, P_);
         solve_loop(3);
@@ -1589,7 +1585,7 @@ class System : public SystemBase {
       launch("vm_near", k_vm_near<R>, dim3(nb), dim3(kBlock), d_sc_.p, (const R4<R>*)pos_.p,
              (const VMDesc*)vms_.p, (int)fields_.size(), (const Body*)bodies_d_.p, vm_near_.p, vmx_.p, vmv_.p,
              bW_.p, bG_.p, bGu_.p, bA_.p, P_);
-      launch("boundary_samples", k_vm_sample<R>, dim3(nb), dim3(kBlock), d_sc_.p, (const uint32_t*)vm_near_.p,
+      launch("boundary_samples", k_vm_sample<R>, dim3(8 * nb), dim3(kBlock), d_sc_.p, (const uint32_t*)vm_near_.p,
              (const R4<R>*)pos_.p, (const R4<R>*)vel_.p, (const VMDesc*)vms_.p, (int)fields_.size(),
              (const Body*)bodies_d_.p, vmx_.p, vmv_.p, bW_.p, bG_.p, bGu_.p, bA_.p, touch_.p, P_);
     }
@@ -2810,10 +2806,12 @@ int sph_autotune(sph_system_t* h, uint32_t steps, sph_tuning* best, double* best
     const bool f32 = h->cfg.precision == SPH_F32;
     sph_tuning cur{};
     h->impl->get_tuning(&cur);
+    // (small scenes' steps differ by less than their timing does: fewer candidates)
+    std::vector<uint32_t> stages = f32 ? std::vector<uint32_t>{1024, 1536, 2048} : std::vector<uint32_t>{512, 1024, 1536};
+    if (f32 && h->impl->num_particles() > 65536) stages.push_back(1792);
     std::vector<sph_tuning> cand;
     for (uint32_t nb : {4u, 8u})
-      for (uint32_t hs : f32 ? std::vector<uint32_t>{1024, 1536, 2048} : std::vector<uint32_t>{512, 1024, 1536})
-        cand.push_back(sph_tuning{nb, hs, cur.sweep_stage});
+      for (uint32_t hs : stages) cand.push_back(sph_tuning{nb, hs, cur.sweep_stage});
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     sph::cuda_check(cudaEventCreate(&e0), "cudaEventCreate");
     std::unique_ptr<CUevent_st, cudaError_t (*)(cudaEvent_t)> g0(e0, cudaEventDestroy);
