@@ -1510,6 +1510,51 @@ __global__ void __launch_bounds__(kBlock, 3) k_vm_sample(
   if (dyn) touch[atomicAdd(&sc->n_touch, 1u)] = (uint32_t)i;
 }
 
+// Visits the particles within h of p (f64, the reference's exact predicate) in
+// bucket order: use(j, x, r2) with the sorted index, the record and the squared
+// distance. An f32 distance test with a margin for the rounding of both
+// positions and of the test itself first puts the candidates that may be in
+// range (a sixth of about 216) on a list in shared memory, so the f64 work runs
+// on those only, all lanes at once. (f64 positions are rounded to f32 for it.)
+constexpr int kNearList = 40;  // entries per thread: kNearList * kBlock words of shared memory
+template <class R, class Use>
+__device__ __forceinline__ void for_each_within(const double p[3], double h, uint32_t mask,
+                                                const uint32_t* __restrict__ start, const R4<R>* __restrict__ x,
+                                                uint32_t* s_list, Use&& use) {
+  const int cx = cell_coord(p[0], h), cy = cell_coord(p[1], h), cz = cell_coord(p[2], h);
+  const float fx = (float)p[0], fy = (float)p[1], fz = (float)p[2];
+  const float m = (float)h * 1.00001f + 4e-7f * (fabsf(fx) + fabsf(fy) + fabsf(fz) + (float)h);
+  const float limit = m * m * 1.00001f;
+  const double h2 = h * h, lo = h2 * (1.0 - 1e-14), hi = h2 * (1.0 + 1e-14);
+  uint32_t* list = s_list + threadIdx.x;
+  int cnt = 0;
+  auto drain = [&]() {
+    for (int k = 0; k < cnt; ++k) {
+      const uint32_t j = list[k * kBlock];
+      const R4<R> xj = x[j];
+      const double qx = (double)xj.x, qy = (double)xj.y, qz = (double)xj.z;
+      const double rx = p[0] - qx, ry = p[1] - qy, rz = p[2] - qz;
+      const double r2 = (rx * rx + ry * ry) + rz * rz;
+      if (r2 < lo || (!(r2 > hi) && in_range_exact(p[0], p[1], p[2], qx, qy, qz, h))) use(j, xj, r2);
+    }
+    cnt = 0;
+  };
+#pragma unroll 1
+  for (int q = 0; q < 27; ++q) {
+    const uint32_t k = morton_key(cx + q % 3 - 1, cy + (q / 3) % 3 - 1, cz + q / 9 - 1, mask);
+    const uint32_t e = start[k + 1];
+    for (uint32_t j = start[k]; j < e; ++j) {
+      const R4<R> xj = x[j];
+      const float dx = fx - (float)xj.x, dy = fy - (float)xj.y, dz = fz - (float)xj.z;
+      if (dx * dx + dy * dy + dz * dz > limit) continue;
+      if (cnt == kNearList) drain();
+      list[cnt * kBlock] = j;
+      ++cnt;
+    }
+  }
+  drain();
+}
+
 // ScalarQuantity at evaluation positions (sph/mod.rs:241-341 with the sums
 // of quantities.rs:14-330), for sensor planes: one thread per position walks
 // the 27 buckets of the fluid grid of the last update (sorted positions and
@@ -1531,56 +1576,34 @@ __global__ void __launch_bounds__(kBlock) k_quantity_at(
   if (t >= n_eval) return;
   const double p[3] = {(double)eval[3 * t], (double)eval[3 * t + 1], (double)eval[3 * t + 2]};
   const double h = P.range;
-  const int cx = cell_coord(p[0], h), cy = cell_coord(p[1], h), cz = cell_coord(p[2], h);
+  __shared__ uint32_t s_list[kNearList * kBlock];
   double s = 0, sx = 0, sy = 0, sz = 0;
-  if (start) {
-    for (int dz = -1; dz <= 1; ++dz)
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const uint32_t k = morton_key(cx + dx, cy + dy, cz + dz, P.mask);
-          const uint32_t e = start[k + 1];
-          for (uint32_t j = start[k]; j < e; ++j) {
-            const R4<R> xj = xv[j];
-            const double qx = (double)xj.x, qy = (double)xj.y, qz = (double)xj.z;
-            if (!in_range_exact(p[0], p[1], p[2], qx, qy, qz, h)) continue;
-            const double rx = p[0] - qx, ry = p[1] - qy, rz = p[2] - qz;
-            const double w = kernel_w_r2<double>((rx * rx + ry * ry) + rz * rz, kd);
-            const double V = (double)xj.w;
-            if (quantity == 1) { s += V0 * w; continue; }
-            const R4<R> vj = vel[j];
-            const double vx = (double)vj.x, vy = (double)vj.y, vz = (double)vj.z, m = (double)vj.w;
-            switch (quantity) {
-              case 0: sx += vx * V * w; sy += vy * V * w; sz += vz * V * w; break;
-              case 2: s += m * w; break;
-              case 3: if (m < V0) s += (V0 / m - 1.0) * m * w; break;
-              case 4: s += (double)press[j] * V * w; break;
-              default: s += 0.5 * m * ((vx * vx + vy * vy) + vz * vz) * V * w; break;
-            }
-          }
-        }
-  }
+  if (start)
+    for_each_within(p, h, P.mask, start, xv, s_list, [&](uint32_t j, const R4<R>& xj, double r2) {
+      const double w = kernel_w_r2<double>(r2, kd);
+      const double V = (double)xj.w;
+      if (quantity == 1) { s += V0 * w; return; }
+      const R4<R> vj = vel[j];
+      const double vx = (double)vj.x, vy = (double)vj.y, vz = (double)vj.z, m = (double)vj.w;
+      switch (quantity) {
+        case 0: sx += vx * V * w; sy += vy * V * w; sz += vz * V * w; break;
+        case 2: s += m * w; break;
+        case 3: if (m < V0) s += (V0 / m - 1.0) * m * w; break;
+        case 4: s += (double)press[j] * V * w; break;
+        default: s += 0.5 * m * ((vx * vx + vy * vy) + vz * vz) * V * w; break;
+      }
+    });
   if (quantity <= 1) {
-    if (G.start) {
-      for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy)
-          for (int dx = -1; dx <= 1; ++dx) {
-            const uint32_t k = morton_key(cx + dx, cy + dy, cz + dz, G.mask);
-            const uint32_t e = G.start[k + 1];
-            for (uint32_t j = G.start[k]; j < e; ++j) {
-              const R4<R> xs = G.xb[j];
-              const double qx = (double)xs.x, qy = (double)xs.y, qz = (double)xs.z;
-              if (!in_range_exact(p[0], p[1], p[2], qx, qy, qz, h)) continue;
-              const double rx = p[0] - qx, ry = p[1] - qy, rz = p[2] - qz;
-              const double vw = (double)xs.w * kernel_w_r2<double>((rx * rx + ry * ry) + rz * rz, kd);
-              if (quantity == 1) {
-                s += vw;
-              } else {
-                const R4<R> vs = G.vb[j];
-                sx += (double)vs.x * vw; sy += (double)vs.y * vw; sz += (double)vs.z * vw;
-              }
-            }
-          }
-    }
+    if (G.start)
+      for_each_within(p, h, G.mask, G.start, G.xb, s_list, [&](uint32_t j, const R4<R>& xs, double r2) {
+        const double vw = (double)xs.w * kernel_w_r2<double>(r2, kd);
+        if (quantity == 1) {
+          s += vw;
+        } else {
+          const R4<R> vs = G.vb[j];
+          sx += (double)vs.x * vw; sy += (double)vs.y * vw; sz += (double)vs.z * vw;
+        }
+      });
     const double ball = 4.0 / 3.0 * 3.14159265358979323846 * (h * h * h);
     for (int b = 0; b < nvm; ++b) {
       const VMDesc& D = vms[b];

@@ -45,22 +45,11 @@ template <class R, class F>
 __device__ __forceinline__ double surf_gather(const double p[3], double h, uint32_t mask,
                                               const uint32_t* __restrict__ start, const R4<R>* __restrict__ xv,
                                               const uint32_t* __restrict__ fid, uint32_t group, F f) {
-  const int cx = cell_coord(p[0], h), cy = cell_coord(p[1], h), cz = cell_coord(p[2], h);
+  __shared__ uint32_t s_list[kNearList * kBlock];
   double s = 0.0;
-  for (int dz = -1; dz <= 1; ++dz)
-    for (int dy = -1; dy <= 1; ++dy)
-      for (int dx = -1; dx <= 1; ++dx) {
-        const uint32_t k = morton_key(cx + dx, cy + dy, cz + dz, mask);
-        const uint32_t e = start[k + 1];
-        for (uint32_t j = start[k]; j < e; ++j) {
-          if (fid[j] != group) continue;
-          const R4<R> x = xv[j];
-          const double qx = (double)x.x, qy = (double)x.y, qz = (double)x.z;
-          if (!in_range_exact(p[0], p[1], p[2], qx, qy, qz, h)) continue;
-          const double rx = p[0] - qx, ry = p[1] - qy, rz = p[2] - qz;
-          s += f(j) * surf_w((rx * rx + ry * ry) + rz * rz, h);
-        }
-      }
+  for_each_within(p, h, mask, start, xv, s_list, [&](uint32_t j, const R4<R>&, double r2) {
+    if (fid[j] == group) s += f(j) * surf_w(r2, h);
+  });
   return s;
 }
 
@@ -90,20 +79,44 @@ __host__ __device__ inline double surf_unkey(unsigned long long k) {
   return v;
 }
 
-// bounds[0..2] = min keys, bounds[3..5] = max keys, bounds[6] = particle count
+// bounds[0..2] = min keys, bounds[3..5] = max keys, bounds[6] = the group's
+// first particle in reference order (reference index << 32 | sorted index; all
+// ones without particles). A warp reduces before it touches the seven words
+// (one atomic per particle and word serialised to 261 us for 64 thousand).
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_surf_bounds(int n, const R4<R>* __restrict__ xv,
-                                                       const uint32_t* __restrict__ fid, uint32_t group,
+                                                       const uint32_t* __restrict__ fid,
+                                                       const uint32_t* __restrict__ ref, uint32_t group,
                                                        unsigned long long* __restrict__ bounds) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || fid[i] != group) return;
-  const R4<R> x = xv[i];
-  const double p[3] = {(double)x.x, (double)x.y, (double)x.z};
-  for (int d = 0; d < 3; ++d) {
-    atomicMin(&bounds[d], surf_key(p[d]));
-    atomicMax(&bounds[3 + d], surf_key(p[d]));
+  unsigned long long lo[4] = {~0ull, ~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    if (fid[i] != group) continue;
+    const R4<R> x = xv[i];
+    const double p[3] = {(double)x.x, (double)x.y, (double)x.z};
+    for (int d = 0; d < 3; ++d) {
+      const unsigned long long k = surf_key(p[d]);
+      lo[d] = k < lo[d] ? k : lo[d];
+      hi[d] = k > hi[d] ? k : hi[d];
+    }
+    const unsigned long long r = (unsigned long long)ref[i] << 32 | (unsigned)i;
+    lo[3] = r < lo[3] ? r : lo[3];
   }
-  atomicAdd(&bounds[6], 1ull);
+  for (int o = 16; o > 0; o >>= 1) {
+    for (int d = 0; d < 4; ++d) {
+      const unsigned long long k = __shfl_down_sync(0xffffffffu, lo[d], o);
+      lo[d] = k < lo[d] ? k : lo[d];
+    }
+    for (int d = 0; d < 3; ++d) {
+      const unsigned long long k = __shfl_down_sync(0xffffffffu, hi[d], o);
+      hi[d] = k > hi[d] ? k : hi[d];
+    }
+  }
+  if ((threadIdx.x & 31) != 0 || lo[3] == ~0ull) return;
+  for (int d = 0; d < 3; ++d) {
+    atomicMin(&bounds[d], lo[d]);
+    atomicMax(&bounds[3 + d], hi[d]);
+  }
+  atomicMin(&bounds[6], lo[3]);
 }
 
 // The lattice: point (i, j, k) at cube * (k0 + (i, j, k)), n points per axis.
@@ -116,18 +129,27 @@ __device__ __forceinline__ double surf_coord(const SurfaceLattice& L, int d, lon
   return L.cube * (double)(L.k0[d] + k);
 }
 
+// A warp takes a brick of 4 x 4 x 2 points (0.75 h wide), whose lanes walk the
+// same few cells: 64 thousand particles' lattice of 1.4 million points took
+// 758 us with 32 points in a row and the f64 predicate for every candidate,
+// 586 us now (issue of the f32 tests and the f64 kernel values).
 template <class R>
-__global__ void __launch_bounds__(kBlock) k_surf_levelset(SurfaceLattice L, long long npoints,
+__global__ void __launch_bounds__(kBlock) k_surf_levelset(SurfaceLattice L, long long nbricks,
                                                          const uint32_t* __restrict__ start,
                                                          const R4<R>* __restrict__ xv,
                                                          const uint32_t* __restrict__ fid, uint32_t group,
                                                          const double* __restrict__ vol, double h, uint32_t mask,
                                                          double* __restrict__ phi) {
-  const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= npoints) return;
-  const long long i = q % L.n[0], j = (q / L.n[0]) % L.n[1], k = q / (L.n[0] * L.n[1]);
+  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (w >= nbricks) return;
+  const int lane = threadIdx.x & 31;
+  const long long b0 = (L.n[0] + 3) / 4, b1 = (L.n[1] + 3) / 4;
+  const long long i = 4 * (w % b0) + (lane & 3), j = 4 * ((w / b0) % b1) + ((lane >> 2) & 3),
+                  k = 2 * (w / (b0 * b1)) + (lane >> 4);
+  if (i >= L.n[0] || j >= L.n[1] || k >= L.n[2]) return;
   const double p[3] = {surf_coord(L, 0, i), surf_coord(L, 1, j), surf_coord(L, 2, k)};
-  phi[q] = surf_gather(p, h, mask, start, xv, fid, group, [&](uint32_t jj) { return vol[jj]; });
+  phi[(k * L.n[1] + j) * L.n[0] + i] =
+      surf_gather(p, h, mask, start, xv, fid, group, [&](uint32_t jj) { return vol[jj]; });
 }
 
 // flag[3 q + d] = 1 when the edge from point q along d crosses the iso value

@@ -15,6 +15,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
@@ -227,6 +228,7 @@ class System : public SystemBase {
     vint_.zero(stream_);
     host_bbox_.clear();
     for (size_t i = 0; i < n; ++i) bbox_add(x[3 * i], x[3 * i + 1], x[3 * i + 2]);
+    note_groups(fid, n);
     fluid_uploaded_ = true;
   }
 
@@ -502,13 +504,6 @@ class System : public SystemBase {
     if (chunk_steps_) throw Error(SPH_ERR_STATE, "a chunk of graph steps is in flight");
     const size_t n = n_;
     if (n == 0) return;
-    std::vector<uint32_t> ids(n);
-    fluid_ids(ids.data());
-    std::vector<double> mass(n);
-    download(SPH_FIELD_MASS, mass.data());
-    std::map<uint32_t, double> groups;
-    for (size_t i = 0; i < n; ++i)
-      if (!groups.count(ids[i])) groups[ids[i]] = mass[i];
     static const SurfaceCases cases = surface_case_table();
     const double h = cfg_.kernel_support_radius, sp = cfg_.rest_density_grid_spacing;
     const double V0 = sp * sp * sp, r = 0.5 * sp, cube = 0.75 * r;
@@ -528,17 +523,18 @@ class System : public SystemBase {
       launch("surface_scan", k_scan_apply, dim3((unsigned)tiles), dim3(kBlock), count, (int)m,
              (const uint32_t*)surf_tiles_.p, outp);
     };
-    for (const auto& g : groups) {
-      const uint32_t group = g.first;
-      const double rest_density = g.second / V0;
+    for (const uint32_t group : group_ids_) {  // (ascending; some may have lost all their particles)
+      const unsigned long long init[7] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull, ~0ull};
+      copy_h2d(surf_bounds_.p, init, 7);
+      launch("surface_bounds", k_surf_bounds<R>, dim3(std::min(nb, 2 * 148)), dim3(kBlock), (int)n,
+             (const R4<R>*)xv_.p, (const uint32_t*)fid_.p, (const uint32_t*)ref_.p, group, surf_bounds_.p);
+      std::vector<unsigned long long> bk = fetch(surf_bounds_.p, 7);
+      if (bk[6] == ~0ull) continue;
+      const double mass = (double)fetch(vel_.p + (uint32_t)bk[6], 1)[0].w;  // of the group's first particle
+      const double rest_density = mass / V0;
       const double m = rest_density * (4.0 / 3.0 * 3.14159265358979323846 * (r * r * r));
       launch("surface_density", k_surf_density<R>, dim3(nb), dim3(kBlock), (int)n, (const uint32_t*)start_.p,
              (const R4<R>*)xv_.p, (const uint32_t*)fid_.p, group, m, h, mask_, surf_vol_.p);
-      const unsigned long long init[7] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull, 0ull};
-      copy_h2d(surf_bounds_.p, init, 7);
-      launch("surface_bounds", k_surf_bounds<R>, dim3(nb), dim3(kBlock), (int)n, (const R4<R>*)xv_.p,
-             (const uint32_t*)fid_.p, group, surf_bounds_.p);
-      std::vector<unsigned long long> bk = fetch(surf_bounds_.p, 7);
       SurfaceLattice L;
       L.cube = cube;
       double npts = 1.0;
@@ -558,7 +554,8 @@ class System : public SystemBase {
       grow(surf_vid_, (size_t)(3 * np + 1));
       grow(surf_tris_, (size_t)(nc + 1));
       grow(surf_toff_, (size_t)(nc + 1));
-      launch("surface_levelset", k_surf_levelset<R>, blocks(np), dim3(kBlock), L, np, (const uint32_t*)start_.p,
+      const long long bricks = ((L.n[0] + 3) / 4) * ((L.n[1] + 3) / 4) * ((L.n[2] + 1) / 2);
+      launch("surface_levelset", k_surf_levelset<R>, blocks(32 * bricks), dim3(kBlock), L, bricks, (const uint32_t*)start_.p,
              (const R4<R>*)xv_.p, (const uint32_t*)fid_.p, group, (const double*)surf_vol_.p, h, mask_,
              surf_phi_.p);
       launch("surface_edges", k_surf_edges, blocks(np), dim3(kBlock), L, np, (const double*)surf_phi_.p,
@@ -829,6 +826,7 @@ class System : public SystemBase {
   int K_ = 64;
   uint32_t T_ = 64, mask_ = 3;
   bool fluid_uploaded_ = false, initialized_ = false;
+  std::set<uint32_t> group_ids_;
   uint64_t steps_ = 0;
   double current_time_ = 0, time_offset_ = 0, wall_ = 0, avg_density_ = 0;
   uint64_t time_offset_steps_ = 0;
@@ -903,6 +901,13 @@ class System : public SystemBase {
   BBox& host_bbox_ = bbox_;
 
   // ---- helpers ---------------------------------------------------------------
+  // The fluid ids that the state may hold (disabling particles only removes some).
+  void note_groups(const uint32_t* fid, size_t n) {
+    group_ids_.clear();
+    if (!fid) group_ids_.insert(0u);
+    for (size_t i = 0; fid && i < n; ++i)
+      if (i == 0 || fid[i] != fid[i - 1]) group_ids_.insert(fid[i]);
+  }
   void bbox_add(double x, double y, double z) {
     const double p[3] = {x, y, z};
     if (!bbox_.any) {
@@ -2089,6 +2094,7 @@ void System<R>::restore(uint64_t steps, double time, size_t n, const double* x, 
   copy_h2d(vel_.p, hv.data(), n);
   copy_h2d(ref_.p, hr.data(), n);
   copy_h2d(fid_.p, hf.data(), n);
+  note_groups(fid, n);
   if (cfg_.integration_scheme == SPH_TAKE_PREDICTED) {
     if (xi) copy_h2d(xint_.p, hxi.data(), n); else xint_.zero(stream_);
     if (vi) copy_h2d(vint_.p, hvi.data(), n); else vint_.zero(stream_);
