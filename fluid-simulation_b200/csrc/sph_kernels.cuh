@@ -2794,6 +2794,13 @@ __global__ void __launch_bounds__(kBlock) k_sample_volumes(const int* __restrict
   xb[d] = o;
 }
 
+// The scalars of the next update, as k_step_epilogue leaves them.
+__global__ void k_next_update(Scalars* sc) {
+  sc->n = sc->n_active;
+  sc->n_below = 0;
+  sc->max_speed = 0;
+}
+
 // ---------------------------------------------------------------------------
 // graph-captured stepping
 // ---------------------------------------------------------------------------

@@ -131,6 +131,18 @@ __global__ void k_state_in(int n, const uint32_t* __restrict__ ref, const double
     vel[d] = q;
   }
 }
+// A whole state from host arrays (checkpoints, uploads): particle i is row i.
+// With no position, only the given integrator slots are written.
+template <class R>
+__global__ void k_state_load(int n, const double* __restrict__ x, const double* __restrict__ v,
+                             const double* __restrict__ m, R4<R>* __restrict__ pos, R4<R>* __restrict__ vel,
+                             uint32_t* __restrict__ ref) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  if (pos) pos[i] = R4<R>{(R)x[3 * i], (R)x[3 * i + 1], (R)x[3 * i + 2], R(0)};
+  if (vel) vel[i] = R4<R>{v ? (R)v[3 * i] : R(0), v ? (R)v[3 * i + 1] : R(0), v ? (R)v[3 * i + 2] : R(0), (R)m[i]};
+  if (ref) ref[i] = (uint32_t)i;
+}
 template <class R>
 __global__ void k_state_out(int n, const uint32_t* __restrict__ ref, const R4<R>* __restrict__ xv,
                             const R4<R>* __restrict__ vel, double* __restrict__ x, double* __restrict__ v) {
@@ -197,6 +209,9 @@ class System : public SystemBase {
     }
     if (h_sc_) cudaFreeHost(h_sc_);
     if (h_meas_) cudaFreeHost(h_meas_);
+    if (h_slice_) cudaFreeHost(h_slice_);
+    for (cudaEvent_t e : slice_event_)
+      if (e) cudaEventDestroy(e);
     if (stream_) cudaStreamDestroy(stream_);
   }
 
@@ -210,19 +225,7 @@ class System : public SystemBase {
     cap_ = std::max<size_t>(n, 1);
     np_ = round_up(cap_, 32);
     alloc_particles();
-    std::vector<R4<R>> hp(cap_), hv(cap_);
-    std::vector<uint32_t> hr(cap_), hf(cap_);
-    for (size_t i = 0; i < n; ++i) {
-      hp[i] = R4<R>{(R)x[3 * i], (R)x[3 * i + 1], (R)x[3 * i + 2], R(0)};
-      const double vx = v ? v[3 * i] : 0.0, vy = v ? v[3 * i + 1] : 0.0, vz = v ? v[3 * i + 2] : 0.0;
-      hv[i] = R4<R>{(R)vx, (R)vy, (R)vz, (R)m[i]};
-      hr[i] = (uint32_t)i;
-      hf[i] = fid ? fid[i] : 0u;
-    }
-    copy_h2d(pos_.p, hp.data(), cap_);
-    copy_h2d(vel_.p, hv.data(), cap_);
-    copy_h2d(ref_.p, hr.data(), cap_);
-    copy_h2d(fid_.p, hf.data(), cap_);
+    load_state(n, x, v, m, fid);
     acc_.zero(stream_);
     xint_.zero(stream_);
     vint_.zero(stream_);
@@ -582,8 +585,8 @@ class System : public SystemBase {
       launch("surface_normals", k_surf_normalize, blocks(nv), dim3(kBlock), (long long)nv, surf_vtx_.p);
       SurfaceMeshOut mo;
       mo.fluid_id = group;
-      mo.vertices = fetch(surf_vtx_.p, (size_t)nv * 6);
-      mo.indices = fetch(surf_idx_.p, (size_t)nt * 3);
+      fetch_into(mo.vertices, surf_vtx_.p, (size_t)nv * 6);
+      fetch_into(mo.indices, surf_idx_.p, (size_t)nt * 3);
       out.push_back(std::move(mo));
     }
   }
@@ -681,8 +684,8 @@ class System : public SystemBase {
       cuda_check(cudaEventCreateWithFlags(&io_ready_, cudaEventDisableTiming), "cudaEventCreate");
     }
     if (xi || vi) {
-      stage_x_.alloc(std::max<size_t>(n3, 3));
-      stage_v_.alloc(std::max<size_t>(n3, 3));
+      stage_x_.alloc(std::max<size_t>(3 * cap_, 3));
+      stage_v_.alloc(std::max<size_t>(3 * cap_, 3));
       // positions and velocities travel on two streams, so two copy engines
       // can carry them at once
       if (xi) cuda_check(cudaMemcpyAsync(stage_x_.p, xi, n3 * sizeof(double), cudaMemcpyHostToDevice, stream_), "H2D");
@@ -704,8 +707,8 @@ class System : public SystemBase {
     early_done_ = false;
     if ((xo || vo) && nsteps > 0) {
       if (nsteps > 1) st = step(nsteps - 1);
-      stage_x_.alloc(std::max<size_t>(n3, 3));
-      stage_v_.alloc(std::max<size_t>(n3, 3));
+      stage_x_.alloc(std::max<size_t>(3 * cap_, 3));
+      stage_v_.alloc(std::max<size_t>(3 * cap_, 3));
       early_xo_ = xo;
       early_vo_ = vo;
       const size_t n_before = n_;
@@ -725,8 +728,8 @@ class System : public SystemBase {
       st = step(nsteps);
     }
     if (xo || vo) {
-      stage_x_.alloc(std::max<size_t>(n3, 3));
-      stage_v_.alloc(std::max<size_t>(n3, 3));
+      stage_x_.alloc(std::max<size_t>(3 * cap_, 3));
+      stage_v_.alloc(std::max<size_t>(3 * cap_, 3));
       launch("state_io", k_state_out<R>, dim3(blocks_for((long long)n_)), dim3(kBlock), (int)n_,
              (const uint32_t*)ref_.p, (const R4<R>*)xv_.p, (const R4<R>*)vel_.p, xo ? stage_x_.p : nullptr,
              vo ? stage_v_.p : nullptr);
@@ -782,7 +785,7 @@ class System : public SystemBase {
                           &tile_sums_, &sbid_, &sbid2_, &sorig_, &sorig2_, &skey_, &sslot_, &sperm_, &scount_,
                           &sstart_, &snap_ref_, &snap_fid_})
       b += d->bytes();
-    b += partials_.bytes() + body_partials_.bytes() + stage_x_.bytes() + stage_v_.bytes();
+    b += partials_.bytes() + body_partials_.bytes() + stage_x_.bytes() + stage_v_.bytes() + stage_m_.bytes();
     b += eval_pos_.bytes() + eval_out_.bytes();
     b += surf_vol_.bytes() + surf_phi_.bytes() + surf_vtx_.bytes() + surf_flag_.bytes() + surf_vid_.bytes() +
          surf_tris_.bytes() + surf_toff_.bytes() + surf_idx_.bytes() + surf_tiles_.bytes() + surf_bounds_.bytes();
@@ -819,6 +822,8 @@ class System : public SystemBase {
   bool early_done_ = false;
   Scalars* h_sc_ = nullptr;
   double* h_meas_ = nullptr;
+  char* h_slice_ = nullptr;  // pinned slices of large readbacks (first use)
+  cudaEvent_t slice_event_[2] = {nullptr, nullptr};
   DBuf<Scalars> d_sc_;
   DBuf<double> d_meas_;
   StepParams<R> P_{};
@@ -830,7 +835,7 @@ class System : public SystemBase {
   uint64_t steps_ = 0;
   double current_time_ = 0, time_offset_ = 0, wall_ = 0, avg_density_ = 0;
   uint64_t time_offset_steps_ = 0;
-  int last_iters_ = 3;
+  double sweep_decay_ = 0.1;  // decay of the solver's error per sweep, last seen (ln of the ratio)
   int nb_ = 4;  // neighbor gather batch (prefetch width) of the neighbor passes
   bool pdl_ = true;       // programmatic dependent launch between the sweep passes
   bool prefetch_ = true;  // sweep passes prefetch the next wave's streams into L2
@@ -859,7 +864,7 @@ class System : public SystemBase {
   // blocks share an SM's shared memory)
   int sweep_hs_ = sizeof(R) == 4 ? 1792 : 1024;
   DBuf<uint32_t> count_, start_, tile_sums_;
-  DBuf<double> partials_, body_partials_, stage_x_, stage_v_;
+  DBuf<double> partials_, body_partials_, stage_x_, stage_v_, stage_m_;
   // boundaries
   std::vector<Body> bodies_;
   DBuf<Body> bodies_d_;
@@ -901,6 +906,30 @@ class System : public SystemBase {
   BBox& host_bbox_ = bbox_;
 
   // ---- helpers ---------------------------------------------------------------
+  template <class T>
+  void h2d(T* dst, const T* src, size_t n) {
+    if (n) cuda_check(cudaMemcpyAsync(dst, src, n * sizeof(T), cudaMemcpyHostToDevice, stream_), "cudaMemcpy H2D");
+  }
+  void load_rows(size_t n, const double* x, const double* v, R4<R>* pos, R4<R>* vel, uint32_t* ref) {
+    if (n)
+      launch("state_io", k_state_load<R>, dim3(blocks_for((long long)n)), dim3(kBlock), (int)n, x, v,
+             (const double*)stage_m_.p, pos, vel, ref);
+  }
+  // Positions, velocities (null: zero), masses and fluid ids (null: zero) from
+  // host arrays in reference order; converted on the device. The copies are
+  // done when it returns (the arrays are the caller's).
+  void load_state(size_t n, const double* x, const double* v, const double* m, const uint32_t* fid) {
+    stage_x_.alloc(std::max<size_t>(3 * cap_, 3));
+    stage_v_.alloc(std::max<size_t>(3 * cap_, 3));
+    stage_m_.alloc(std::max<size_t>(cap_, 1));
+    h2d(stage_x_.p, x, 3 * n);
+    if (v) h2d(stage_v_.p, v, 3 * n);
+    h2d(stage_m_.p, m, n);
+    if (fid) h2d(fid_.p, fid, n);
+    else fid_.zero(stream_);
+    load_rows(n, stage_x_.p, v ? stage_v_.p : nullptr, pos_.p, vel_.p, ref_.p);
+    sync();
+  }
   // The fluid ids that the state may hold (disabling particles only removes some).
   void note_groups(const uint32_t* fid, size_t n) {
     group_ids_.clear();
@@ -934,6 +963,31 @@ class System : public SystemBase {
       sync();
     }
     return h;
+  }
+  // A large readback through pinned memory in slices, each copied out while the
+  // next one travels, into a vector that is filled once (not zeroed first).
+  template <class T>
+  void fetch_into(std::vector<T>& out, const T* src, size_t n) {
+    constexpr size_t slice = (size_t)1 << 20;
+    if (!h_slice_) {
+      cuda_check(cudaMallocHost((void**)&h_slice_, 2 * slice), "cudaMallocHost");
+      for (cudaEvent_t& e : slice_event_) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    }
+    const size_t per = slice / sizeof(T), count = (n + per - 1) / per;
+    auto request = [&](size_t k) {
+      const size_t at = k * per, m = std::min(per, n - at);
+      cuda_check(cudaMemcpyAsync(h_slice_ + (k & 1) * slice, src + at, m * sizeof(T), cudaMemcpyDeviceToHost, stream_), "D2H");
+      cuda_check(cudaEventRecord(slice_event_[k & 1], stream_), "event");
+    };
+    out.clear();
+    out.reserve(n);
+    for (size_t k = 0; k < std::min<size_t>(2, count); ++k) request(k);
+    for (size_t k = 0; k < count; ++k) {
+      cuda_check(cudaEventSynchronize(slice_event_[k & 1]), "event");
+      const T* h = reinterpret_cast<const T*>(h_slice_ + (k & 1) * slice);
+      out.insert(out.end(), h, h + std::min(per, n - k * per));
+      if (k + 2 < count) request(k + 2);
+    }
   }
   void sync() { cuda_check(cudaStreamSynchronize(stream_), "cudaStreamSynchronize"); }
   void need_iisph() {
@@ -1464,22 +1518,34 @@ class System : public SystemBase {
       solve_loop_graph();
       return;
     }
-    int batch = after >= 0 ? after + 1 : std::max(3, last_iters_);
+    // A solve takes three sweeps at least; then the host reads the flag and the
+    // error. Each further batch is as long as the error's decay per sweep (of
+    // this solve so far, else of the last one) says that the solve still needs:
+    // a check costs the stream about 12 us of idling, a sweep launched in vain
+    // 11 us (133 thousand particles) to 25 us (one million), and a batch as long
+    // as the last solve launched up to 19 of those when a solve of 22 sweeps was
+    // followed by one of 3. Timed (profiling) solves run one sweep per check, so
+    // that every timed sweep launch does a sweep's work; the results are the same.
+    int batch = after >= 0 ? after + 1 : profiling_ ? 1 : 3;
     if (after < 0 && cfg_.max_solver_iterations) batch = std::min(batch, (int)cfg_.max_solver_iterations);
-    // Timed (profiling) solves run one sweep per host check, so that every
-    // timed sweep launch does a sweep's work (no launch that finds the loop
-    // converged and returns); the results are the same either way.
-    if (profiling_ && after < 0) batch = 1;
     for (int k = 0; k < batch; ++k) iisph_iteration(after, k == 0);
     if (after >= 0) return;
-    int launched = batch;
+    double err_before = 0.0;
+    int sweeps_before = 0;
     for (;;) {
-      cuda_check(cudaMemcpyAsync(&h_sc_->converged, &d_sc_.p->converged, sizeof(int), cudaMemcpyDeviceToHost, stream_), "memcpy");
+      cuda_check(cudaMemcpyAsync(h_sc_, d_sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, stream_), "memcpy");
       sync();
+      const double err = h_sc_->err;
+      const int sweeps = h_sc_->iterations;
+      if (sweeps_before > 0 && sweeps > sweeps_before && err > 0.0 && err < err_before)
+        sweep_decay_ = std::log(err_before / err) / (sweeps - sweeps_before);
       if (h_sc_->converged) break;
-      const int more = profiling_ ? 1 : launched < 16 ? 2 : 4;
-      for (int k = 0; k < more; ++k) iisph_iteration(after, false);
-      launched += more;
+      double need = cfg_.target_density_error > 0.0 && err > cfg_.target_density_error && std::isfinite(err)
+                        ? std::log(err / cfg_.target_density_error) / sweep_decay_ : 2.0;
+      batch = profiling_ ? 1 : (int)std::min(64.0, std::max(2.0, std::ceil(need)));
+      for (int k = 0; k < batch; ++k) iisph_iteration(after, false);
+      err_before = err;
+      sweeps_before = sweeps;
     }
   }
 
@@ -1547,7 +1613,6 @@ class System : public SystemBase {
     sync();
     collect_profile();
     avg_density_ = h_sc_->avg_density;
-    if (h_sc_->iterations > 0) last_iters_ = h_sc_->iterations;
     if (h_sc_->max_nbrs > K_ || h_sc_->max_halo > hcap_) {
       // Neighbor or halo capacity exceeded: grow it and redo the update on
       // the same (already integrated) state. Reaction forces gathered so far
@@ -1684,7 +1749,7 @@ class System : public SystemBase {
       copy_h2d(ref_.p, ref_all.data(), n_new);
       n_ = n_new;
     }
-    copy_h2d(d_sc_.p, &next, 1);
+    launch("next_update", k_next_update, dim3(1), dim3(1), d_sc_.p);
     *h_sc_ = next;
   }
 
@@ -1783,7 +1848,6 @@ class System : public SystemBase {
     steps_ += c;
     if (cfg_.cfl_time_step) current_time_ = s.time_acc;
     avg_density_ = s.avg_density;
-    if (s.iterations > 0) last_iters_ = s.iterations;
     launches_ += (uint64_t)c * graphs_[0].kernels + 3ull * s.loop_sweeps;
     wall_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - chunk_t0_).count() / c;
     o.status = s.status_any == 2 ? SPH_NOT_CONVERGED : SPH_OK;
@@ -2080,24 +2144,21 @@ void System<R>::restore(uint64_t steps, double time, size_t n, const double* x, 
   if (!initialized_) throw Error(SPH_ERR_STATE, "initialize before restoring a checkpoint");
   if (n > cap_) throw Error(SPH_ERR_INVALID, "checkpoint holds more particles than the system");
   n_ = n;
-  std::vector<R4<R>> hp(n), hv(n), hxi(n), hvi(n);
-  std::vector<uint32_t> hr(n), hf(n);
-  for (size_t i = 0; i < n; ++i) {
-    hp[i] = R4<R>{(R)x[3 * i], (R)x[3 * i + 1], (R)x[3 * i + 2], R(0)};
-    hv[i] = R4<R>{(R)v[3 * i], (R)v[3 * i + 1], (R)v[3 * i + 2], (R)m[i]};
-    hr[i] = (uint32_t)i;
-    hf[i] = fid ? fid[i] : 0u;
-    if (xi) hxi[i] = R4<R>{(R)xi[3 * i], (R)xi[3 * i + 1], (R)xi[3 * i + 2], R(0)};
-    if (vi) hvi[i] = R4<R>{(R)vi[3 * i], (R)vi[3 * i + 1], (R)vi[3 * i + 2], (R)m[i]};
-  }
-  copy_h2d(pos_.p, hp.data(), n);
-  copy_h2d(vel_.p, hv.data(), n);
-  copy_h2d(ref_.p, hr.data(), n);
-  copy_h2d(fid_.p, hf.data(), n);
+  load_state(n, x, v, m, fid);
   note_groups(fid, n);
   if (cfg_.integration_scheme == SPH_TAKE_PREDICTED) {
-    if (xi) copy_h2d(xint_.p, hxi.data(), n); else xint_.zero(stream_);
-    if (vi) copy_h2d(vint_.p, hvi.data(), n); else vint_.zero(stream_);
+    if (xi) {
+      h2d(stage_x_.p, xi, 3 * n);
+      load_rows(n, stage_x_.p, nullptr, xint_.p, nullptr, nullptr);
+    } else {
+      xint_.zero(stream_);
+    }
+    if (vi) {
+      h2d(stage_v_.p, vi, 3 * n);
+      load_rows(n, nullptr, stage_v_.p, nullptr, vint_.p, nullptr);
+    } else {
+      vint_.zero(stream_);
+    }
   }
   acc_.zero(stream_);
   steps_ = steps;
