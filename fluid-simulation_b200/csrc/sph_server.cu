@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "sph_host.hpp"
+#include "sph_pool.hpp"
 
 namespace sph {
 
@@ -230,6 +231,7 @@ class Server {
   }
 
  private:
+  PoolUse pool_;  // the scenes' memory is reused from scene to scene
   sph_server_config cfg_;
   uint64_t budget_ = 0;
   Clock::time_point t0_;

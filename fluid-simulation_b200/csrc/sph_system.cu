@@ -25,6 +25,7 @@
 #include "sph_fields.cuh"
 #include "sph_formats.hpp"
 #include "sph_host.hpp"
+#include "sph_pool.hpp"
 #include "sph_kernels.cuh"
 #include "sph_surface.cuh"
 
@@ -43,8 +44,9 @@ struct DBuf {
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
   ~DBuf() { release(); }
+  // (no stream uses a buffer that is released or allocated anew)
   void release() {
-    if (p) cudaFree(p);
+    Pool::get().free(p);
     p = nullptr;
     n = 0;
   }
@@ -52,7 +54,9 @@ struct DBuf {
     if (count == n && p) return;
     release();
     if (count == 0) return;
-    cuda_check(cudaMalloc((void**)&p, count * sizeof(T)), "cudaMalloc");
+    int dev = 0;
+    cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+    p = static_cast<T*>(Pool::get().alloc(count * sizeof(T), dev));
     n = count;
   }
   void zero(cudaStream_t s) {
@@ -183,33 +187,32 @@ class System : public SystemBase {
     }
     cuda_check(cudaSetDevice(c.device), "cudaSetDevice");
     cuda_check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
-    cuda_check(cudaMallocHost((void**)&h_sc_, sizeof(Scalars)), "cudaMallocHost");
-    cuda_check(cudaMallocHost((void**)&h_meas_, 2 * sizeof(double)), "cudaMallocHost");
+    h_sc_ = static_cast<Scalars*>(Pool::get().alloc(sizeof(Scalars), Pool::kHost));
+    h_meas_ = static_cast<double*>(Pool::get().alloc(2 * sizeof(double), Pool::kHost));
     d_sc_.alloc(1);
     d_meas_.alloc(2);
     std::memset(h_sc_, 0, sizeof(Scalars));
     upload_serendipity_tables();
   }
   ~System() override {
-    if (chunk_steps_) cudaEventSynchronize(chunk_event_);
+    // everything the streams still run ends before the buffers go back to the pool
+    if (stream_) cudaStreamSynchronize(stream_);
+    if (io_stream_) cudaStreamSynchronize(io_stream_);
     destroy_graphs();
     if (chunk_event_) cudaEventDestroy(chunk_event_);
     if (body_stream_) cudaStreamDestroy(body_stream_);
-    if (io_stream_) {
-      cudaStreamSynchronize(io_stream_);
-      cudaStreamDestroy(io_stream_);
-    }
+    if (io_stream_) cudaStreamDestroy(io_stream_);
     if (io_ready_) cudaEventDestroy(io_ready_);
-    if (h_chunk_sc_) cudaFreeHost(h_chunk_sc_);
+    Pool::get().free(h_chunk_sc_);
     for (auto& kv : prof_) {
       for (auto& e : kv.second.pool) {
         cudaEventDestroy(e.first);
         cudaEventDestroy(e.second);
       }
     }
-    if (h_sc_) cudaFreeHost(h_sc_);
-    if (h_meas_) cudaFreeHost(h_meas_);
-    if (h_slice_) cudaFreeHost(h_slice_);
+    Pool::get().free(h_sc_);
+    Pool::get().free(h_meas_);
+    Pool::get().free(h_slice_);
     for (cudaEvent_t e : slice_event_)
       if (e) cudaEventDestroy(e);
     if (stream_) cudaStreamDestroy(stream_);
@@ -811,6 +814,7 @@ class System : public SystemBase {
     size_t used = 0;
   };
 
+  PoolUse pool_;  // first member: released after every buffer
   sph_config cfg_;
   cudaStream_t stream_ = nullptr;
   uint32_t contact_fixed_sweeps_ = 0;  // 0: the reference's merit test
@@ -970,7 +974,7 @@ class System : public SystemBase {
   void fetch_into(std::vector<T>& out, const T* src, size_t n) {
     constexpr size_t slice = (size_t)1 << 20;
     if (!h_slice_) {
-      cuda_check(cudaMallocHost((void**)&h_slice_, 2 * slice), "cudaMallocHost");
+      h_slice_ = static_cast<char*>(Pool::get().alloc(2 * slice, Pool::kHost));
       for (cudaEvent_t& e : slice_event_) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
     }
     const size_t per = slice / sizeof(T), count = (n + per - 1) / per;
@@ -1893,7 +1897,7 @@ class System : public SystemBase {
     destroy_graphs();
     if (!body_stream_) cuda_check(cudaStreamCreateWithFlags(&body_stream_, cudaStreamNonBlocking), "cudaStreamCreate");
     if (!chunk_event_) cuda_check(cudaEventCreateWithFlags(&chunk_event_, cudaEventDisableTiming), "cudaEventCreate");
-    if (!h_chunk_sc_) cuda_check(cudaMallocHost((void**)&h_chunk_sc_, sizeof(Scalars)), "cudaMallocHost");
+    if (!h_chunk_sc_) h_chunk_sc_ = static_cast<Scalars*>(Pool::get().alloc(sizeof(Scalars), Pool::kHost));
     alloc_snapshot();
     // capturing swaps the host-side buffer pointers as a launch would; two
     // captures in a row bring them back to where they started
