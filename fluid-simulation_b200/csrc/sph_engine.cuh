@@ -43,6 +43,7 @@ struct Scalars {
   int n;                           // particles entering this update
   int n_active;                    // particles after disabling
   int n_below;                     // particles disabled in this update
+  int n_in, n_disabled;            // n and n_below of the last update (k_volume resets those)
   int max_nbrs;                    // largest fluid neighbor count seen
   int iterations;                  // IISPH sweeps of the last solve
   int converged;                   // IISPH loop flag (1 = stop)

@@ -164,12 +164,19 @@ __global__ void __launch_bounds__(kBlock) k_integrate_key(
 }
 
 // Step prologue: active count and the CFL time increment (sph/mod.rs:825-829).
-template <class R>
-__global__ void k_prologue(Scalars* sc, StepParams<R> P, int accumulate_time) {
+// One thread of the first scan kernel runs it: everything before it in the step
+// has ended there, and nothing before the scan's end reads its results.
+struct Prologue {
+  Scalars* sc;  // null: no prologue (other scans)
+  int cfl, accumulate_time;
+  double cfl_number, spacing, dt_max;
+};
+__device__ __forceinline__ void run_prologue(const Prologue& P) {
+  Scalars* sc = P.sc;
   sc->n_active = sc->n - sc->n_below;
   // simulated time of a CFL step advances by the increment it integrated with
   // (the one chosen by the previous update); graph-captured steps keep it here
-  if (accumulate_time) sc->time_acc += sc->dt;
+  if (P.accumulate_time) sc->time_acc += sc->dt;
   if (P.cfl) {
     const double ms = __longlong_as_double((long long)sc->max_speed);
     const double c = P.cfl_number * P.spacing / ms;  // +inf at rest
@@ -188,7 +195,10 @@ __global__ void k_prologue(Scalars* sc, StepParams<R> P, int accumulate_time) {
 }
 
 // ---------------------------------------------------------------------------
-// 2. exclusive scan of bucket counts (3 phases); clears the counts for reuse
+// 2. exclusive scan of bucket counts; clears the counts for reuse. Tile sums,
+// then every block adds up the tiles before its own (DIRECT); from kScanDirect
+// tiles on (2^22 buckets, large surface lattices) a kernel of its own scans the
+// tile sums in between.
 // ---------------------------------------------------------------------------
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kBlock * kScanItems;
@@ -231,9 +241,11 @@ __device__ __forceinline__ void scan_load8(const uint32_t* __restrict__ in, int 
   }
 }
 
+constexpr int kScanDirect = 2048;
 __global__ void __launch_bounds__(kBlock) k_scan_tiles(const uint32_t* __restrict__ in, int m,
-                                                      uint32_t* __restrict__ tile_sums) {
+                                                      uint32_t* __restrict__ tile_sums, Prologue prologue) {
   __shared__ uint32_t sh[32];
+  if (prologue.sc && blockIdx.x == 0 && threadIdx.x == 0) run_prologue(prologue);
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
   scan_load8(in, base, m, v);
@@ -261,6 +273,7 @@ __global__ void __launch_bounds__(1024) k_scan_tile_sums(uint32_t* __restrict__ 
     }
 }
 
+template <bool DIRECT>
 __global__ void __launch_bounds__(kBlock) k_scan_apply(uint32_t* __restrict__ in, int m,
                                                       const uint32_t* __restrict__ tile_sums,
                                                       uint32_t* __restrict__ out) {
@@ -271,7 +284,14 @@ __global__ void __launch_bounds__(kBlock) k_scan_apply(uint32_t* __restrict__ in
   uint32_t s = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) s += v[k];
-  uint32_t run = block_excl_scan_u32(s, sh, nullptr) + tile_sums[blockIdx.x];
+  uint32_t before = 0;
+  if (DIRECT) {
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += kBlock) before += tile_sums[t];
+    block_excl_scan_u32(before, sh, &before);
+  } else {
+    before = tile_sums[blockIdx.x];
+  }
+  uint32_t run = block_excl_scan_u32(s, sh, nullptr) + before;
   if (base + 8 <= m) {
     uint32_t o[8];
 #pragma unroll
@@ -297,7 +317,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_apply(uint32_t* __restrict__ in
 }
 
 // ---------------------------------------------------------------------------
-// 3. scatter, in-bucket ordering by reference index, gather
+// 3. scatter, then gather with in-bucket ordering by reference index
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kBlock) k_scatter(const int* __restrict__ n_ptr,
                                                    const uint32_t* __restrict__ key,
@@ -309,47 +329,38 @@ __global__ void __launch_bounds__(kBlock) k_scatter(const int* __restrict__ n_pt
   perm[start[key[i]] + slot[i]] = (uint32_t)i;
 }
 
-// The first slot of every bucket orders the bucket's entries by `order`
-// (the reference index), which makes the sorted order independent of the
-// atomic slot assignment.
-__global__ void __launch_bounds__(kBlock) k_bucket_order(const int* __restrict__ n_ptr,
-                                                        const uint32_t* __restrict__ key,
-                                                        const uint32_t* __restrict__ start,
-                                                        const uint32_t* __restrict__ order,
-                                                        uint32_t* __restrict__ perm) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= *n_ptr) return;
-  const uint32_t k = key[perm[d]];
-  const uint32_t b = start[k];
-  if ((uint32_t)d != b) return;
-  const uint32_t e = start[k + 1];
-  for (uint32_t a = b + 1; a < e; ++a) {
-    const uint32_t pa = perm[a];
-    const uint32_t oa = order[pa];
-    uint32_t c = a;
-    while (c > b) {
-      const uint32_t pc = perm[c - 1];
-      if (order[pc] <= oa) break;
-      perm[c] = pc;
-      --c;
-    }
-    perm[c] = pa;
-  }
+// The place of sorted entry d in its bucket ordered by `order` (the reference
+// index), which makes the sorted order independent of the atomic slot
+// assignment: every entry counts the smaller ones of its bucket. (One thread
+// per bucket sorting by insertion took 14 to 25 us where a sphere's samples
+// crowd a bucket.)
+__device__ __forceinline__ uint32_t ranked_place(uint32_t j, const uint32_t* __restrict__ key,
+                                                 const uint32_t* __restrict__ start,
+                                                 const uint32_t* __restrict__ order,
+                                                 const uint32_t* __restrict__ perm) {
+  const uint32_t k = key[j], b = start[k], e = start[k + 1], mine = order[j];
+  uint32_t rank = 0;
+#pragma unroll 4
+  for (uint32_t t = b; t < e; ++t) rank += order[perm[t]] < mine ? 1u : 0u;
+  return b + rank;
 }
 
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_gather_particles(
-    const int* __restrict__ n_ptr, const uint32_t* __restrict__ perm,
-    const R4<R>* __restrict__ pos, const R4<R>* __restrict__ vel, const uint32_t* __restrict__ ref,
-    const uint32_t* __restrict__ fid, R4<R>* __restrict__ pos2, R4<R>* __restrict__ vel2,
-    uint32_t* __restrict__ ref2, uint32_t* __restrict__ fid2) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= *n_ptr) return;
-  const uint32_t j = perm[d];
-  pos2[d] = pos[j];
-  vel2[d] = vel[j];
-  ref2[d] = ref[j];
-  fid2[d] = fid[j];
+    const int* __restrict__ n_ptr, const uint32_t* __restrict__ perm, const uint32_t* __restrict__ key,
+    const uint32_t* __restrict__ start, const R4<R>* __restrict__ pos, const R4<R>* __restrict__ vel,
+    const uint32_t* __restrict__ ref, const uint32_t* __restrict__ fid, R4<R>* __restrict__ pos2,
+    R4<R>* __restrict__ vel2, uint32_t* __restrict__ ref2, uint32_t* __restrict__ fid2) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= *n_ptr) return;
+  const uint32_t j = perm[t];
+  const R4<R> x = pos[j], v = vel[j];
+  const uint32_t r = ref[j], f = fid[j];
+  const uint32_t d = ranked_place(j, key, start, ref, perm);
+  pos2[d] = x;
+  vel2[d] = v;
+  ref2[d] = r;
+  fid2[d] = f;
 }
 
 // boundary samples: key + histogram (no integration)
@@ -371,13 +382,14 @@ __global__ void __launch_bounds__(kBlock) k_sample_key(const int* __restrict__ n
 
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_gather_samples(
-    const int* __restrict__ n_ptr, const uint32_t* __restrict__ perm,
-    const R4<R>* __restrict__ xb, const R4<R>* __restrict__ vb, const uint32_t* __restrict__ bid,
-    const uint32_t* __restrict__ orig, R4<R>* __restrict__ xb2, R4<R>* __restrict__ vb2,
-    uint32_t* __restrict__ bid2, uint32_t* __restrict__ orig2) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= *n_ptr) return;
-  const uint32_t j = perm[d];
+    const int* __restrict__ n_ptr, const uint32_t* __restrict__ perm, const uint32_t* __restrict__ key,
+    const uint32_t* __restrict__ start, const R4<R>* __restrict__ xb, const R4<R>* __restrict__ vb,
+    const uint32_t* __restrict__ bid, const uint32_t* __restrict__ orig, R4<R>* __restrict__ xb2,
+    R4<R>* __restrict__ vb2, uint32_t* __restrict__ bid2, uint32_t* __restrict__ orig2) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= *n_ptr) return;
+  const uint32_t j = perm[t];
+  const uint32_t d = ranked_place(j, key, start, orig, perm);
   xb2[d] = xb[j];
   vb2[d] = vb[j];
   bid2[d] = bid[j];
@@ -802,7 +814,7 @@ struct OrderQueues {
   }
 };
 
-// Neighbor search and volume of one block of sorted particles.
+// Neighbor search and kernel sum of one block of sorted particles.
 //
 // Halo: the block's cells are marked, each with its 26 neighbors, in a bitmap
 // over their bounding box (rows along x), so the rank of a set bit is the
@@ -832,8 +844,7 @@ template <class R, bool ORDER>
 __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
     Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const uint32_t* __restrict__ start,
     R4<R>* __restrict__ xv, uint16_t* __restrict__ nbr, uint32_t* __restrict__ ncnt,
-    uint32_t* __restrict__ halo_idx, uint32_t* __restrict__ halo_n, const R* __restrict__ bW,
-    int has_boundary, int hcap, StepParams<R> P) {
+    uint32_t* __restrict__ halo_idx, uint32_t* __restrict__ halo_n, int hcap, StepParams<R> P) {
   extern __shared__ __align__(32) unsigned char dsm[];
   __shared__ int s_own[kSearchCells];        // per cell: own bucket's halo offset - its first particle
   __shared__ uint8_t s_head[kSearchCells];   // per cell: its first thread
@@ -1170,10 +1181,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
       if (kept == stored) break;  // all of them
       found.cnt -= stored - kept;
     }
-    R denom = P.V0 * sum;
-    if (has_boundary) denom += bW[i];
-    const R V = P.V0 / denom;
-    xv[i] = R4<R>{xi.x, xi.y, xi.z, V};
+    xv[i] = R4<R>{xi.x, xi.y, xi.z, sum};  // (k_volume puts the volume in its place)
     ncnt[i] = (uint32_t)found.cnt;
   }
   // The lists in whole groups of four. The unused slots of the last group hold
@@ -2575,26 +2583,40 @@ __global__ void __launch_bounds__(kBlock) k_split_density(
 }
 
 // ---------------------------------------------------------------------------
-// 9. reductions: average density after the update (sph/mod.rs:444-486) and
+// 9. volumes (quantities.rs:14-61) from the kernel sums and the boundary's
+//    share, with the average density after the update (sph/mod.rs:444-486);
 //    measurement sums (density error, kinetic energy) in f64
 // ---------------------------------------------------------------------------
+// The last block also sets up the next update's scalars, leaving the particles
+// that entered this one and those it disabled in n_in and n_disabled (nothing
+// after the sort reads n, n_below or max_speed).
 template <class R>
-__global__ void __launch_bounds__(kBlock) k_avg_density(Scalars* __restrict__ sc,
-                                                       const R4<R>* __restrict__ xv,
-                                                       const R4<R>* __restrict__ vel,
-                                                       double* __restrict__ partials,
-                                                       StepParams<R> P) {
+__global__ void __launch_bounds__(kBlock) k_volume(Scalars* __restrict__ sc, R4<R>* __restrict__ xv,
+                                                  const R4<R>* __restrict__ vel, const R* __restrict__ bW,
+                                                  int has_boundary, double* __restrict__ partials,
+                                                  StepParams<R> P) {
   __shared__ double sh[32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = sc->n_active;
   double d = 0.0;
   if (i < n) {
-    const double V = (double)xv[i].w, m = (double)vel[i].w, V0 = (double)P.V0;
+    const R sum = xv[i].w;
+    R denom = P.V0 * sum;
+    if (has_boundary) denom += bW[i];
+    const R Vr = P.V0 / denom;
+    xv[i].w = Vr;
+    const double V = (double)Vr, m = (double)vel[i].w, V0 = (double)P.V0;
     d = V < V0 ? m / V : m / V0;
   }
   double total;
-  if (last_block_total(block_sum(d, sh), partials, &sc->done_blocks, &total, sh))
+  if (last_block_total(block_sum(d, sh), partials, &sc->done_blocks, &total, sh)) {
     sc->avg_density = n > 0 ? total / (double)n : 0.0;
+    sc->n_in = sc->n;
+    sc->n_disabled = sc->n_below;
+    sc->n = n;
+    sc->n_below = 0;
+    sc->max_speed = 0;
+  }
 }
 
 // out[0] = sum (V < V0 ? V0/V : 1), out[1] = sum 1/2 m |v|^2
@@ -2794,13 +2816,6 @@ __global__ void __launch_bounds__(kBlock) k_sample_volumes(const int* __restrict
   xb[d] = o;
 }
 
-// The scalars of the next update, as k_step_epilogue leaves them.
-__global__ void k_next_update(Scalars* sc) {
-  sc->n = sc->n_active;
-  sc->n_below = 0;
-  sc->max_speed = 0;
-}
-
 // ---------------------------------------------------------------------------
 // graph-captured stepping
 // ---------------------------------------------------------------------------
@@ -2825,21 +2840,17 @@ __global__ void k_loop_cond(cudaGraphConditionalHandle h, const Scalars* __restr
 }
 
 // End of a graph-captured step: records what the per-step host check would
-// have acted on (then the host replays the chunk on the per-step path) and
-// prepares the scalars of the next update exactly as that check does.
+// have acted on (then the host replays the chunk on the per-step path).
 __global__ void k_step_epilogue(Scalars* sc, int K, int hcap, int solver_loop) {
   unsigned int t = 0;
   if (sc->max_nbrs > K || sc->max_halo > hcap) t |= 1u;
   sc->chunk_max_nbrs = max(sc->chunk_max_nbrs, sc->max_nbrs);
   sc->chunk_max_halo = max(sc->chunk_max_halo, sc->max_halo);
-  if (sc->n_below > 0) t |= 2u;
+  if (sc->n_disabled > 0) t |= 2u;
   if (solver_loop && !sc->converged) t |= 4u;
   sc->trouble |= t;
   if (sc->status == 2) sc->status_any = 2;
   if (solver_loop) sc->loop_sweeps += (unsigned long long)sc->iterations;
-  sc->n = sc->n_active;
-  sc->n_below = 0;
-  sc->max_speed = 0;
 }
 
 // ---------------------------------------------------------------------------

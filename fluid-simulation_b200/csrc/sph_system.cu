@@ -521,13 +521,8 @@ class System : public SystemBase {
     const int nb = blocks_for((long long)n);
     auto blocks = [](long long m) { return dim3((unsigned)((m + kBlock - 1) / kBlock)); };
     auto scan_u32 = [&](uint32_t* count, long long m, uint32_t* outp) {
-      const long long tiles = (m + kScanTile - 1) / kScanTile;
-      grow(surf_tiles_, (size_t)tiles);
-      launch("surface_scan", k_scan_tiles, dim3((unsigned)tiles), dim3(kBlock), (const uint32_t*)count, (int)m,
-             surf_tiles_.p);
-      launch("surface_scan", k_scan_tile_sums, dim3(1), dim3(1024), surf_tiles_.p, (int)tiles);
-      launch("surface_scan", k_scan_apply, dim3((unsigned)tiles), dim3(kBlock), count, (int)m,
-             (const uint32_t*)surf_tiles_.p, outp);
+      grow(surf_tiles_, (size_t)((m + kScanTile - 1) / kScanTile));
+      scan("surface_scan", count, m, outp, surf_tiles_.p);
     };
     for (const uint32_t group : group_ids_) {  // (ascending; some may have lost all their particles)
       const unsigned long long init[7] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull, ~0ull};
@@ -1217,23 +1212,28 @@ class System : public SystemBase {
   }
 
   // exclusive scan of count[0..m) into out, clearing count
-  void scan(uint32_t* count, uint32_t m, uint32_t* out) {
+  void scan(const char* name, uint32_t* count, long long m, uint32_t* out, uint32_t* tile_sums,
+            const Prologue& prologue = Prologue{}) {
     const int tiles = (int)((m + kScanTile - 1) / kScanTile);
-    launch("scan", k_scan_tiles, dim3(tiles), dim3(kBlock), (const uint32_t*)count, (int)m, tile_sums_.p);
-    launch("scan", k_scan_tile_sums, dim3(1), dim3(1024), tile_sums_.p, tiles);
-    launch("scan", k_scan_apply, dim3(tiles), dim3(kBlock), count, (int)m, (const uint32_t*)tile_sums_.p, out);
+    launch(name, k_scan_tiles, dim3(tiles), dim3(kBlock), (const uint32_t*)count, (int)m, tile_sums, prologue);
+    if (tiles <= kScanDirect) {
+      launch(name, k_scan_apply<true>, dim3(tiles), dim3(kBlock), count, (int)m, (const uint32_t*)tile_sums, out);
+    } else {
+      launch(name, k_scan_tile_sums, dim3(1), dim3(1024), tile_sums, tiles);
+      launch(name, k_scan_apply<false>, dim3(tiles), dim3(kBlock), count, (int)m, (const uint32_t*)tile_sums, out);
+    }
   }
 
   void sort_particles() {
     const int nb = blocks_for((long long)n_);
     const int* dn = &d_sc_.p->n;
-    scan(count_.p, T_ + 2, start_.p);
+    const Prologue prologue{d_sc_.p, P_.cfl, (capturing_ && cfg_.cfl_time_step) ? 1 : 0, P_.cfl_number, P_.spacing,
+                            P_.dt_max};
+    scan("scan", count_.p, T_ + 2, start_.p, tile_sums_.p, prologue);
     launch("sort", k_scatter, dim3(nb), dim3(kBlock), dn, (const uint32_t*)key_.p, (const uint32_t*)slot_.p,
            (const uint32_t*)start_.p, perm_.p);
-    launch("sort", k_bucket_order, dim3(nb), dim3(kBlock), dn, (const uint32_t*)key_.p, (const uint32_t*)start_.p,
-           (const uint32_t*)ref_.p, perm_.p);
     launch("sort", k_gather_particles<R>, dim3(nb), dim3(kBlock), dn, (const uint32_t*)perm_.p,
-           (const R4<R>*)pos_.p, (const R4<R>*)vel_.p, (const uint32_t*)ref_.p, (const uint32_t*)fid_.p,
+           (const uint32_t*)key_.p, (const uint32_t*)start_.p, (const R4<R>*)pos_.p, (const R4<R>*)vel_.p, (const uint32_t*)ref_.p, (const uint32_t*)fid_.p,
            pos2_.p, vel2_.p, ref2_.p, fid2_.p);
     swap_particle_buffers();
   }
@@ -1255,13 +1255,11 @@ class System : public SystemBase {
     const int* dn = ns_d_.p;
     launch("sample_sort", k_sample_key<R>, dim3(nb), dim3(kBlock), dn, (const R4<R>*)xb_.p, skey_.p, sslot_.p,
            scount_.p, P_.range, mask_);
-    scan(scount_.p, T_ + 2, sstart_.p);
+    scan("sample_sort", scount_.p, T_ + 2, sstart_.p, tile_sums_.p);
     launch("sample_sort", k_scatter, dim3(nb), dim3(kBlock), dn, (const uint32_t*)skey_.p, (const uint32_t*)sslot_.p,
            (const uint32_t*)sstart_.p, sperm_.p);
-    launch("sample_sort", k_bucket_order, dim3(nb), dim3(kBlock), dn, (const uint32_t*)skey_.p,
-           (const uint32_t*)sstart_.p, (const uint32_t*)sorig_.p, sperm_.p);
     launch("sample_sort", k_gather_samples<R>, dim3(nb), dim3(kBlock), dn, (const uint32_t*)sperm_.p,
-           (const R4<R>*)xb_.p, (const R4<R>*)vb_.p, (const uint32_t*)sbid_.p, (const uint32_t*)sorig_.p,
+           (const uint32_t*)skey_.p, (const uint32_t*)sstart_.p, (const R4<R>*)xb_.p, (const R4<R>*)vb_.p, (const uint32_t*)sbid_.p, (const uint32_t*)sorig_.p,
            xb2_.p, vb2_.p, sbid2_.p, sorig2_.p);
     swap_sample_buffers();
   }
@@ -1631,15 +1629,13 @@ class System : public SystemBase {
   }
 
  private:
-  // The kernels of one update, from integration to the average density.
+  // The kernels of one update, from integration to the accelerations.
   void issue_update(int mode) {
     const int nb = blocks_for((long long)n_);
     const bool sample_dyn = boundary_kind_ == 1 && any_dynamic_;
     launch("integrate_key", k_integrate_key<R>, dim3(nb), dim3(kBlock), d_sc_.p, pos_.p, vel_.p,
            (const R4<R>*)acc_.p, (const R4<R>*)xint_.p, (const R4<R>*)vint_.p, mode, key_.p, slot_.p,
            count_.p, P_);
-    launch("prologue", k_prologue<R>, dim3(1), dim3(1), d_sc_.p, P_,
-           (capturing_ && cfg_.cfl_time_step) ? 1 : 0);
     sort_particles();
     if ((early_xo_ || early_vo_) && !capturing_ && !early_done_) issue_early_readback();
     if (sample_dyn) {
@@ -1667,10 +1663,10 @@ class System : public SystemBase {
     const bool order = sizeof(R) == 4 && (cfg_.pressure_solver == SPH_IISPH || cfg_.pressure_solver == SPH_IISPH_W_OST);
     launch_s("neighbors_density", order ? k_neighbors_density<R, sizeof(R) == 4> : k_neighbors_density<R, false>,
              dim3(nb), dim3(kBlock), kSearchSmem, d_sc_.p, (const R4<R>*)pos_.p, (const uint32_t*)start_.p, xv_.p,
-             nbr_.p, ncnt_.p, halo_idx_.p, halo_n_.p, (const R*)bW_.p, boundary_kind_ ? 1 : 0, hcap_, P_);
+             nbr_.p, ncnt_.p, halo_idx_.p, halo_n_.p, hcap_, P_);
+    launch("volume", k_volume<R>, dim3(nb), dim3(kBlock), d_sc_.p, xv_.p, (const R4<R>*)vel_.p, (const R*)bW_.p,
+           boundary_kind_ ? 1 : 0, partials_.p, P_);
     calc_acceleration();
-    launch("avg_density", k_avg_density<R>, dim3(nb), dim3(kBlock), d_sc_.p, (const R4<R>*)xv_.p,
-           (const R4<R>*)vel_.p, partials_.p, P_);
   }
 
   // sph_step_host's readback of the sorted, integrated state in reference
@@ -1724,14 +1720,9 @@ class System : public SystemBase {
   // moved the removed particles behind the active range; replay the swaps on
   // the reference indices here.
   void finish_disable() {
-    const int below = h_sc_->n_below;
-    const size_t n_old = (size_t)h_sc_->n;
+    const int below = h_sc_->n_disabled;
+    const size_t n_old = (size_t)h_sc_->n_in;
     const size_t n_new = (size_t)h_sc_->n_active;
-    // set up the scalars for the next update
-    Scalars next = *h_sc_;
-    next.n = (int)n_new;
-    next.n_below = 0;
-    next.max_speed = 0;
     if (below > 0) {
       std::vector<uint32_t> ref_all = fetch(ref_.p, n_old);
       std::vector<char> is_below(n_old, 0);
@@ -1753,8 +1744,6 @@ class System : public SystemBase {
       copy_h2d(ref_.p, ref_all.data(), n_new);
       n_ = n_new;
     }
-    launch("next_update", k_next_update, dim3(1), dim3(1), d_sc_.p);
-    *h_sc_ = next;
   }
 
   // ---- graph-captured stepping --------------------------------------------------
