@@ -79,6 +79,22 @@ __device__ __forceinline__ bool last_block_total(double block_value, double* par
   return threadIdx.x == 0;
 }
 
+// Programmatic dependent launch: a kernel launched with programmatic stream
+// serialization may start while the kernel before it finishes its last wave.
+// grid_dep_wait() returns once that kernel has completed and its writes are
+// visible; everything before it may read only data the earlier kernel does
+// not write. grid_dep_release() lets the next kernel start launching (once
+// every block of this grid has started). Both are no-ops in a plain launch.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+// The start of a kernel that reads what the kernel before it wrote: its blocks
+// are on their SMs by then, and the next kernel's may follow (small scenes, where
+// a step is a dozen kernels of 3 to 30 us, save the launch latency between them).
+__device__ __forceinline__ void grid_dep_begin() {
+  grid_dep_wait();
+  grid_dep_release();
+}
+
 // ---------------------------------------------------------------------------
 // Rigid-body helpers (f64), nalgebra semantics (rigid_body_motion.rs)
 // ---------------------------------------------------------------------------
@@ -244,6 +260,7 @@ __device__ __forceinline__ void scan_load8(const uint32_t* __restrict__ in, int 
 constexpr int kScanDirect = 2048;
 __global__ void __launch_bounds__(kBlock) k_scan_tiles(const uint32_t* __restrict__ in, int m,
                                                       uint32_t* __restrict__ tile_sums, Prologue prologue) {
+  grid_dep_begin();
   __shared__ uint32_t sh[32];
   if (prologue.sc && blockIdx.x == 0 && threadIdx.x == 0) run_prologue(prologue);
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
@@ -258,6 +275,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_tiles(const uint32_t* __restric
 }
 
 __global__ void __launch_bounds__(1024) k_scan_tile_sums(uint32_t* __restrict__ tile_sums, int ntiles) {
+  grid_dep_begin();
   __shared__ uint32_t sh[32];
   // each thread owns a contiguous run of tiles
   const int per = (ntiles + blockDim.x - 1) / blockDim.x;
@@ -277,6 +295,7 @@ template <bool DIRECT>
 __global__ void __launch_bounds__(kBlock) k_scan_apply(uint32_t* __restrict__ in, int m,
                                                       const uint32_t* __restrict__ tile_sums,
                                                       uint32_t* __restrict__ out) {
+  grid_dep_begin();
   __shared__ uint32_t sh[32];
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
@@ -324,6 +343,7 @@ __global__ void __launch_bounds__(kBlock) k_scatter(const int* __restrict__ n_pt
                                                    const uint32_t* __restrict__ slot,
                                                    const uint32_t* __restrict__ start,
                                                    uint32_t* __restrict__ perm) {
+  grid_dep_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= *n_ptr) return;
   perm[start[key[i]] + slot[i]] = (uint32_t)i;
@@ -351,6 +371,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_particles(
     const uint32_t* __restrict__ start, const R4<R>* __restrict__ pos, const R4<R>* __restrict__ vel,
     const uint32_t* __restrict__ ref, const uint32_t* __restrict__ fid, R4<R>* __restrict__ pos2,
     R4<R>* __restrict__ vel2, uint32_t* __restrict__ ref2, uint32_t* __restrict__ fid2) {
+  grid_dep_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= *n_ptr) return;
   const uint32_t j = perm[t];
@@ -500,15 +521,6 @@ __device__ __forceinline__ void stage_done() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
 }
-
-// Programmatic dependent launch: a kernel launched with programmatic stream
-// serialization may start while the kernel before it finishes its last wave.
-// grid_dep_wait() returns once that kernel has completed and its writes are
-// visible; everything before it may read only data the earlier kernel does
-// not write. grid_dep_release() lets the next kernel start launching (once
-// every block of this grid has started). Both are no-ops in a plain launch.
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
 // Copies the block's halo records to shared memory: copy(l, g) moves the
 // record of particle g to position l. Four halo indices per thread are read
@@ -845,6 +857,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
     Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const uint32_t* __restrict__ start,
     R4<R>* __restrict__ xv, uint16_t* __restrict__ nbr, uint32_t* __restrict__ ncnt,
     uint32_t* __restrict__ halo_idx, uint32_t* __restrict__ halo_n, int hcap, StepParams<R> P) {
+  grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   __shared__ int s_own[kSearchCells];        // per cell: own bucket's halo offset - its first particle
   __shared__ uint8_t s_head[kSearchCells];   // per cell: its first thread
@@ -1331,6 +1344,7 @@ __global__ void __launch_bounds__(kBlock) k_vm_near(
     const Body* __restrict__ bodies, uint32_t* __restrict__ near_list, R4<R>* __restrict__ vmx,
     R4<R>* __restrict__ vmv, R* __restrict__ bW, R4<R>* __restrict__ bG, R4<R>* __restrict__ bGu,
     R4<R>* __restrict__ bA, StepParams<R> P) {
+  grid_dep_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= sc->n_active) return;
   const R4<R> xr = pos[i];
@@ -1433,6 +1447,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_vm_sample(
     const R4<R>* __restrict__ vel, const VMDesc* __restrict__ vms, int nvm, const Body* __restrict__ bodies,
     R4<R>* __restrict__ vmx, R4<R>* __restrict__ vmv, R* __restrict__ bW, R4<R>* __restrict__ bG,
     R4<R>* __restrict__ bGu, R4<R>* __restrict__ bA, uint32_t* __restrict__ touch, StepParams<R> P) {
+  grid_dep_begin();
   const int lane = threadIdx.x & 31, e = lane & 7;
   const unsigned group = 0xffu << (lane & ~7);
   const int t = (blockIdx.x * kBlock + threadIdx.x) >> 3;
@@ -1733,6 +1748,7 @@ __global__ void __launch_bounds__(kBlock) k_sample_boundary(
     Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const R4<R>* __restrict__ vel, SampleGrid<R> G,
     const Body* __restrict__ bodies, int any_dynamic, R* __restrict__ bW, R4<R>* __restrict__ bG,
     R4<R>* __restrict__ bGu, R4<R>* __restrict__ bA, uint32_t* __restrict__ touch, StepParams<R> P) {
+  grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   __shared__ uint32_t s_key[kSampleBlock], s_heads[kSampleBlock / 32];
   __shared__ uint8_t s_head[kSampleBlock + 1], s_near[kSampleBlock];  // per cell: first particle; it has candidates
@@ -2079,6 +2095,7 @@ __global__ void __launch_bounds__(kBlock) k_accel(
     const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv, const R4<R>* __restrict__ vel,
     NbrArgs N, BoundaryArgs<R> B, R4<R>* __restrict__ acc, R4<R>* __restrict__ vstar,
     R* __restrict__ press, int write_vstar, StepParams<R> P) {
+  grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   const HaloView H = halo_view(N);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2163,6 +2180,7 @@ template <class R>
 __global__ void __launch_bounds__(kBlock) k_pressure_accel(
     const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv, const R4<R>* __restrict__ vel,
     const R* __restrict__ press, NbrArgs N, BoundaryArgs<R> B, R4<R>* __restrict__ out, StepParams<R> P) {
+  grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   const HaloView H = halo_view(N);
   // this particle's own data and first list batch travel while the halo stages
@@ -2221,6 +2239,7 @@ __global__ void __launch_bounds__(kBlock) k_iisph_source_diag(
     const R4<R>* __restrict__ vstar, NbrArgs N, BoundaryArgs<R> B, R* __restrict__ s_out,
     R* __restrict__ aii_out, R* __restrict__ press, R4<R>* __restrict__ TA, R4<R>* __restrict__ TB,
     R2<R>* __restrict__ SA, R4<R>* __restrict__ xq_out, StepParams<R> P) {
+  grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   const HaloView H = halo_view(N);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2538,6 +2557,7 @@ __global__ void __launch_bounds__(kBlock) k_split_density(
     const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv, const R4<R>* __restrict__ vel,
     const R4<R>* __restrict__ vstar, NbrArgs N, BoundaryArgs<R> B, R* __restrict__ press,
     R* __restrict__ rho_pred, StepParams<R> P) {
+  grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   const HaloView H = halo_view(N);
   // records {x, V} and {v*, m} (the acceleration pass stores m in v*.w)
@@ -2595,6 +2615,7 @@ __global__ void __launch_bounds__(kBlock) k_volume(Scalars* __restrict__ sc, R4<
                                                   const R4<R>* __restrict__ vel, const R* __restrict__ bW,
                                                   int has_boundary, double* __restrict__ partials,
                                                   StepParams<R> P) {
+  grid_dep_begin();
   __shared__ double sh[32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = sc->n_active;

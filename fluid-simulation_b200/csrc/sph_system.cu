@@ -197,10 +197,14 @@ class System : public SystemBase {
   ~System() override {
     // everything the streams still run ends before the buffers go back to the pool
     if (stream_) cudaStreamSynchronize(stream_);
+    if (side_stream_) cudaStreamSynchronize(side_stream_);
     if (io_stream_) cudaStreamSynchronize(io_stream_);
     destroy_graphs();
     if (chunk_event_) cudaEventDestroy(chunk_event_);
     if (body_stream_) cudaStreamDestroy(body_stream_);
+    if (side_stream_) cudaStreamDestroy(side_stream_);
+    for (cudaEvent_t e : side_event_)
+      if (e) cudaEventDestroy(e);
     if (io_stream_) cudaStreamDestroy(io_stream_);
     if (io_ready_) cudaEventDestroy(io_ready_);
     Pool::get().free(h_chunk_sc_);
@@ -816,6 +820,10 @@ class System : public SystemBase {
   // sph_step_host's overlapped readback of the last step
   cudaStream_t io_stream_ = nullptr;
   cudaEvent_t io_ready_ = nullptr;
+  // the boundary's work beside the neighbor search
+  cudaStream_t side_stream_ = nullptr;
+  cudaEvent_t side_event_[2] = {nullptr, nullptr};
+  bool on_side_ = false, side_open_ = false;
   double* early_xo_ = nullptr;
   double* early_vo_ = nullptr;
   bool early_done_ = false;
@@ -1215,12 +1223,12 @@ class System : public SystemBase {
   void scan(const char* name, uint32_t* count, long long m, uint32_t* out, uint32_t* tile_sums,
             const Prologue& prologue = Prologue{}) {
     const int tiles = (int)((m + kScanTile - 1) / kScanTile);
-    launch(name, k_scan_tiles, dim3(tiles), dim3(kBlock), (const uint32_t*)count, (int)m, tile_sums, prologue);
+    launch_dep(name, k_scan_tiles, dim3(tiles), dim3(kBlock), 0, (const uint32_t*)count, (int)m, tile_sums, prologue);
     if (tiles <= kScanDirect) {
-      launch(name, k_scan_apply<true>, dim3(tiles), dim3(kBlock), count, (int)m, (const uint32_t*)tile_sums, out);
+      launch_dep(name, k_scan_apply<true>, dim3(tiles), dim3(kBlock), 0, count, (int)m, (const uint32_t*)tile_sums, out);
     } else {
-      launch(name, k_scan_tile_sums, dim3(1), dim3(1024), tile_sums, tiles);
-      launch(name, k_scan_apply<false>, dim3(tiles), dim3(kBlock), count, (int)m, (const uint32_t*)tile_sums, out);
+      launch_dep(name, k_scan_tile_sums, dim3(1), dim3(1024), 0, tile_sums, tiles);
+      launch_dep(name, k_scan_apply<false>, dim3(tiles), dim3(kBlock), 0, count, (int)m, (const uint32_t*)tile_sums, out);
     }
   }
 
@@ -1230,9 +1238,9 @@ class System : public SystemBase {
     const Prologue prologue{d_sc_.p, P_.cfl, (capturing_ && cfg_.cfl_time_step) ? 1 : 0, P_.cfl_number, P_.spacing,
                             P_.dt_max};
     scan("scan", count_.p, T_ + 2, start_.p, tile_sums_.p, prologue);
-    launch("sort", k_scatter, dim3(nb), dim3(kBlock), dn, (const uint32_t*)key_.p, (const uint32_t*)slot_.p,
+    launch_dep("sort", k_scatter, dim3(nb), dim3(kBlock), 0, dn, (const uint32_t*)key_.p, (const uint32_t*)slot_.p,
            (const uint32_t*)start_.p, perm_.p);
-    launch("sort", k_gather_particles<R>, dim3(nb), dim3(kBlock), dn, (const uint32_t*)perm_.p,
+    launch_dep("sort", k_gather_particles<R>, dim3(nb), dim3(kBlock), 0, dn, (const uint32_t*)perm_.p,
            (const uint32_t*)key_.p, (const uint32_t*)start_.p, (const R4<R>*)pos_.p, (const R4<R>*)vel_.p, (const uint32_t*)ref_.p, (const uint32_t*)fid_.p,
            pos2_.p, vel2_.p, ref2_.p, fid2_.p);
     swap_particle_buffers();
@@ -1565,37 +1573,37 @@ class System : public SystemBase {
     constexpr int NB = decltype(NBc)::value;
     switch (cfg_.pressure_solver) {
       case SPH_SESPH:
-        launch_s("accel_sesph", k_accel<R, 1>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(), acc_.p,
+        launch_dep("accel_sesph", k_accel<R, 1>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(), acc_.p,
                vstar_.p, press_.p, 0, P_);
         body_react();
         break;
       case SPH_SESPH_W_SPLITTING:
-        launch_s("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
+        launch_dep("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
                acc_.p, vstar_.p, press_.p, 1, P_);
-        launch_s("split_density", k_split_density<R, NB>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
+        launch_dep("split_density", k_split_density<R, NB>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
                (const R4<R>*)vstar_.p, nbr, bargs(), press_.p, rho_pred_.p, P_);
-        launch_s("pressure_accel", k_pressure_accel<R>, dim3(nb), dim3(kBlock), sm_xp, csc, xv, vel,
+        launch_dep("pressure_accel", k_pressure_accel<R>, dim3(nb), dim3(kBlock), sm_xp, csc, xv, vel,
                (const R*)press_.p, nbr, bargs(), acc_.p, P_);
         body_react();
         break;
       case SPH_IISPH:
-        launch_s("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
+        launch_dep("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
                acc_.p, vstar_.p, press_.p, 2, P_);
-        launch_s("iisph_source_diag", k_iisph_source_diag<R, 1>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
+        launch_dep("iisph_source_diag", k_iisph_source_diag<R, 1>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
                (const R4<R>*)vstar_.p, nbr, bargs(), s_.p, aii_.p, press_.p, TA_.p, TB_.p, SA_.p, xq_.p, P_);
         solve_loop(-1);
         final_pressure_accel<1>();
         body_react();
         break;
       case SPH_IISPH_W_OST:
-        launch_s("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
+        launch_dep("accel_nonpressure", k_accel<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel, nbr, bargs(),
                acc_.p, vstar_.p, press_.p, 2, P_);
-        launch_s("iisph_source_diag", k_iisph_source_diag<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
+        launch_dep("iisph_source_diag", k_iisph_source_diag<R, 0>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
                (const R4<R>*)vstar_.p, nbr, bargs(), s_.p, aii_.p, press_.p, TA_.p, TB_.p, SA_.p, xq_.p, P_);
         solve_loop(3);
         final_pressure_accel<2>();  // IISPHwOST takes no dynamic boundaries
         launch("ost_predict", k_ost_predict<R>, dim3(nb), dim3(kBlock), d_sc_.p, (const R4<R>*)acc_.p, vstar_.p);
-        launch_s("iisph_source_diag", k_iisph_source_diag<R, 1>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
+        launch_dep("iisph_source_diag", k_iisph_source_diag<R, 1>, dim3(nb), dim3(kBlock), sm_xv, csc, xv, vel,
                (const R4<R>*)vstar_.p, nbr, bargs(), s_.p, aii_.p, press_.p, TA_.p, TB_.p, SA_.p, xq_.p, P_);
         solve_loop(-1);
         final_pressure_accel<2>();
@@ -1610,7 +1618,12 @@ class System : public SystemBase {
   // System::update (sph/mod.rs:674-731); mode 0/1 integrate first (EulerCromer
   // / TakePredicted, euler_cromer.rs:12-25 / take_predicted.rs:14-27), 2 not.
   void update(int mode) {
-    issue_update(mode);
+    try {
+      issue_update(mode);
+    } catch (...) {
+      abandon_side();
+      throw;
+    }
     cuda_check(cudaMemcpyAsync(h_sc_, d_sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, stream_), "memcpy");
     sync();
     collect_profile();
@@ -1638,6 +1651,10 @@ class System : public SystemBase {
            count_.p, P_);
     sort_particles();
     if ((early_xo_ || early_vo_) && !capturing_ && !early_done_) issue_early_readback();
+    // The boundary's share needs the sorted particles only, and nothing needs it
+    // before the volumes: it runs beside the neighbor search (both leave SMs idle
+    // in a small scene and at their ends).
+    if (boundary_kind_) fork_side();
     if (sample_dyn) {
       const int sb = blocks_for((long long)ns_);
       launch("body_samples", k_body_samples<R>, dim3(sb), dim3(kBlock), (const int*)ns_d_.p,
@@ -1647,26 +1664,63 @@ class System : public SystemBase {
     }
     if (boundary_kind_ == 1) {
       const bool split = cfg_.pressure_solver == SPH_SESPH_W_SPLITTING;
-      launch_s("boundary_samples", split ? k_sample_boundary<R, true> : k_sample_boundary<R, false>,
+      launch_dep("boundary_samples", split ? k_sample_boundary<R, true> : k_sample_boundary<R, false>,
                dim3((unsigned)((n_ + kSampleBlock - 1) / kSampleBlock) + (n_ == 0)), dim3(kBlock),
                sizeof(SampleStage<R>) * (kBlock / 32), d_sc_.p, (const R4<R>*)pos_.p, (const R4<R>*)vel_.p,
                sample_grid(), (const Body*)bodies_d_.p, any_dynamic_ ? 1 : 0, bW_.p, bG_.p, bGu_.p, bA_.p, touch_.p, P_);
     } else if (boundary_kind_ == 2) {
-      launch("vm_near", k_vm_near<R>, dim3(nb), dim3(kBlock), d_sc_.p, (const R4<R>*)pos_.p,
+      launch_dep("vm_near", k_vm_near<R>, dim3(nb), dim3(kBlock), 0, d_sc_.p, (const R4<R>*)pos_.p,
              (const VMDesc*)vms_.p, (int)fields_.size(), (const Body*)bodies_d_.p, vm_near_.p, vmx_.p, vmv_.p,
              bW_.p, bG_.p, bGu_.p, bA_.p, P_);
-      launch("boundary_samples", k_vm_sample<R>, dim3(8 * nb), dim3(kBlock), d_sc_.p, (const uint32_t*)vm_near_.p,
+      launch_dep("boundary_samples", k_vm_sample<R>, dim3(8 * nb), dim3(kBlock), 0, d_sc_.p, (const uint32_t*)vm_near_.p,
              (const R4<R>*)pos_.p, (const R4<R>*)vel_.p, (const VMDesc*)vms_.p, (int)fields_.size(),
              (const Body*)bodies_d_.p, vmx_.p, vmv_.p, bW_.p, bG_.p, bGu_.p, bA_.p, touch_.p, P_);
     }
+    if (boundary_kind_) leave_side();
     // IISPH in f32 re-reads the lists in every sweep pass: they come out ordered for shared-memory banks
     const bool order = sizeof(R) == 4 && (cfg_.pressure_solver == SPH_IISPH || cfg_.pressure_solver == SPH_IISPH_W_OST);
-    launch_s("neighbors_density", order ? k_neighbors_density<R, sizeof(R) == 4> : k_neighbors_density<R, false>,
+    launch_dep("neighbors_density", order ? k_neighbors_density<R, sizeof(R) == 4> : k_neighbors_density<R, false>,
              dim3(nb), dim3(kBlock), kSearchSmem, d_sc_.p, (const R4<R>*)pos_.p, (const uint32_t*)start_.p, xv_.p,
              nbr_.p, ncnt_.p, halo_idx_.p, halo_n_.p, hcap_, P_);
-    launch("volume", k_volume<R>, dim3(nb), dim3(kBlock), d_sc_.p, xv_.p, (const R4<R>*)vel_.p, (const R*)bW_.p,
+    join_side();
+    launch_impl(dep_launch() && !boundary_kind_, "volume", k_volume<R>, dim3(nb), dim3(kBlock), 0, d_sc_.p, xv_.p, (const R4<R>*)vel_.p, (const R*)bW_.p,
            boundary_kind_ ? 1 : 0, partials_.p, P_);
     calc_acceleration();
+  }
+
+  // Launches between fork_side() and leave_side() go to a second stream behind
+  // what the first one has been given so far; join_side() makes the first wait
+  // for them. Timed (profiling) runs keep to one stream, so that the events
+  // around each kernel bracket it alone.
+  void fork_side() {
+    if (profiling_ && !capturing_) return;
+    if (!side_stream_) {
+      cuda_check(cudaStreamCreateWithFlags(&side_stream_, cudaStreamNonBlocking), "cudaStreamCreate");
+      for (cudaEvent_t& e : side_event_) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    }
+    cuda_check(cudaEventRecord(side_event_[0], stream_), "event");
+    cuda_check(cudaStreamWaitEvent(side_stream_, side_event_[0], 0), "event");
+    std::swap(stream_, side_stream_);
+    on_side_ = true;
+  }
+  void leave_side() {
+    if (!on_side_) return;
+    on_side_ = false;
+    std::swap(stream_, side_stream_);
+    cuda_check(cudaEventRecord(side_event_[1], side_stream_), "event");
+    side_open_ = true;
+  }
+  void join_side() {
+    if (!side_open_) return;
+    side_open_ = false;
+    cuda_check(cudaStreamWaitEvent(stream_, side_event_[1], 0), "event");
+  }
+  // After an error between the two: the streams trade places again and the side
+  // stream's work ends.
+  void abandon_side() {
+    if (on_side_) std::swap(stream_, side_stream_);
+    on_side_ = side_open_ = false;
+    if (side_stream_ && !capturing_) cudaStreamSynchronize(side_stream_);
   }
 
   // sph_step_host's readback of the sorted, integrated state in reference
@@ -1911,6 +1965,7 @@ class System : public SystemBase {
       const int loop = cfg_.pressure_solver == SPH_IISPH || cfg_.pressure_solver == SPH_IISPH_W_OST;
       launch("step_epilogue", k_step_epilogue, dim3(1), dim3(1), d_sc_.p, K_, hcap_, loop);
     } catch (...) {
+      abandon_side();
       capturing_ = false;
       in_loop_body_ = false;
       cudaGraph_t junk = nullptr;
