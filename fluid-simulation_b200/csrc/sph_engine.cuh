@@ -56,6 +56,8 @@ struct Scalars {
   int max_halo;                    // largest block halo (particles) seen
   unsigned int vm_near;            // particles within the support radius of a volume map
   unsigned int n_touch;            // particles with a neighbor on a dynamic body
+  unsigned int barrier_count, barrier_gen;  // grid barrier of the cooperative solve
+  int barrier_timeout;             // 1: a block of it gave up waiting
   // graph-captured stepping (the host reads these once per chunk)
   double time_acc;                 // simulated time under CFL steps
   unsigned int trouble;            // bits: 1 neighbor overflow, 2 disabled particles, 4 unconverged

@@ -2074,8 +2074,8 @@ struct SweepList {
 // own halo position, so a pass whose pair term is zero at r = 0 needs no
 // per-neighbor count test. The four records of a group are gathered before
 // they are used.
-template <class R, class Load, class Use>
-__device__ __forceinline__ void sweep_groups(SweepList<R>& L, Load&& load, Use&& use) {
+template <class List, class Load, class Use>
+__device__ __forceinline__ void sweep_groups(List& L, Load&& load, Use&& use) {
   for (int g = 0; g < L.ng; ++g) {
     const uint2 w = L.next(g);
     const auto d0 = load(w.x & 0xffffu);
@@ -2406,6 +2406,25 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_accel(
   }
 }
 
+// End of a sweep (one thread): error, sweep count, stop test (iisph.rs:378-393).
+__device__ __forceinline__ void end_sweep(Scalars* sc, double total, int n, int after, double tde, int cap) {
+  const double err = n > 0 ? total / (double)n * 100.0 : 0.0;
+  const int it = sc->iterations + 1;
+  sc->iterations = it;
+  sc->err = err;
+  bool stop;
+  if (after >= 0) {
+    stop = it > after;
+  } else {
+    stop = it > 2 && err < tde;
+    if (!stop && cap > 0 && it >= cap) {
+      stop = true;
+      sc->status = 2;  // not converged within the cap
+    }
+  }
+  if (stop) sc->converged = 1;
+}
+
 // pass B: A_i = dt^2 [a_i . (S_i + bG_i) - sum_j (V_j a_j) . gradW_ij];
 // p_i <- max(p_i + omega (s_i - A_i) / a_ii, 0) where a_ii < -eps; the
 // residual e_i = |A_i - s_i| where s_i < 0, summed in f64 over all N (last
@@ -2490,23 +2509,228 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_jacobi
   }
   const double bs = block_sum(e, sh);
   double total;
-  if (last_block_total(bs, partials, &sc->done_blocks, &total, sh)) {
-    const double err = n > 0 ? total / (double)n * 100.0 : 0.0;
-    const int it = sc->iterations + 1;
-    sc->iterations = it;
-    sc->err = err;
-    bool stop;
-    if (after >= 0) {
-      stop = it > after;
-    } else {
-      stop = it > 2 && err < P.tde;
-      if (!stop && P.iteration_cap > 0 && it >= P.iteration_cap) {
-        stop = true;
-        sc->status = 2;  // not converged within the cap
+  if (last_block_total(bs, partials, &sc->done_blocks, &total, sh)) end_sweep(sc, total, n, after, P.tde, P.iteration_cap);
+}
+
+// ---------------------------------------------------------------------------
+// A whole solve in one cooperative launch, for scenes whose blocks are on the
+// GPU all at once: the sweeps' passes A and B as above (same operations, same
+// order), with a barrier over the grid between them. A particle's own data
+// stay in registers; records that other blocks rewrite between two barriers are
+// read past L1.
+//
+// What bounds it: latency (records, lists, barrier, reduction). A sweep as two
+// launches takes the launches as well, and either a host that reads the error
+// between batches of sweeps or a while-node. KEEP: the lists are copied to shared
+// memory once (a warp alone on its scheduler waits for every group read from L2).
+// The 3 sweeps of 5 thousand particles took 42 us with u's second records staged
+// one load at a time; 431 -> 151 us per step stepped by calls and 138 -> 123 us in a
+// graph against a launch per pass, 5 thousand particles, four sweeps.
+// ---------------------------------------------------------------------------
+template <class T>
+__device__ __forceinline__ T load_l2(const T* p) {
+  T r;
+  if constexpr (sizeof(T) == 8) {
+    reinterpret_cast<int2&>(r) = __ldcg(reinterpret_cast<const int2*>(p));
+  } else {
+#pragma unroll
+    for (int o = 0; o < (int)(sizeof(T) / 16); ++o)
+      reinterpret_cast<int4*>(&r)[o] = __ldcg(reinterpret_cast<const int4*>(p) + o);
+  }
+  return r;
+}
+
+// Four records of a thread, requested before the first is stored.
+template <class T>
+__device__ __forceinline__ void stage_batch(const HaloView& H, const uint32_t (&g)[4], int l0, const T* src, T* dst) {
+  T r[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) r[u] = load_l2(&src[g[u]]);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int l = l0 + u * kBlock + (int)threadIdx.x;
+    if (l < H.size) dst[l] = r[u];
+  }
+}
+
+// Barrier over a cooperative grid. The last block to arrive runs last() (all its
+// threads) before it lets the others go. The wait is bounded: a block that gives
+// up sets barrier_timeout and returns false, and so do the others in turn.
+constexpr int kBarrierPolls = 1 << 22;
+template <class F>
+__device__ __forceinline__ bool grid_barrier(Scalars* sc, F&& last) {
+  __shared__ unsigned s_gen;
+  __shared__ int s_last, s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_gen = *(volatile unsigned*)&sc->barrier_gen;  // (before the arrival: it cannot move on until then)
+    __threadfence();
+    s_last = atomicAdd(&sc->barrier_count, 1u) == gridDim.x - 1;
+    s_ok = 1;
+  }
+  __syncthreads();
+  if (s_last) {
+    __threadfence();
+    last();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      sc->barrier_count = 0;
+      __threadfence();
+      atomicAdd(&sc->barrier_gen, 1u);
+    }
+  } else if (threadIdx.x == 0) {
+    int polls = 0;
+    while (*(volatile unsigned*)&sc->barrier_gen == s_gen) {
+      if (++polls == kBarrierPolls) {
+        sc->barrier_timeout = 1;
+        s_ok = 0;
+        break;
       }
     }
-    if (stop) sc->converged = 1;
+    __threadfence();
   }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// The groups of a particle's neighbor list from shared memory, after SweepList.
+struct KeptList {
+  const uint2* p;
+  int ng;
+  __device__ __forceinline__ uint2 next(int g) const { return p[g * 32]; }
+};
+
+template <class R, bool KEEP>
+__global__ void __launch_bounds__(kBlock, (sizeof(R) == 4 ? 4 : 2) / (KEEP ? 2 : 1)) k_solve(
+    Scalars* sc, const R4<R>* __restrict__ TA, const R4<R>* __restrict__ TB, const R2<R>* __restrict__ SA,
+    R4<R>* xq, R4<R>* xu, R2<R>* uu, R* press, NbrArgs N, double* partials, int after, int limit,
+    StepParams<R> P) {
+  __shared__ double sh[32];
+  extern __shared__ __align__(32) unsigned char dsm[];
+  if (*(volatile int*)&sc->converged) return;  // (set between barriers only: every block sees the same)
+  R4<R>* s_a = reinterpret_cast<R4<R>*>(dsm);
+  R2<R>* s_b = reinterpret_cast<R2<R>*>(s_a + N.hs);
+  const HaloView H = halo_view(N);
+  const int i = blockIdx.x * kBlock + threadIdx.x;
+  const int n = sc->n_active;
+  const bool act = i < n;
+  const int cnt = act ? min((int)N.ncnt[i], N.K) : 0;
+  const HaloFirst hf = halo_first(H);
+  const R dt = (R)sc->dt;
+  R4<R> xi{}, Ti{}, Tb{};
+  R2<R> sa{};
+  R p = 0;
+  if (act) {
+    xi = xq[i];
+    Ti = TA[i];
+    Tb = TB[i];
+    sa = SA[i];
+    p = press[i];
+  }
+  uint2* s_nbr = reinterpret_cast<uint2*>(s_b + N.hs) + (threadIdx.x >> 5) * 8 * N.K + (threadIdx.x & 31);
+  if (KEEP) {
+    SweepList<R> L;
+    L.begin(N, act ? i : 0, cnt);
+    for (int g = 0; g < L.ng; ++g) s_nbr[g * 32] = L.next(g);
+  }
+  auto list = [&] {
+    if constexpr (KEEP) {
+      return KeptList{s_nbr, (cnt + 3) >> 2};
+    } else {
+      SweepList<R> L;
+      L.begin(N, act ? i : 0, cnt);
+      return L;
+    }
+  };
+  const R ih = P.k.inv_h;
+  for (int sweep = 0; sweep < limit; ++sweep) {
+    // pass A
+    R4<R> u4{};
+    R2<R> u2{};
+    {
+      auto L = list();
+      stage_halo_from(H, hf, [&](int l, uint32_t g) { async_copy(&s_a[l], &xq[g]); });
+      stage_done();
+      if (act) {
+        R px = 0, py = 0, pz = 0;
+        auto pair = [&](const R4<R>& r) {
+          const R rx = xi.x - r.x, ry = xi.y - r.y, rz = xi.z - r.z;
+          const R t = r.w * grad_third(rx, ry, rz, ih);
+          px += t * rx; py += t * ry; pz += t * rz;
+        };
+        if (H.staged)
+          sweep_groups(L, [&](uint32_t l) { return s_a[l]; }, pair);
+        else
+          sweep_groups(L, [&](uint32_t l) { return load_l2(&xq[H.idx[l]]); }, pair);
+        const R cg = R(-3) * P.k.cg;
+        const R fx = p * Ti.x + cg * px, fy = p * Ti.y + cg * py, fz = p * Ti.z + cg * pz;
+        const R c = Ti.w;
+        u4 = R4<R>{xi.x, xi.y, xi.z, c * fx};
+        u2 = R2<R>{c * fy, c * fz};
+        xu[i] = u4;
+        uu[i] = u2;
+      }
+    }
+    if (!grid_barrier(sc, [] {})) return;
+    // pass B
+    double e = 0.0;
+    {
+      auto L = list();
+      stage_halo_from(H, hf, [&](int l, uint32_t g) { async_copy(&s_a[l], &xu[g]); });
+      // (f32: eight-byte records, for which cp.async has no form past L1)
+      if constexpr (sizeof(R2<R>) == 16) {
+        stage_halo_from(H, hf, [&](int l, uint32_t g) { async_copy(&s_b[l], &uu[g]); });
+      } else if (H.staged) {
+        stage_batch(H, hf.g, 0, uu, s_b);
+        for (int l0 = 4 * kBlock; l0 < H.size; l0 += 4 * kBlock) {
+          uint32_t g[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int l = l0 + u * kBlock + (int)threadIdx.x;
+            g[u] = l < H.size ? __ldg(H.idx + l) : 0u;
+          }
+          stage_batch(H, g, l0, uu, s_b);
+        }
+      }
+      stage_done();
+      if (act) {
+        R sum = 0;
+        struct Rec {
+          R4<R> a;
+          R2<R> b;
+        };
+        auto pair = [&](const Rec& d) {
+          const R rx = xi.x - d.a.x, ry = xi.y - d.a.y, rz = xi.z - d.a.z;
+          sum += grad_third(rx, ry, rz, ih) * (d.a.w * rx + d.b.x * ry + d.b.y * rz);
+        };
+        if (H.staged)
+          sweep_groups(L, [&](uint32_t l) { return Rec{s_a[l], s_b[l]}; }, pair);
+        else
+          sweep_groups(L, [&](uint32_t l) { const uint32_t g = H.idx[l]; return Rec{load_l2(&xu[g]), load_l2(&uu[g])}; }, pair);
+        const R iV = R(1) / Tb.w;
+        const R ax = u4.w * iV, ay = u2.x * iV, az = u2.y * iV;
+        const R tot = ax * Tb.x + ay * Tb.y + az * Tb.z + R(3) * P.k.cg * sum;
+        const R A = dt * dt * tot;
+        const R s = sa.x, aii = sa.y;
+        R pn = p;
+        if (aii < -P.min_diag) pn = fmax(p + P.omega * (s - A) / aii, R(0));
+        p = pn;
+        xq[i] = R4<R>{xi.x, xi.y, xi.z, Tb.w * pn};
+        if (s < R(0)) e = fabs((double)A - (double)s);
+      }
+    }
+    const double bs = block_sum(e, sh);
+    if (threadIdx.x == 0) partials[blockIdx.x] = bs;
+    const bool ok = grid_barrier(sc, [&] {  // (the sum of last_block_total)
+      double t = 0;
+      for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) t += ((volatile double*)partials)[b];
+      t = block_sum(t, sh);
+      if (threadIdx.x == 0) end_sweep(sc, t, n, after, P.tde, P.iteration_cap);
+    });
+    if (!ok) return;
+    if (*(volatile int*)&sc->converged) break;
+  }
+  if (act) press[i] = p;
 }
 
 // IISPHwOST between the solves: v* += dt a_p1 (iisph_optimized_source_term.rs:97-110)

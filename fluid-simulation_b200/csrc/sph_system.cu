@@ -1490,22 +1490,69 @@ class System : public SystemBase {
              (const R2<R>*)SA_.p, (const R4<R>*)xu_.p, (const R2<R>*)uu_.p, N, press_.p, xq_.p, partials_.p,
              after, P_);
   }
-  // The distance, in blocks, of a sweep pass's L2 prefetch (0 when it is
-  // off): half the blocks resident on the whole GPU at once, so a block's
-  // lines arrive about half a block lifetime ahead (on the 1M scene a whole
-  // wave ahead measured 2 % slower, two waves 10 %).
-  int resident_blocks(const void* fn, size_t smem) {
-    if (!prefetch_) return 0;
+  // How a solve is launched. 2: one cooperative launch that keeps the neighbor
+  // lists in shared memory, where the GPU holds all blocks with them (f32: two
+  // blocks an SM, 75 thousand particles; f64: one, 37 thousand); 1: one
+  // cooperative launch, lists read every sweep (f32: four blocks an SM, f64: two);
+  // 0: a launch per pass, for more blocks, for the scene server (whose scenes
+  // share the SMs; a cooperative launch waits until all its blocks fit) and for
+  // timed (profiling) runs. Stepping by calls, a launch per pass has the host
+  // read the error now and then; in a captured graph a while-node does that, and
+  // reading the lists again costs what the launches saved, so there it is 2 or 0.
+  // us per step of the serving scenes, four sweeps, launch per pass -> one launch:
+  //   by calls  f32 5k 431 -> 151, 64k 511 -> 205, 148k 551 -> 281; f64 5k 567 -> 313, 72k 650 -> 414
+  //   graph     f32 5k 138 -> 123, 36k 200 -> 161, 64k 204 -> 177; f64 2k 205 -> 182, 36k 348 -> 346
+  //             without the lists kept: f32 110k 228 -> 219, 125k 238 -> 244, 148k 267 -> 270; f64 64k 357 -> 367
+  size_t solve_smem(bool keep) const {
+    return (size_t)sweep_hs_ * (sizeof(R4<R>) + sizeof(R2<R>)) + (keep ? (size_t)kBlock * K_ * sizeof(uint16_t) : 0);
+  }
+  int solve_at_once() {
+    if (!dep_launch()) return 0;
+    const int nb = blocks_for((long long)n_);
+    if (solve_smem(true) <= (size_t)(kMaxSmemPerBlock - kStaticSmemReserve) &&
+        nb <= gpu_blocks((const void*)k_solve<R, true>, solve_smem(true)))
+      return 2;
+    return !capturing_ && nb <= gpu_blocks((const void*)k_solve<R, false>, solve_smem(false)) ? 1 : 0;
+  }
+  void launch_solve(int after, int limit) {
+    NbrArgs N = nargs();
+    N.hs = sweep_hs_;
+    const bool keep = solve_at_once() == 2;
+    const size_t smem = solve_smem(keep);
+    const auto kernel = keep ? k_solve<R, true> : k_solve<R, false>;
+    allow_smem((const void*)kernel, smem);
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(blocks_for((long long)n_));
+    lc.blockDim = dim3(kBlock);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = stream_;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    cuda_check(cudaLaunchKernelEx(&lc, kernel, d_sc_.p, (const R4<R>*)TA_.p, (const R4<R>*)TB_.p,
+                                  (const R2<R>*)SA_.p, xq_.p, xu_.p, uu_.p, press_.p, N, partials_.p, after, limit, P_),
+               "solve");
+    if (!capturing_) ++launches_;
+    else ++capture_kernels_;
+  }
+  // Blocks of a kernel that the whole GPU holds at once.
+  int gpu_blocks(const void* fn, size_t smem) {
     auto it = resident_.find({fn, smem});
     if (it != resident_.end()) return it->second;
     allow_smem(fn, smem);
     int per_sm = 0, sms = 0;
     cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, smem), "occupancy");
     cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attribute");
-    const int r = std::max(0, per_sm * sms / 2);
-    resident_[{fn, smem}] = r;
-    return r;
+    return resident_[{fn, smem}] = per_sm * sms;
   }
+
+  // The distance, in blocks, of a sweep pass's L2 prefetch (0 when it is
+  // off): half the blocks resident on the whole GPU at once, so a block's
+  // lines arrive about half a block lifetime ahead (on the 1M scene a whole
+  // wave ahead measured 2 % slower, two waves 10 %).
+  int resident_blocks(const void* fn, size_t smem) { return prefetch_ ? gpu_blocks(fn, smem) / 2 : 0; }
 
   // The pressure acceleration after a solve (a13 with the solved pressures;
   // OUT 1: +=, OUT 2: overwrite) as one more sweep pass A: the per-solve
@@ -1520,13 +1567,28 @@ class System : public SystemBase {
              (R4<R>*)nullptr, (R2<R>*)nullptr, P_, acc_.p, (const R4<R>*)TB_.p);
   }
 
+  static constexpr int kSolveSweeps = 4096;  // sweeps of one cooperative launch without a sweep cap
   // resolve_pressure_globally's loop (iisph.rs:419-550). Sweeps run on the
   // device and stop themselves once converged; the host only checks the flag
   // after a batch sized by the previous solve.
   void solve_loop(int after) {
     if (capturing_ && after < 0) {
-      solve_loop_graph();
+      if (solve_at_once()) launch_solve(after, P_.iteration_cap > 0 ? P_.iteration_cap : kGraphSweepLimit);
+      else solve_loop_graph();
       return;
+    }
+    if (solve_at_once()) {
+      // (a solve with a sweep cap always ends by itself; without one the host
+      // looks after kSolveSweeps)
+      launch_solve(after, after >= 0 ? after + 1 : cfg_.max_solver_iterations ? (int)cfg_.max_solver_iterations : kSolveSweeps);
+      if (after >= 0 || cfg_.max_solver_iterations) return;
+      for (;;) {
+        cuda_check(cudaMemcpyAsync(h_sc_, d_sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, stream_), "memcpy");
+        sync();
+        check_barrier();
+        if (h_sc_->converged) return;
+        launch_solve(after, kSolveSweeps);
+      }
     }
     // A solve takes three sweeps at least; then the host reads the flag and the
     // error. Each further batch is as long as the error's decay per sweep (of
@@ -1626,6 +1688,7 @@ class System : public SystemBase {
     }
     cuda_check(cudaMemcpyAsync(h_sc_, d_sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, stream_), "memcpy");
     sync();
+    check_barrier();
     collect_profile();
     avg_density_ = h_sc_->avg_density;
     if (h_sc_->max_nbrs > K_ || h_sc_->max_halo > hcap_) {
@@ -1686,6 +1749,10 @@ class System : public SystemBase {
     launch_impl(dep_launch() && !boundary_kind_, "volume", k_volume<R>, dim3(nb), dim3(kBlock), 0, d_sc_.p, xv_.p, (const R4<R>*)vel_.p, (const R*)bW_.p,
            boundary_kind_ ? 1 : 0, partials_.p, P_);
     calc_acceleration();
+  }
+
+  void check_barrier() const {
+    if (h_sc_->barrier_timeout) throw Error(SPH_ERR_CUDA, "the solver's blocks did not meet at their barrier");
   }
 
   // Launches between fork_side() and leave_side() go to a second stream behind
@@ -1876,6 +1943,7 @@ class System : public SystemBase {
     chunk_steps_ = 0;
     cuda_check(cudaEventSynchronize(chunk_event_), "chunk");
     const Scalars s = *h_chunk_sc_;
+    if (s.barrier_timeout) throw Error(SPH_ERR_CUDA, "the solver's blocks did not meet at their barrier");
     o.steps = c;
     if (s.trouble) {
       restore_snapshot();
@@ -1895,7 +1963,7 @@ class System : public SystemBase {
     steps_ += c;
     if (cfg_.cfl_time_step) current_time_ = s.time_acc;
     avg_density_ = s.avg_density;
-    launches_ += (uint64_t)c * graphs_[0].kernels + 3ull * s.loop_sweeps;
+    launches_ += (uint64_t)c * graphs_[0].kernels + (graphs_[0].while_node ? 3ull * s.loop_sweeps : 0ull);
     wall_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - chunk_t0_).count() / c;
     o.status = s.status_any == 2 ? SPH_NOT_CONVERGED : SPH_OK;
     return o;
@@ -1907,8 +1975,9 @@ class System : public SystemBase {
     cudaGraphExec_t exec = nullptr;
     const void* key = nullptr;  // position buffer the captured step starts from
     uint64_t kernels = 0;       // kernel nodes outside the solver loops
+    bool while_node = false;    // the solver loop is a while-node
   };
-  static constexpr int kGraphSweepLimit = 10000;  // while-node bound without a sweep cap
+  static constexpr int kGraphSweepLimit = 10000;  // a captured solve's bound without a sweep cap
   StepGraph graphs_[2];
   uint32_t graph_chunk_ = 0, chunk_steps_ = 0;
   size_t graph_n_ = 0;
@@ -1954,6 +2023,7 @@ class System : public SystemBase {
 
   void capture_step(StepGraph& g) {
     g.key = (const void*)pos_.p;
+    g.while_node = solve_at_once() != 2;
     capture_kernels_ = 0;
     cuda_check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
     capturing_ = true;
