@@ -1,24 +1,29 @@
-// CUDA kernels of the SPH step engine (sm_100a). One thread per particle;
-// neighbor lists are stored warp-tiled (see nbr_slot): the 32 particles of a
-// warp own one contiguous block, and each lane reads four consecutive
-// neighbors with one 128-bit load, so a warp streams its lists as 512-byte
-// coalesced, page-local reads. Gathered neighbor state comes through L1/L2
-// because the cell sort keeps spatial neighbors close in memory.
+// CUDA kernels of the SPH step engine (sm_100a). Mostly one thread per particle;
+// neighbor lists hold 16-bit positions in the block's halo and are stored
+// warp-tiled (see nbr_slot): the 32 particles of a warp own one contiguous
+// block, and each lane reads four consecutive neighbors with one 64-bit load, so
+// a warp streams its lists as 256-byte coalesced reads. Gathered neighbor state
+// comes from shared memory, where a block stages its halo's records.
 //
 // Reference functions each kernel restates (paths under simulation_lib/src/):
 //   k_integrate_key      integration_schemes/euler_cromer.rs:12-25,
 //                        take_predicted.rs:14-27, sph/mod.rs:674-699 (disable,
 //                        max speed), spatial_hashing.rs:27-46 (cells)
-//   k_sort_*             spatial_hashing.rs:27-37 (populate) as a counting sort
+//   k_scan_*, k_scatter, k_gather_particles
+//                        spatial_hashing.rs:27-37 (populate) as a counting sort
 //   k_neighbors_density  spatial_hashing.rs:75-158, neighbor_search/mod.rs:118-155,
-//                        sph/quantities.rs:14-61 (get_volume)
+//                        sph/quantities.rs:14-61 (get_volume's fluid sum)
+//   k_volume             sph/quantities.rs:14-61 (get_volume), average density
 //   k_sample_boundary    boundary_handling/static_sample_boundary.rs:157-168,
 //                        sph/non_pressure_accelerations.rs (boundary viscosity)
-//   k_vm_sample          boundary_handling/volume_map_boundary.rs:1259-1424,
+//   k_vm_near, k_vm_sample
+//                        boundary_handling/volume_map_boundary.rs:1259-1424,
 //                        utilities/discretization.rs:437-557
 //   k_accel              sph/non_pressure_accelerations.rs:19-185,
 //                        pressure_solver/mod.rs:90-195, sesph.rs:31-67
-//   k_iisph_*            pressure_solver/iisph.rs:117-560,
+//   k_body_react         the reactions of boundary viscosity and pressure
+//   k_iisph_source_diag, k_sweep_*, k_solve
+//                        pressure_solver/iisph.rs:117-560,
 //                        iisph_optimized_source_term.rs:53-217
 //   k_body_*             boundary_handling/rigid_body_motion.rs:135-201
 //   k_quantity_at        sph/mod.rs:241-341, sph/quantities.rs:14-330

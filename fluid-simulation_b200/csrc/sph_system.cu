@@ -2,9 +2,10 @@
 //
 // A `System<R>` owns one scene's device state and its CUDA stream and runs
 // the reference's step (sph/mod.rs:125-144, update :674-731) as a fixed
-// sequence of kernel launches. The only host synchronisation per step is the
-// final read of the step scalars (and, for IISPH with a target density
-// error, a convergence check after the first batch of sweeps).
+// sequence of kernel launches; the boundary pass runs on a second stream beside
+// the neighbor search. The only host synchronisation per step is the final read
+// of the step scalars (and, for IISPH scenes whose solve is a launch per pass, a
+// convergence check after each batch of sweeps).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
