@@ -2528,9 +2528,10 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_jacobi
 // launches takes the launches as well, and either a host that reads the error
 // between batches of sweeps or a while-node. KEEP: the lists are copied to shared
 // memory once (a warp alone on its scheduler waits for every group read from L2).
-// The 3 sweeps of 5 thousand particles took 42 us with u's second records staged
-// one load at a time; 431 -> 151 us per step stepped by calls and 138 -> 123 us in a
-// graph against a launch per pass, 5 thousand particles, four sweeps.
+// 5 thousand particles: 15 us a sweep; per step of four sweeps against a launch per
+// pass 431 -> 151 us stepped by calls and 138 -> 123 us in a graph (8 steps with the
+// lists read every sweep 1171 us, kept 997 us, and with u's second records
+// requested four at a time 984 us).
 // ---------------------------------------------------------------------------
 template <class T>
 __device__ __forceinline__ T load_l2(const T* p) {
