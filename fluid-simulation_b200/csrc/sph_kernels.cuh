@@ -1189,7 +1189,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
         }
       }
       sum = acc.s;
-      if (!(acc.farthest >= P.range2_lo)) break;
+      // (a list that is cut off at the capacity keeps its count, so that the update is redone with a larger one)
+      if (!(acc.farthest >= P.range2_lo) || found.cnt > P.K) break;
       // some neighbor lies inside the guard band: keep those the exact predicate keeps
       int kept = 0;
       for (int k = 0; k < stored; ++k) {

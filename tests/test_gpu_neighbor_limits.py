@@ -1,0 +1,45 @@
+"""The fluid neighbor search at its limits: candidates in the guard band of a list
+that is longer than its capacity.
+
+Lists are compared, as sets per particle, with a brute-force f64 search (the
+reference's predicate, sqrt((dx^2 + dy^2) + dz^2) < h).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(x, h, spacing, solver="SESPH", precision="f32", **parameters):
+    from sphgpu import GpuSystem, make_config
+    params = dict(rest_density_grid_spacing=spacing, kernel_support_radius=h, disable_particles_below=-1e6,
+                  time_increment=1e-4, stiffness=10.0, max_solver_iterations=3, **parameters)
+    g = GpuSystem(make_config({"pressure_solver": solver, "integration_scheme": "EulerCromer",
+                               "boundary_handling": "StaticSampleBoundary"}, params, precision=precision))
+    g.upload_fluid(x, None, np.full(len(x), 1000.0 * spacing ** 3))
+    g.initialize()
+    return g
+
+
+def _near(x, i, h):
+    d = x[i] - x
+    return np.nonzero(np.sqrt((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2]) < h)[0]
+
+
+# A lattice has whole shells of neighbors at the support radius: 24 at sqrt(6)
+# and sqrt(10) spacings, 56 and 122 nearer ones. In a ball of that radius the
+# center's list is longer than the capacity with the shell and shorter without it;
+# every other list is shorter.
+@pytest.mark.parametrize("shell,capacity", [(6, 72), (10, 132)])
+@pytest.mark.parametrize("solver", ["SESPH", "IISPH"])
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+def test_shell_at_the_support_radius_beyond_the_capacity(shell, capacity, solver, precision):
+    spacing = 1.0 / 64
+    h = np.sqrt(shell) * spacing
+    c = np.arange(-4, 5)
+    x = np.stack(np.meshgrid(c, c, c, indexing="ij"), -1).reshape(-1, 3)
+    x = x[(x * x).sum(1) <= shell] * spacing + 0.25
+    with _system(x, h, spacing, solver, precision, neighbor_capacity=capacity) as g:
+        off, idx = g.fluid_neighbors()
+    for i in range(len(x)):
+        assert np.array_equal(np.sort(idx[off[i]:off[i + 1]]), _near(x, i, h)), i
