@@ -670,12 +670,18 @@ struct RangeTest32 {
     return hits;
   }
 };
+// f64: NaN results keep a sign (inf - inf gives a negative one), so the test is on
+// the magnitude of r^2: its upper word, the sign shifted out, minus the limit's,
+// rounded up (a shell of 2^-18 more candidates, which the exact predicate decides).
 struct RangeTest64 {
-  double x, y, z, limit;
-  __device__ __forceinline__ RangeTest64(const R4<double>& xi, double lim) : x(xi.x), y(xi.y), z(xi.z), limit(lim) {}
-  __device__ __forceinline__ double one(double a, double b, double c) const {
+  double x, y, z;
+  uint32_t limit;
+  __device__ __forceinline__ RangeTest64(const R4<double>& xi, double lim) : x(xi.x), y(xi.y), z(xi.z) {
+    limit = ((uint32_t)__double2hiint(lim) >> 1) + 1u;
+  }
+  __device__ __forceinline__ uint32_t one(double a, double b, double c) const {
     const double dx = a - x, dy = b - y, dz = c - z;
-    return dz * dz + (dy * dy + (dx * dx - limit));
+    return ((uint32_t)__double2hiint(dz * dz + (dy * dy + dx * dx)) >> 1) - limit;
   }
   __device__ __forceinline__ uint32_t run(const double* px, const double* py, const double* pz, int n) const {
     uint32_t hits = 0;
@@ -683,8 +689,8 @@ struct RangeTest64 {
       const double2 a = *reinterpret_cast<const double2*>(px + c);
       const double2 b = *reinterpret_cast<const double2*>(py + c);
       const double2 d = *reinterpret_cast<const double2*>(pz + c);
-      hits = __funnelshift_l(sign_word(one(a.x, b.x, d.x)), hits, 1);
-      hits = __funnelshift_l(sign_word(one(a.y, b.y, d.y)), hits, 1);
+      hits = __funnelshift_l(one(a.x, b.x, d.x), hits, 1);
+      hits = __funnelshift_l(one(a.y, b.y, d.y), hits, 1);
     }
     return hits;
   }

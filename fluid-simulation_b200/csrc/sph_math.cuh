@@ -6,7 +6,6 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
-#include <math_constants.h>
 
 namespace sph {
 
@@ -176,10 +175,6 @@ __device__ __forceinline__ bool in_range(const R4<R>& a, const R4<R>& b, double 
   return in_range_exact((double)a.x, (double)a.y, (double)a.z, (double)b.x, (double)b.y,
                         (double)b.z, range);
 }
-
-// The word of a number that holds its sign bit (bit 31; NaN results carry 0).
-__device__ __forceinline__ uint32_t sign_word(float v) { return (uint32_t)__float_as_int(v); }
-__device__ __forceinline__ uint32_t sign_word(double v) { return (uint32_t)__double2hiint(v); }
 
 // Cell of a position: floor(p / cell_size) in f64, saturated to i32 like
 // Rust's `as i32` (spatial_hashing.rs:40-46).

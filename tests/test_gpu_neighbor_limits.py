@@ -1,5 +1,5 @@
 """The fluid neighbor search at its limits: candidates in the guard band of a list
-that is longer than its capacity.
+that is longer than its capacity, positions that are not finite.
 
 Lists are compared, as sets per particle, with a brute-force f64 search (the
 reference's predicate, sqrt((dx^2 + dy^2) + dz^2) < h).
@@ -43,3 +43,26 @@ def test_shell_at_the_support_radius_beyond_the_capacity(shell, capacity, solver
         off, idx = g.fluid_neighbors()
     for i in range(len(x)):
         assert np.array_equal(np.sort(idx[off[i]:off[i + 1]]), _near(x, i, h)), i
+
+
+# Not a number and infinite positions are nobody's neighbors and have none (every
+# comparison with such a distance is false), whatever the sign of the NaN.
+@pytest.mark.parametrize("value", [0x7FF8 << 48, 0xFFF8 << 48, 0x7FF0 << 48, 0xFFF0 << 48])
+@pytest.mark.parametrize("count", [1, 3])
+@pytest.mark.parametrize("solver", ["SESPH", "IISPH"])
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+def test_positions_that_are_not_finite_have_no_neighbors(value, count, solver, precision):
+    h = 0.04
+    c = (np.arange(5) + 0.5) * 0.5 * h
+    x = np.stack(np.meshgrid(c, c, c, indexing="ij"), -1).reshape(-1, 3).astype(np.float32).astype(np.float64)
+    x[10:10 + count, 1] = np.array([value], np.uint64).view(np.float64)[0]
+    with _system(x, h, 0.5 * h, solver, precision) as g:
+        off, idx = g.fluid_neighbors()
+    for i in range(len(x)):
+        got = np.sort(idx[off[i]:off[i + 1]])
+        if 10 <= i < 10 + count:
+            got = got[got != i]  # (the row of a particle holds the particle itself)
+            assert len(got) == 0, i
+        else:
+            with np.errstate(invalid="ignore"):
+                assert np.array_equal(got, _near(x, i, h)), i
