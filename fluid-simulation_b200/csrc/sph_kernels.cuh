@@ -844,10 +844,10 @@ struct OrderQueues {
 // cell's place in the halo and the three cells of a stencil row lie side by
 // side: a cell's candidates are nine runs of halo positions. A block whose
 // Morton keys cross a boundary of 16^3 cells, where the curve jumps, keeps
-// one box on either side of it (a cell that both hold is in the halo twice,
-// which only costs room). A block whose boxes or cells are too many (sparse
-// particles) sorts the stencil keys instead and visits 27 buckets per
-// particle.
+// one box on either side of it (a cell that both hold is in the halo twice, as is
+// one on either end of a box that spans the bucket grid; it only costs room). A block whose boxes or cells are too many (sparse
+// particles), or whose halo would outgrow 16-bit positions with such second
+// copies, sorts the stencil keys instead and visits 27 buckets per particle.
 //
 // Candidates: each particle walks its cell's runs in pieces of up to 32
 // positions, four at a time, two per packed f32 instruction. A test is
@@ -1001,31 +1001,36 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
         H += total;
       }
       if (tid == 0) s_off[D] = (uint16_t)min(H, 65535u);
+      // (buckets that are in it twice may take a halo over the 65535 positions that lists can
+      // address: without the second copies it may fit)
+      if (H > 65535u) boxed = false;
       __syncthreads();
-      // the halo's particle indices, and its positions where they fit: eight lanes per cell
-      for (uint32_t r = tid >> 3; r < D; r += kBlock / 8) {
-        const uint32_t o = s_off[r], e = s_off[r + 1], f = s_first[r];
-        for (uint32_t l = o + (tid & 7); l < e; l += 8) {
-          if (l < (uint32_t)hcap) hidx[l] = f + (l - o);
-          if (l < kStage) {
-            const R4<R>* p = &pos[f + (l - o)];
-            async_copy(&s_px[l], &p->x);
-            async_copy(&s_py[l], &p->y);
-            async_copy(&s_pz[l], &p->z);
+      if (boxed) {
+        // the halo's particle indices, and its positions where they fit: eight lanes per cell
+        for (uint32_t r = tid >> 3; r < D; r += kBlock / 8) {
+          const uint32_t o = s_off[r], e = s_off[r + 1], f = s_first[r];
+          for (uint32_t l = o + (tid & 7); l < e; l += 8) {
+            if (l < (uint32_t)hcap) hidx[l] = f + (l - o);
+            if (l < kStage) {
+              const R4<R>* p = &pos[f + (l - o)];
+              async_copy(&s_px[l], &p->x);
+              async_copy(&s_py[l], &p->y);
+              async_copy(&s_pz[l], &p->z);
+            }
           }
         }
+        for (int e = tid; e < 9 * (int)nheads; e += kBlock) {
+          const int h = e / 9, q = e - 9 * h;
+          const int3 c = s_cell[s_head[h]];
+          const int e1 = split ? (int)((morton_key(c.x, c.y, c.z, P.mask) >> jump) & 1u) : 0;
+          const int r = cell_rank(bit_of(c, e1, q % 3 - 1, q / 3 - 1));
+          const uint32_t o = s_off[r];
+          s_row[e] = o | ((uint32_t)(s_off[r + 3] - o) << 16);
+          if (q == 4) s_own[h] = (int)s_off[r + 1] - (int)s_first[r + 1];
+        }
+        stage_done();  // the construction buffers become the lists
+        if (active) own_local = s_own[hr] + i;
       }
-      for (int e = tid; e < 9 * (int)nheads; e += kBlock) {
-        const int h = e / 9, q = e - 9 * h;
-        const int3 c = s_cell[s_head[h]];
-        const int e1 = split ? (int)((morton_key(c.x, c.y, c.z, P.mask) >> jump) & 1u) : 0;
-        const int r = cell_rank(bit_of(c, e1, q % 3 - 1, q / 3 - 1));
-        const uint32_t o = s_off[r];
-        s_row[e] = o | ((uint32_t)(s_off[r + 3] - o) << 16);
-        if (q == 4) s_own[h] = (int)s_off[r + 1] - (int)s_first[r + 1];
-      }
-      stage_done();  // the construction buffers become the lists
-      if (active) own_local = s_own[hr] + i;
     }
   }
   if (!boxed) {

@@ -1,5 +1,6 @@
 """The fluid neighbor search at its limits: candidates in the guard band of a list
-that is longer than its capacity, positions that are not finite.
+that is longer than its capacity, positions that are not finite, a halo as large as
+16-bit positions allow.
 
 Lists are compared, as sets per particle, with a brute-force f64 search (the
 reference's predicate, sqrt((dx^2 + dy^2) + dz^2) < h).
@@ -66,3 +67,23 @@ def test_positions_that_are_not_finite_have_no_neighbors(value, count, solver, p
         else:
             with np.errstate(invalid="ignore"):
                 assert np.array_equal(got, _near(x, i, h)), i
+
+
+# Blocks on both sides of a corner see the same eight cells from either side: 34000
+# particles, 68000 halo positions with the second copies. Alone, the particles have a
+# bucket grid of eight cells per axis, on whose edge the corner lies; with one far away,
+# the grid is larger and the Morton curve jumps there. 16 ulp as in the search's own test.
+@pytest.mark.parametrize("far", [0, 1])
+def test_halo_beyond_16_bit_positions_only_with_second_copies(far):
+    from sphgpu import capi
+    h, n = 0.04, 34000
+    rng = np.random.default_rng(1)
+    x = np.column_stack([rng.uniform(0.01, 1.99, n), rng.uniform(0.01, 1.99, n), rng.uniform(15.01, 16.99, n)]) * h
+    x = np.concatenate([x, np.full((far, 3), 40.0 * h)]).astype(np.float32).astype(np.float64)
+    with _system(x, h, 0.5 * h) as g:
+        vol = g.download(capi.FIELD_VOLUME)
+    for i in rng.integers(0, n, 200):
+        d = x[i] - x[_near(x, i, h)]
+        q = np.sqrt((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2]) / h
+        w = 16.0 / np.pi / h ** 3 * (np.maximum(1 - q, 0) ** 3 - 4 * np.maximum(0.5 - q, 0) ** 3)
+        assert abs(vol[i] * w.sum() - 1.0) < 16 * 2.0 ** -23, i
