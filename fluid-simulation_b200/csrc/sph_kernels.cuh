@@ -2573,10 +2573,12 @@ __device__ __forceinline__ void stage_batch(const HaloView& H, const uint32_t (&
 
 // Barrier over a cooperative grid. The last block to arrive runs last() (all its
 // threads) before it lets the others go. The wait is bounded: a block that gives
-// up sets barrier_timeout and returns false, and so do the others in turn.
-constexpr int kBarrierPolls = 1 << 22;
+// up after `polls` looks sets barrier_timeout and returns false, and so do the
+// others in turn. The arrival count is then left as it is, and no solve runs on it
+// (k_solve looks at barrier_timeout first) until a restart sets the scalars anew.
+constexpr int kBarrierPolls = 1 << 22;  // some seconds
 template <class F>
-__device__ __forceinline__ bool grid_barrier(Scalars* sc, F&& last) {
+__device__ __forceinline__ bool grid_barrier(Scalars* sc, int polls, F&& last) {
   __shared__ unsigned s_gen;
   __shared__ int s_last, s_ok;
   __syncthreads();
@@ -2597,9 +2599,9 @@ __device__ __forceinline__ bool grid_barrier(Scalars* sc, F&& last) {
       atomicAdd(&sc->barrier_gen, 1u);
     }
   } else if (threadIdx.x == 0) {
-    int polls = 0;
+    int looks = 0;
     while (*(volatile unsigned*)&sc->barrier_gen == s_gen) {
-      if (++polls == kBarrierPolls) {
+      if (++looks >= polls) {
         sc->barrier_timeout = 1;
         s_ok = 0;
         break;
@@ -2621,11 +2623,13 @@ struct KeptList {
 template <class R, bool KEEP>
 __global__ void __launch_bounds__(kBlock, (sizeof(R) == 4 ? 4 : 2) / (KEEP ? 2 : 1)) k_solve(
     Scalars* sc, const R4<R>* __restrict__ TA, const R4<R>* __restrict__ TB, const R2<R>* __restrict__ SA,
-    R4<R>* xq, R4<R>* xu, R2<R>* uu, R* press, NbrArgs N, double* partials, int after, int limit,
+    R4<R>* xq, R4<R>* xu, R2<R>* uu, R* press, NbrArgs N, double* partials, int after, int limit, int polls,
     StepParams<R> P) {
   __shared__ double sh[32];
   extern __shared__ __align__(32) unsigned char dsm[];
-  if (*(volatile int*)&sc->converged) return;  // (set between barriers only: every block sees the same)
+  // (converged is set between barriers only: every block sees the same. A timeout is an
+  // earlier launch's, or another block's that gave up on this one: this one gives up too)
+  if (*(volatile int*)&sc->converged || *(volatile int*)&sc->barrier_timeout) return;
   R4<R>* s_a = reinterpret_cast<R4<R>*>(dsm);
   R2<R>* s_b = reinterpret_cast<R2<R>*>(s_a + N.hs);
   const HaloView H = halo_view(N);
@@ -2689,7 +2693,7 @@ __global__ void __launch_bounds__(kBlock, (sizeof(R) == 4 ? 4 : 2) / (KEEP ? 2 :
         uu[i] = u2;
       }
     }
-    if (!grid_barrier(sc, [] {})) return;
+    if (!grid_barrier(sc, polls, [] {})) return;
     // pass B
     double e = 0.0;
     {
@@ -2739,7 +2743,7 @@ __global__ void __launch_bounds__(kBlock, (sizeof(R) == 4 ? 4 : 2) / (KEEP ? 2 :
     }
     const double bs = block_sum(e, sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = bs;
-    const bool ok = grid_barrier(sc, [&] {  // (the sum of last_block_total)
+    const bool ok = grid_barrier(sc, polls, [&] {  // (the sum of last_block_total)
       double t = 0;
       for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) t += ((volatile double*)partials)[b];
       t = block_sum(t, sh);

@@ -322,6 +322,7 @@ class System : public SystemBase {
     steps_ = 0;
     current_time_ = 0.0;
     update(2);  // System::new_boxed's first update (sph/mod.rs:418-419)
+    read_solve_limits();
     initialized_ = true;
   }
 
@@ -1533,7 +1534,7 @@ class System : public SystemBase {
     lc.attrs = at;
     lc.numAttrs = 1;
     cuda_check(cudaLaunchKernelEx(&lc, kernel, d_sc_.p, (const R4<R>*)TA_.p, (const R4<R>*)TB_.p,
-                                  (const R2<R>*)SA_.p, xq_.p, xu_.p, uu_.p, press_.p, N, partials_.p, after, limit, P_),
+                                  (const R2<R>*)SA_.p, xq_.p, xu_.p, uu_.p, press_.p, N, partials_.p, after, limit, polls_, P_),
                "solve");
     if (!capturing_) ++launches_;
     else ++capture_kernels_;
@@ -1569,6 +1570,20 @@ class System : public SystemBase {
   }
 
   static constexpr int kSolveSweeps = 4096;  // sweeps of one cooperative launch without a sweep cap
+  // The limits of a cooperative solve (tests lower them): the looks of a block that
+  // waits at its barrier, the sweeps of a launch without a sweep cap. Read once a system
+  // is initialized, and again when it restarts from a checkpoint.
+  int polls_ = kBarrierPolls, solve_sweeps_ = kSolveSweeps;
+  void read_solve_limits() {
+    auto read = [](const char* name, int usual) {
+      const char* e = std::getenv(name);
+      return e ? std::max(1, std::min(std::atoi(e), usual)) : usual;
+    };
+    const int polls = read("SPHGPU_BARRIER_POLLS", kBarrierPolls);
+    if (polls != polls_) destroy_graphs();  // the captured launches carry the old one
+    polls_ = polls;
+    solve_sweeps_ = read("SPHGPU_SOLVE_SWEEPS", kSolveSweeps);
+  }
   // resolve_pressure_globally's loop (iisph.rs:419-550). Sweeps run on the
   // device and stop themselves once converged; the host only checks the flag
   // after a batch sized by the previous solve.
@@ -1580,15 +1595,15 @@ class System : public SystemBase {
     }
     if (solve_at_once()) {
       // (a solve with a sweep cap always ends by itself; without one the host
-      // looks after kSolveSweeps)
-      launch_solve(after, after >= 0 ? after + 1 : cfg_.max_solver_iterations ? (int)cfg_.max_solver_iterations : kSolveSweeps);
+      // looks after solve_sweeps_)
+      launch_solve(after, after >= 0 ? after + 1 : cfg_.max_solver_iterations ? (int)cfg_.max_solver_iterations : solve_sweeps_);
       if (after >= 0 || cfg_.max_solver_iterations) return;
       for (;;) {
         cuda_check(cudaMemcpyAsync(h_sc_, d_sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, stream_), "memcpy");
         sync();
         check_barrier();
         if (h_sc_->converged) return;
-        launch_solve(after, kSolveSweeps);
+        launch_solve(after, solve_sweeps_);
       }
     }
     // A solve takes three sweeps at least; then the host reads the flag and the
@@ -2263,6 +2278,7 @@ void System<R>::restore(uint64_t steps, double time, size_t n, const double* x, 
   if (!initialized_) throw Error(SPH_ERR_STATE, "initialize before restoring a checkpoint");
   if (n > cap_) throw Error(SPH_ERR_INVALID, "checkpoint holds more particles than the system");
   n_ = n;
+  read_solve_limits();
   load_state(n, x, v, m, fid);
   note_groups(fid, n);
   if (cfg_.integration_scheme == SPH_TAKE_PREDICTED) {
@@ -2289,6 +2305,10 @@ void System<R>::restore(uint64_t steps, double time, size_t n, const double* x, 
   s.n_active = (int)n;
   s.n_below = 0;
   s.max_speed = 0;
+  // (after an error: the solver's barrier and the reductions start afresh)
+  s.barrier_count = s.barrier_gen = 0;
+  s.barrier_timeout = 0;
+  s.done_blocks = 0;
   copy_h2d(d_sc_.p, &s, 1);
   *h_sc_ = s;
   update(2);  // continue_from_checkpoint (sph/mod.rs:362-378)
