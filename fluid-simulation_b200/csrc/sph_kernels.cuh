@@ -92,6 +92,11 @@ __device__ __forceinline__ bool last_block_total(double block_value, double* par
 // every block of this grid has started). Both are no-ops in a plain launch.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+// Such a kernel's pointers carry no __restrict__: the kernel before may still write
+// what they point to, so the promise does not hold, and with it the compiler may read
+// through the non-coherent cache or move an access above the wait. (__ldg is for
+// what nothing has written since the kernel before the last one ended: halo indices
+// behind the volume pass, field nodes.)
 // The start of a kernel that reads what the kernel before it wrote: its blocks
 // are on their SMs by then, and the next kernel's may follow (small scenes, where
 // a step is a dozen kernels of 3 to 30 us, save the launch latency between them).
@@ -251,7 +256,7 @@ __device__ __forceinline__ uint32_t block_excl_scan_u32(uint32_t v, uint32_t* sh
 // A thread's kScanItems consecutive counts: two 16-byte loads when they lie
 // inside [0, m) (the arrays are 16-byte aligned and base is a multiple of 8).
 static_assert(kScanItems == 8, "two uint4 per thread");
-__device__ __forceinline__ void scan_load8(const uint32_t* __restrict__ in, int base, int m, uint32_t v[8]) {
+__device__ __forceinline__ void scan_load8(const uint32_t* in, int base, int m, uint32_t v[8]) {
   if (base + 8 <= m) {
     const uint4 a = __ldcs(reinterpret_cast<const uint4*>(in + base));
     const uint4 b = __ldcs(reinterpret_cast<const uint4*>(in + base) + 1);
@@ -263,8 +268,8 @@ __device__ __forceinline__ void scan_load8(const uint32_t* __restrict__ in, int 
 }
 
 constexpr int kScanDirect = 2048;
-__global__ void __launch_bounds__(kBlock) k_scan_tiles(const uint32_t* __restrict__ in, int m,
-                                                      uint32_t* __restrict__ tile_sums, Prologue prologue) {
+__global__ void __launch_bounds__(kBlock) k_scan_tiles(const uint32_t* in, int m,
+                                                      uint32_t* tile_sums, Prologue prologue) {
   grid_dep_begin();
   __shared__ uint32_t sh[32];
   if (prologue.sc && blockIdx.x == 0 && threadIdx.x == 0) run_prologue(prologue);
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_tiles(const uint32_t* __restric
   if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_tile_sums(uint32_t* __restrict__ tile_sums, int ntiles) {
+__global__ void __launch_bounds__(1024) k_scan_tile_sums(uint32_t* tile_sums, int ntiles) {
   grid_dep_begin();
   __shared__ uint32_t sh[32];
   // each thread owns a contiguous run of tiles
@@ -297,9 +302,9 @@ __global__ void __launch_bounds__(1024) k_scan_tile_sums(uint32_t* __restrict__ 
 }
 
 template <bool DIRECT>
-__global__ void __launch_bounds__(kBlock) k_scan_apply(uint32_t* __restrict__ in, int m,
-                                                      const uint32_t* __restrict__ tile_sums,
-                                                      uint32_t* __restrict__ out) {
+__global__ void __launch_bounds__(kBlock) k_scan_apply(uint32_t* in, int m,
+                                                      const uint32_t* tile_sums,
+                                                      uint32_t* out) {
   grid_dep_begin();
   __shared__ uint32_t sh[32];
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
@@ -343,11 +348,11 @@ __global__ void __launch_bounds__(kBlock) k_scan_apply(uint32_t* __restrict__ in
 // ---------------------------------------------------------------------------
 // 3. scatter, then gather with in-bucket ordering by reference index
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) k_scatter(const int* __restrict__ n_ptr,
-                                                   const uint32_t* __restrict__ key,
-                                                   const uint32_t* __restrict__ slot,
-                                                   const uint32_t* __restrict__ start,
-                                                   uint32_t* __restrict__ perm) {
+__global__ void __launch_bounds__(kBlock) k_scatter(const int* n_ptr,
+                                                   const uint32_t* key,
+                                                   const uint32_t* slot,
+                                                   const uint32_t* start,
+                                                   uint32_t* perm) {
   grid_dep_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= *n_ptr) return;
@@ -359,10 +364,10 @@ __global__ void __launch_bounds__(kBlock) k_scatter(const int* __restrict__ n_pt
 // assignment: every entry counts the smaller ones of its bucket. (One thread
 // per bucket sorting by insertion took 14 to 25 us where a sphere's samples
 // crowd a bucket.)
-__device__ __forceinline__ uint32_t ranked_place(uint32_t j, const uint32_t* __restrict__ key,
-                                                 const uint32_t* __restrict__ start,
-                                                 const uint32_t* __restrict__ order,
-                                                 const uint32_t* __restrict__ perm) {
+__device__ __forceinline__ uint32_t ranked_place(uint32_t j, const uint32_t* key,
+                                                 const uint32_t* start,
+                                                 const uint32_t* order,
+                                                 const uint32_t* perm) {
   const uint32_t k = key[j], b = start[k], e = start[k + 1], mine = order[j];
   uint32_t rank = 0;
 #pragma unroll 4
@@ -372,10 +377,10 @@ __device__ __forceinline__ uint32_t ranked_place(uint32_t j, const uint32_t* __r
 
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_gather_particles(
-    const int* __restrict__ n_ptr, const uint32_t* __restrict__ perm, const uint32_t* __restrict__ key,
-    const uint32_t* __restrict__ start, const R4<R>* __restrict__ pos, const R4<R>* __restrict__ vel,
-    const uint32_t* __restrict__ ref, const uint32_t* __restrict__ fid, R4<R>* __restrict__ pos2,
-    R4<R>* __restrict__ vel2, uint32_t* __restrict__ ref2, uint32_t* __restrict__ fid2) {
+    const int* n_ptr, const uint32_t* perm, const uint32_t* key,
+    const uint32_t* start, const R4<R>* pos, const R4<R>* vel,
+    const uint32_t* ref, const uint32_t* fid, R4<R>* pos2,
+    R4<R>* vel2, uint32_t* ref2, uint32_t* fid2) {
   grid_dep_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= *n_ptr) return;
@@ -865,9 +870,9 @@ struct OrderQueues {
 // order; in this form 270 us for both.
 template <class R, bool ORDER>
 __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
-    Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const uint32_t* __restrict__ start,
-    R4<R>* __restrict__ xv, uint16_t* __restrict__ nbr, uint32_t* __restrict__ ncnt,
-    uint32_t* __restrict__ halo_idx, uint32_t* __restrict__ halo_n, int hcap, StepParams<R> P) {
+    Scalars* sc, const R4<R>* pos, const uint32_t* start,
+    R4<R>* xv, uint16_t* nbr, uint32_t* ncnt,
+    uint32_t* halo_idx, uint32_t* halo_n, int hcap, StepParams<R> P) {
   grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   __shared__ int s_own[kSearchCells];        // per cell: own bucket's halo offset - its first particle
@@ -1357,10 +1362,10 @@ __device__ bool ser_gradient(const DevField& F, double px, double py, double pz,
 // passes are bound by f64 issue and the latency of the node loads).
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_vm_near(
-    Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const VMDesc* __restrict__ vms, int nvm,
-    const Body* __restrict__ bodies, uint32_t* __restrict__ near_list, R4<R>* __restrict__ vmx,
-    R4<R>* __restrict__ vmv, R* __restrict__ bW, R4<R>* __restrict__ bG, R4<R>* __restrict__ bGu,
-    R4<R>* __restrict__ bA, StepParams<R> P) {
+    Scalars* sc, const R4<R>* pos, const VMDesc* vms, int nvm,
+    const Body* bodies, uint32_t* near_list, R4<R>* vmx,
+    R4<R>* vmv, R* bW, R4<R>* bG, R4<R>* bGu,
+    R4<R>* bA, StepParams<R> P) {
   grid_dep_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= sc->n_active) return;
@@ -1460,10 +1465,10 @@ __device__ __forceinline__ R boundary_viscosity(const V3<R>& r, const V3<R>& dv,
 
 template <class R>
 __global__ void __launch_bounds__(kBlock, 3) k_vm_sample(
-    Scalars* __restrict__ sc, const uint32_t* __restrict__ near_list, const R4<R>* __restrict__ pos,
-    const R4<R>* __restrict__ vel, const VMDesc* __restrict__ vms, int nvm, const Body* __restrict__ bodies,
-    R4<R>* __restrict__ vmx, R4<R>* __restrict__ vmv, R* __restrict__ bW, R4<R>* __restrict__ bG,
-    R4<R>* __restrict__ bGu, R4<R>* __restrict__ bA, uint32_t* __restrict__ touch, StepParams<R> P) {
+    Scalars* sc, const uint32_t* near_list, const R4<R>* pos,
+    const R4<R>* vel, const VMDesc* vms, int nvm, const Body* bodies,
+    R4<R>* vmx, R4<R>* vmv, R* bW, R4<R>* bG,
+    R4<R>* bGu, R4<R>* bA, uint32_t* touch, StepParams<R> P) {
   grid_dep_begin();
   const int lane = threadIdx.x & 31, e = lane & 7;
   const unsigned group = 0xffu << (lane & ~7);
@@ -1762,9 +1767,9 @@ struct SampleStage {  // per warp
 
 template <class R, bool SPLIT>
 __global__ void __launch_bounds__(kBlock) k_sample_boundary(
-    Scalars* __restrict__ sc, const R4<R>* __restrict__ pos, const R4<R>* __restrict__ vel, SampleGrid<R> G,
-    const Body* __restrict__ bodies, int any_dynamic, R* __restrict__ bW, R4<R>* __restrict__ bG,
-    R4<R>* __restrict__ bGu, R4<R>* __restrict__ bA, uint32_t* __restrict__ touch, StepParams<R> P) {
+    Scalars* sc, const R4<R>* pos, const R4<R>* vel, SampleGrid<R> G,
+    const Body* bodies, int any_dynamic, R* bW, R4<R>* bG,
+    R4<R>* bGu, R4<R>* bA, uint32_t* touch, StepParams<R> P) {
   grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   __shared__ uint32_t s_key[kSampleBlock], s_heads[kSampleBlock / 32];
@@ -2109,9 +2114,9 @@ __device__ __forceinline__ void sweep_groups(List& L, Load&& load, Use&& use) {
 // PRESS: 0 none, 1 SESPH state equation from the volume on the fly
 template <class R, int PRESS>
 __global__ void __launch_bounds__(kBlock) k_accel(
-    const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv, const R4<R>* __restrict__ vel,
-    NbrArgs N, BoundaryArgs<R> B, R4<R>* __restrict__ acc, R4<R>* __restrict__ vstar,
-    R* __restrict__ press, int write_vstar, StepParams<R> P) {
+    const Scalars* sc, const R4<R>* xv, const R4<R>* vel,
+    NbrArgs N, BoundaryArgs<R> B, R4<R>* acc, R4<R>* vstar,
+    R* press, int write_vstar, StepParams<R> P) {
   grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   const HaloView H = halo_view(N);
@@ -2195,8 +2200,8 @@ __global__ void __launch_bounds__(kBlock) k_accel(
 // acc += accel (the solvers with Jacobi sweeps take it from k_sweep_accel)
 template <class R>
 __global__ void __launch_bounds__(kBlock) k_pressure_accel(
-    const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv, const R4<R>* __restrict__ vel,
-    const R* __restrict__ press, NbrArgs N, BoundaryArgs<R> B, R4<R>* __restrict__ out, StepParams<R> P) {
+    const Scalars* sc, const R4<R>* xv, const R4<R>* vel,
+    const R* press, NbrArgs N, BoundaryArgs<R> B, R4<R>* out, StepParams<R> P) {
   grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   const HaloView H = halo_view(N);
@@ -2252,10 +2257,10 @@ __global__ void __launch_bounds__(kBlock) k_pressure_accel(
 // velocity-divergence source of IISPHwOST's first solve.
 template <class R, int VP>
 __global__ void __launch_bounds__(kBlock) k_iisph_source_diag(
-    const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv, const R4<R>* __restrict__ vel,
-    const R4<R>* __restrict__ vstar, NbrArgs N, BoundaryArgs<R> B, R* __restrict__ s_out,
-    R* __restrict__ aii_out, R* __restrict__ press, R4<R>* __restrict__ TA, R4<R>* __restrict__ TB,
-    R2<R>* __restrict__ SA, R4<R>* __restrict__ xq_out, StepParams<R> P) {
+    const Scalars* sc, const R4<R>* xv, const R4<R>* vel,
+    const R4<R>* vstar, NbrArgs N, BoundaryArgs<R> B, R* s_out,
+    R* aii_out, R* press, R4<R>* TA, R4<R>* TB,
+    R2<R>* SA, R4<R>* xq_out, StepParams<R> P) {
   grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   const HaloView H = halo_view(N);
@@ -2355,9 +2360,9 @@ __global__ void __launch_bounds__(kBlock) k_iisph_source_diag(
 // reaction on dynamic bodies is k_body_react).
 template <class R, int OUT = 0>
 __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_accel(
-    const Scalars* __restrict__ sc, const R* __restrict__ press, const R4<R>* __restrict__ TA,
-    const R4<R>* __restrict__ xq, NbrArgs N, R4<R>* __restrict__ xu, R2<R>* __restrict__ uu, StepParams<R> P,
-    R4<R>* __restrict__ acc, const R4<R>* __restrict__ TB) {
+    const Scalars* sc, const R* press, const R4<R>* TA,
+    const R4<R>* xq, NbrArgs N, R4<R>* xu, R2<R>* uu, StepParams<R> P,
+    R4<R>* acc, const R4<R>* TB) {
   grid_dep_release();
   extern __shared__ __align__(32) unsigned char dsm[];
   const HaloView H = halo_view(N);
@@ -2449,9 +2454,9 @@ __device__ __forceinline__ void end_sweep(Scalars* sc, double total, int n, int 
 // AFTER >= 0: stop after AFTER+1 sweeps; AFTER < 0: target density error.
 template <class R>
 __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_jacobi(
-    Scalars* __restrict__ sc, const R4<R>* __restrict__ TB, const R2<R>* __restrict__ SA,
-    const R4<R>* __restrict__ xu, const R2<R>* __restrict__ uu, NbrArgs N, R* __restrict__ press,
-    R4<R>* __restrict__ xq, double* __restrict__ partials, int after, StepParams<R> P) {
+    Scalars* sc, const R4<R>* TB, const R2<R>* SA,
+    const R4<R>* xu, const R2<R>* uu, NbrArgs N, R* press,
+    R4<R>* xq, double* partials, int after, StepParams<R> P) {
   grid_dep_release();
   __shared__ double sh[32];
   extern __shared__ __align__(32) unsigned char dsm[];
@@ -2800,9 +2805,9 @@ __global__ void __launch_bounds__(kBlock) k_ost_commit(const Scalars* __restrict
 //                      + (m_i/V0) bW + dt v*_i . bGu, p = k max(V0/(m_i/rho*) - 1, 0)
 template <class R, int NB>
 __global__ void __launch_bounds__(kBlock) k_split_density(
-    const Scalars* __restrict__ sc, const R4<R>* __restrict__ xv, const R4<R>* __restrict__ vel,
-    const R4<R>* __restrict__ vstar, NbrArgs N, BoundaryArgs<R> B, R* __restrict__ press,
-    R* __restrict__ rho_pred, StepParams<R> P) {
+    const Scalars* sc, const R4<R>* xv, const R4<R>* vel,
+    const R4<R>* vstar, NbrArgs N, BoundaryArgs<R> B, R* press,
+    R* rho_pred, StepParams<R> P) {
   grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   const HaloView H = halo_view(N);
@@ -2857,9 +2862,9 @@ __global__ void __launch_bounds__(kBlock) k_split_density(
 // that entered this one and those it disabled in n_in and n_disabled (nothing
 // after the sort reads n, n_below or max_speed).
 template <class R>
-__global__ void __launch_bounds__(kBlock) k_volume(Scalars* __restrict__ sc, R4<R>* __restrict__ xv,
-                                                  const R4<R>* __restrict__ vel, const R* __restrict__ bW,
-                                                  int has_boundary, double* __restrict__ partials,
+__global__ void __launch_bounds__(kBlock) k_volume(Scalars* sc, R4<R>* xv,
+                                                  const R4<R>* vel, const R* bW,
+                                                  int has_boundary, double* partials,
                                                   StepParams<R> P) {
   grid_dep_begin();
   __shared__ double sh[32];
@@ -3100,7 +3105,7 @@ __global__ void k_chunk_begin(Scalars* sc, double time) {
 // until the sweep kernel sets `converged` or `limit` sweeps have run. Every
 // body execution either finds `converged` set or adds one to `iterations`,
 // so the loop ends after at most `limit` bodies.
-__global__ void k_loop_cond(cudaGraphConditionalHandle h, const Scalars* __restrict__ sc, int limit) {
+__global__ void k_loop_cond(cudaGraphConditionalHandle h, const Scalars* sc, int limit) {
   grid_dep_wait();
   const unsigned int more = (!sc->converged && sc->iterations < limit) ? 1u : 0u;
   cudaGraphSetConditional(h, more);
