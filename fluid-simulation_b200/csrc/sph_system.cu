@@ -233,10 +233,11 @@ class System : public SystemBase {
     cap_ = std::max<size_t>(n, 1);
     np_ = round_up(cap_, 32);
     alloc_particles();
-    load_state(n, x, v, m, fid);
+    // (before load_state waits for the stream: another upload gives these back to the pool)
     acc_.zero(stream_);
     xint_.zero(stream_);
     vint_.zero(stream_);
+    load_state(n, x, v, m, fid);
     host_bbox_.clear();
     for (size_t i = 0; i < n; ++i) bbox_add(x[3 * i], x[3 * i + 1], x[3 * i + 2]);
     note_groups(fid, n);
