@@ -258,10 +258,12 @@ class Server {
     for (const auto& b : j.samples) s->add_sample_boundary(b.x.size() / 3, b.x.data(), b.dyn ? &b.rigid : nullptr);
     for (const auto& f : j.vmaps)
       s->add_volume_map(f.sd, f.sn.data(), f.vd, f.vn.data(), f.dyn ? &f.rigid : nullptr);
-    s->initialize();
     // concurrent scenes share the SMs: blocks of an early-launched dependent
-    // kernel would hold SM resources another scene's kernels could use
+    // kernel would hold SM resources another scene's kernels could use, and the
+    // first update's solve in one cooperative launch would wait until all its
+    // blocks fit beside theirs
     s->set_dependent_launch(false);
+    s->initialize();
     s->set_step_graphs(cfg_.chunk_steps);
     j.sys = std::move(s);
     // the inputs are on the device now
