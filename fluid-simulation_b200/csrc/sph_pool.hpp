@@ -91,16 +91,9 @@ class Pool {
     if (last) trim();
   }
 
-  // Gives everything kept back to the driver.
-  void trim() {
-    std::lock_guard<std::mutex> lock(mu_);
-    for (auto& k : kept_) {
-      for (auto& c : k.second.blocks)
-        for (void* p : c.second) raw_free(p, k.first);
-      k.second.blocks.clear();
-      k.second.bytes = 0;
-    }
-  }
+  // Gives everything kept back to the driver, or what is kept of one device.
+  void trim() { trim_if([](int) { return true; }); }
+  void trim(int where) { trim_if([where](int w) { return w == where; }); }
 
   size_t kept_bytes(int where) {
     std::lock_guard<std::mutex> lock(mu_);
@@ -108,6 +101,18 @@ class Pool {
   }
 
  private:
+  template <class F>
+  void trim_if(F&& of) {
+    std::lock_guard<std::mutex> lock(mu_);
+    for (auto& k : kept_) {
+      if (!of(k.first)) continue;
+      for (auto& c : k.second.blocks)
+        for (void* p : c.second) raw_free(p, k.first);
+      k.second.blocks.clear();
+      k.second.bytes = 0;
+    }
+  }
+
   struct Kept {
     std::map<size_t, std::vector<void*>> blocks;
     size_t bytes = 0;

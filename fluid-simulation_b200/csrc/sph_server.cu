@@ -82,9 +82,10 @@ static uint64_t estimate_bytes(const SceneJob& j) {
   double per = 4 * w * 8 + 4 * 8 + w * 2 + 2 * K + 4 * 8192.0 / 256;  // state, sort, p/bW, lists, halo table
   if (ps != SPH_SESPH) per += 4 * w;                    // predicted velocity
   if (ps == SPH_IISPH || ps == SPH_IISPH_W_OST) per += 2 * w + 18 * w;  // s, a_ii; sweep records xq, xu, uu, TA, TB, SA
-  if (ps == SPH_SESPH_W_SPLITTING) per += w;
+  if (ps == SPH_SESPH_W_SPLITTING) per += w + 4 * w;    // predicted density, bGu
   if (j.cfg.integration_scheme == SPH_TAKE_PREDICTED) per += 2 * 4 * w * 2;
   per += 3 * 4 * w + 8;                                 // snapshot
+  per += 2 * 4;                                         // touch list, particles near a volume map
   per += j.vmaps.size() * 2 * 4 * w;                    // volume-map samples
   size_t ns = 0;
   for (const auto& s : j.samples) ns += s.x.size() / 3;
@@ -109,7 +110,7 @@ static uint64_t estimate_bytes(const SceneJob& j) {
   while (mbits < 8 && (double)(1u << mbits) < ext) ++mbits;
   const double T = (double)(1u << (3 * mbits)) + 2;
   bytes += T * 4 * (ns ? 4 : 2) + 2 * 8 * (double)(n / 256 + 1);
-  return (uint64_t)(bytes * 1.1) + (4u << 20);
+  return (uint64_t)(bytes * 1.15) + (4u << 20);  // (the pool's size classes round up by an eighth at most)
 }
 
 class Server {
@@ -336,6 +337,9 @@ class Server {
         done_cv_.notify_all();
         cv_.notify_all();
       }
+      // what the pool keeps of earlier scenes counts against the budget as well
+      // (reserved_ changes on this thread alone)
+      if (reserved_ + Pool::get().kept_bytes(cfg_.device) > budget_) Pool::get().trim(cfg_.device);
       if (job) {
         job->result.start_s = now();
         try {

@@ -238,6 +238,9 @@ class System : public SystemBase {
     xint_.zero(stream_);
     vint_.zero(stream_);
     load_state(n, x, v, m, fid);
+    stage_x_.release();  // (steps with host buffers and restarts take them again)
+    stage_v_.release();
+    stage_m_.release();
     host_bbox_.clear();
     for (size_t i = 0; i < n; ++i) bbox_add(x[3 * i], x[3 * i + 1], x[3 * i + 2]);
     note_groups(fid, n);

@@ -167,6 +167,9 @@ typedef struct sph_system sph_system_t;
 /* Creates an empty system on cfg->device. Rejects the pairings the reference
  * rejects in SystemConstructor::new (sph/setup/mod.rs:229-244). */
 int sph_create(const sph_config* cfg, sph_system_t** out);
+/* While any system or scene server of the process lives, up to 1 GiB per device
+ * and 64 MiB of pinned memory of destroyed systems are kept for the next ones.
+ * The last one to go gives them back, as does an allocation that fails. */
 void sph_destroy(sph_system_t* h);
 /* Deep copy of all device state (SPHSystem: DynClone, sci-phi-backend/src/lib.rs:111). */
 int sph_clone(const sph_system_t* h, sph_system_t** out);
@@ -421,7 +424,8 @@ typedef struct sph_server sph_server_t;
 
 typedef struct sph_server_config {
   int device;                   /* CUDA device ordinal */
-  uint64_t memory_budget_bytes; /* 0: 90 % of the device memory free at creation */
+  uint64_t memory_budget_bytes; /* scenes and memory kept for reuse; 0: 90 % of the device
+                                   memory free at creation */
   uint32_t max_active;          /* scenes on the device at once; 0: 64 */
   uint32_t chunk_steps;         /* graph launches per host check; 0: 25 */
 } sph_server_config;
