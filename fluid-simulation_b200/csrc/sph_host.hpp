@@ -74,6 +74,7 @@ class SystemBase {
   // programmatic dependent launch between the sweep passes (on by default;
   // the scene server turns it off: its scenes share the SMs)
   virtual void set_dependent_launch(bool on) = 0;
+  virtual void release_staging() = 0;  // of uploads; taken again when needed
   virtual uint32_t contact_sweeps() const = 0;
   virtual void rigid_state(int bi, double* out) = 0;
   virtual void set_rigid_state(int bi, const double* in) = 0;

@@ -256,6 +256,7 @@ class Server {
   void build(SceneJob& j) {
     std::unique_ptr<SystemBase> s(create_system(j.cfg));
     s->upload_fluid(j.m.size(), j.x.data(), j.v.data(), j.m.data(), j.fid.data());
+    s->release_staging();
     for (const auto& b : j.samples) s->add_sample_boundary(b.x.size() / 3, b.x.data(), b.dyn ? &b.rigid : nullptr);
     for (const auto& f : j.vmaps)
       s->add_volume_map(f.sd, f.sn.data(), f.vd, f.vn.data(), f.dyn ? &f.rigid : nullptr);

@@ -238,9 +238,6 @@ class System : public SystemBase {
     xint_.zero(stream_);
     vint_.zero(stream_);
     load_state(n, x, v, m, fid);
-    stage_x_.release();  // (steps with host buffers and restarts take them again)
-    stage_v_.release();
-    stage_m_.release();
     host_bbox_.clear();
     for (size_t i = 0; i < n; ++i) bbox_add(x[3 * i], x[3 * i + 1], x[3 * i + 2]);
     note_groups(fid, n);
@@ -1397,6 +1394,11 @@ class System : public SystemBase {
     if (pdl_ == on) return;
     pdl_ = on;
     destroy_graphs();  // the captured launches carry the old setting
+  }
+  void release_staging() override {  // (the calls that use it wait for their copies)
+    stage_x_.release();
+    stage_v_.release();
+    stage_m_.release();
   }
   void set_contact_sweeps(uint32_t fixed) override {
     if (chunk_steps_) throw Error(SPH_ERR_STATE, "a chunk of graph steps is in flight");
