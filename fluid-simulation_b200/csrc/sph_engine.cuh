@@ -47,7 +47,7 @@ struct Scalars {
   int max_nbrs;                    // largest fluid neighbor count seen
   int iterations;                  // IISPH sweeps of the last solve
   int converged;                   // IISPH loop flag (1 = stop)
-  double err;                      // IISPH average predicted density error (%)
+  double err, err_before;          // IISPH average predicted density error (%), now and a sweep earlier
   double avg_density;              // average mass density after the update
   unsigned int done_blocks;        // last-block-done counter for reductions
   int status;                      // 0 ok, 2 not converged within the cap

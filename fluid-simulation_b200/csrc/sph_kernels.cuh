@@ -2433,6 +2433,7 @@ __device__ __forceinline__ void end_sweep(Scalars* sc, double total, int n, int 
   const double err = n > 0 ? total / (double)n * 100.0 : 0.0;
   const int it = sc->iterations + 1;
   sc->iterations = it;
+  sc->err_before = sc->err;
   sc->err = err;
   bool stop;
   if (after >= 0) {

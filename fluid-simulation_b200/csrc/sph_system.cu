@@ -845,7 +845,6 @@ class System : public SystemBase {
   uint64_t steps_ = 0;
   double current_time_ = 0, time_offset_ = 0, wall_ = 0, avg_density_ = 0;
   uint64_t time_offset_steps_ = 0;
-  double sweep_decay_ = 0.1;  // decay of the solver's error per sweep, last seen (ln of the ratio)
   int nb_ = 4;  // neighbor gather batch (prefetch width) of the neighbor passes
   bool pdl_ = true;       // programmatic dependent launch between the sweep passes
   bool prefetch_ = true;  // sweep passes prefetch the next wave's streams into L2
@@ -1591,8 +1590,7 @@ class System : public SystemBase {
     solve_sweeps_ = read("SPHGPU_SOLVE_SWEEPS", kSolveSweeps);
   }
   // resolve_pressure_globally's loop (iisph.rs:419-550). Sweeps run on the
-  // device and stop themselves once converged; the host only checks the flag
-  // after a batch sized by the previous solve.
+  // device and stop themselves once converged.
   void solve_loop(int after) {
     if (capturing_ && after < 0) {
       if (solve_at_once()) launch_solve(after, P_.iteration_cap > 0 ? P_.iteration_cap : kGraphSweepLimit);
@@ -1613,34 +1611,34 @@ class System : public SystemBase {
       }
     }
     // A solve takes three sweeps at least; then the host reads the flag and the
-    // error. Each further batch is as long as the error's decay per sweep (of
-    // this solve so far, else of the last one) says that the solve still needs:
-    // a check costs the stream about 12 us of idling, a sweep launched in vain
-    // 11 us (133 thousand particles) to 25 us (one million), and a batch as long
-    // as the last solve launched up to 19 of those when a solve of 22 sweeps was
-    // followed by one of 3. Timed (profiling) solves run one sweep per check, so
-    // that every timed sweep launch does a sweep's work; the results are the same.
+    // error, and launches a further batch (next_batch). Timed (profiling) solves run
+    // one sweep per check, so that every timed sweep launch does a sweep's work; the
+    // results are the same.
     int batch = after >= 0 ? after + 1 : profiling_ ? 1 : 3;
     if (after < 0 && cfg_.max_solver_iterations) batch = std::min(batch, (int)cfg_.max_solver_iterations);
     for (int k = 0; k < batch; ++k) iisph_iteration(after, k == 0);
     if (after >= 0) return;
-    double err_before = 0.0;
-    int sweeps_before = 0;
     for (;;) {
       cuda_check(cudaMemcpyAsync(h_sc_, d_sc_.p, sizeof(Scalars), cudaMemcpyDeviceToHost, stream_), "memcpy");
       sync();
-      const double err = h_sc_->err;
-      const int sweeps = h_sc_->iterations;
-      if (sweeps_before > 0 && sweeps > sweeps_before && err > 0.0 && err < err_before)
-        sweep_decay_ = std::log(err_before / err) / (sweeps - sweeps_before);
       if (h_sc_->converged) break;
-      double need = cfg_.target_density_error > 0.0 && err > cfg_.target_density_error && std::isfinite(err)
-                        ? std::log(err / cfg_.target_density_error) / sweep_decay_ : 2.0;
-      batch = profiling_ ? 1 : (int)std::min(64.0, std::max(2.0, std::ceil(need)));
+      batch = profiling_ ? 1 : next_batch(h_sc_->iterations);
       for (int k = 0; k < batch; ++k) iisph_iteration(after, false);
-      err_before = err;
-      sweeps_before = sweeps;
     }
+  }
+  // Sweeps to launch before the host looks again: as many as the error's last decay says
+  // that the solve still needs, at most twice those done, four when the error is not
+  // falling, and none beyond the sweep cap. A look costs the stream about 12 us of idling,
+  // a sweep launched in vain 11 us (133 thousand particles) to 25 us (one million). Only
+  // this solve's own errors decide, so that a flow's first solve is launched as its tenth.
+  int next_batch(int sweeps) const {
+    const double err = h_sc_->err, before = h_sc_->err_before, tde = cfg_.target_density_error;
+    double n = 4.0;
+    if (tde > 0.0 && err > tde && before > err && std::isfinite(before))
+      n = std::max(2.0, std::min(std::ceil(std::log(err / tde) / std::log(before / err)),
+                                 std::min(64.0, std::max(8.0, 2.0 * sweeps))));
+    if (cfg_.max_solver_iterations) n = std::min(n, (double)cfg_.max_solver_iterations - sweeps);
+    return std::max(1, (int)n);
   }
 
   void calc_acceleration() {

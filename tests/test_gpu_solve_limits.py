@@ -1,6 +1,6 @@
 """The cooperative solve at its limits: which launches a step makes, a launch that
-ends before the solve does, a barrier whose wait runs out, and two solves at once
-whose blocks each fill the GPU.
+ends before the solve does, a barrier whose wait runs out, two solves at once whose
+blocks each fill the GPU, and the sweeps that a launch per pass makes in vain.
 
 SPHGPU_BARRIER_POLLS and SPHGPU_SOLVE_SWEEPS lower the looks of a waiting block and
 the sweeps of one launch; they are read once a system is initialized and again when
@@ -106,3 +106,49 @@ def test_two_solves_at_once_that_each_fill_the_gpu():
     for t in threads:
         t.join()
     assert _same(states[0], states["alone"]) and _same(states[1], states["alone"])
+
+
+@pytest.mark.parametrize("cap", [4, 10, 40, 100])
+def test_no_sweep_is_launched_beyond_the_cap(monkeypatch, cap):
+    # an error that is never reached: two launches per sweep of the cap, no more
+    from sphgpu import scenes
+    monkeypatch.setenv("SPHGPU_DEPENDENT_LAUNCH", "0")
+    launches = []
+    for c in (3, cap):
+        with scenes.build_system(_scene(8000, c, 1e-9)) as g:
+            launches.append([_step(g) for _ in range(3)])
+    for (base, three), (got, sweeps) in zip(*launches):
+        assert (three, sweeps) == (3, cap)
+        assert got - base == 2 * (cap - 3)
+
+
+@pytest.mark.parametrize("n", [8000, 160000])
+def test_the_launches_of_a_solve_do_not_depend_on_earlier_ones(monkeypatch, n):
+    # the same state after other flows; a converging solve has sweeps in vain, but no
+    # more than twice those that it took
+    from sphgpu import scenes
+    monkeypatch.setenv("SPHGPU_DEPENDENT_LAUNCH", "0")
+    sc = _scene(n, 100, 0.1)
+    ck = None
+    out = []
+    for history in range(3):
+        with scenes.build_system(sc) as g:
+            if ck is None:
+                ck = g.get_fluid_checkpoint()
+                x = ck["position"]
+                ck["velocity"] = -8.0 * (x - x.mean(0))
+            if history == 1:
+                g.step_forward_in_time(8)
+            if history == 2:
+                g.continue_from_checkpoint(dict(ck, velocity=0.25 * ck["velocity"]))
+                g.step_forward_in_time(2)
+            before = g.launch_count()
+            g.continue_from_checkpoint(ck)
+            got = [(g.launch_count() - before, g.step_stats()["solver_iterations"])]
+            out.append(got + [_step(g) for _ in range(3)])
+    assert out[1] == out[0] and out[2] == out[0]
+    assert max(s for _, s in out[0]) > 6, out[0]
+    with scenes.build_system(_scene(n, 3, 0.1)) as g:
+        base = _step(g)[0]
+    for launches, sweeps in out[0][1:]:
+        assert launches - base <= 2 * (sweeps - 3) + 2 * max(8, 2 * sweeps), out[0]
