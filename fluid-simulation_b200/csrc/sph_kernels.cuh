@@ -625,28 +625,6 @@ static_assert(kHaloKeys * (sizeof(uint32_t) + sizeof(uint16_t)) <= kSearchX + kS
 static_assert(kBoxCells / 32 * (sizeof(uint32_t) + sizeof(uint16_t)) + (kHaloCells + 2) * sizeof(uint16_t) +
                       kHaloCells * sizeof(uint32_t) + kBlock * sizeof(int3) <= kSearchL, "halo construction buffers");
 
-// Two f32 operations in one instruction (each rounded like the scalar one).
-__device__ __forceinline__ unsigned long long pack2(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 // Distance tests of one particle against n staged candidates (n a multiple of
 // four, px/py/pz 16-byte aligned): the sign bit of r^2 - limit of candidate c
 // ends at bit n - 1 - c.
@@ -706,8 +684,7 @@ using RangeTest = std::conditional_t<sizeof(R) == 4, RangeTest32, RangeTest64>;
 // Compensated (Kahan) sum of W over the neighbors in list order, on top of the
 // self term W(0) = alpha/h^3 / 2; add() takes the coordinates of four
 // neighbors, of which the first n count, and keeps the largest squared
-// distance. f32: two kernel values per packed instruction (the square root is r^2 rsqrt(r^2) with one Heron step, its
-// residual in one fma, which gives the rounded root).
+// distance. f32: two kernel values per packed instruction.
 struct KernelSum32 {
   unsigned long long x, y, z;
   float ih, cw, s, c = 0.f, farthest = 0.f;
@@ -726,16 +703,9 @@ struct KernelSum32 {
     // (a coincident neighbor keeps a finite root)
     const float r0 = fmaxf(__uint_as_float((uint32_t)r2), 1e-35f);
     const float r1 = fmaxf(__uint_as_float((uint32_t)(r2 >> 32)), 1e-35f);
-    const unsigned long long d = pack2(r0, r1);
     farthest = fmaxf(farthest, r0);
     if (n > 1) farthest = fmaxf(farthest, r1);
-    float i0, i1;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i0) : "f"(r0));
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i1) : "f"(r1));
-    const unsigned long long inv = pack2(i0, i1);
-    const unsigned long long minus = pack2(-1.f, -1.f), half = pack2(0.5f, 0.5f);
-    unsigned long long r = mul2(d, inv);
-    r = fma2(fma2(mul2(r, minus), r, d), mul2(inv, half), r);
+    const unsigned long long half = pack2(0.5f, 0.5f), r = roots2(r0, r1);
     // -|r|/h, in scalar form: a packed product and the packed sums behind it
     // were measured to round once, and with them the volumes' last bits change
     const unsigned long long q = pack2(__fmul_rn(__uint_as_float((uint32_t)r), ih),
@@ -2391,7 +2361,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_accel(
   R px = 0, py = 0, pz = 0;
   auto pair = [&](const R4<R>& r) {
     const R rx = xi.x - r.x, ry = xi.y - r.y, rz = xi.z - r.z;
-    const R t = r.w * grad_third(rx, ry, rz, ih);
+    const R t = r.w * grad_third_close(rx, ry, rz, ih);
     px += t * rx; py += t * ry; pz += t * rz;
   };
   if (H.staged) {
@@ -2683,7 +2653,7 @@ __global__ void __launch_bounds__(kBlock, (sizeof(R) == 4 ? 4 : 2) / (KEEP ? 2 :
         R px = 0, py = 0, pz = 0;
         auto pair = [&](const R4<R>& r) {
           const R rx = xi.x - r.x, ry = xi.y - r.y, rz = xi.z - r.z;
-          const R t = r.w * grad_third(rx, ry, rz, ih);
+          const R t = r.w * grad_third_close(rx, ry, rz, ih);
           px += t * rx; py += t * ry; pz += t * rz;
         };
         if (H.staged)

@@ -72,14 +72,51 @@ __host__ KernelConst<R> make_kernel_const(double h) {
 template <class R>
 __device__ __forceinline__ R sq(R x) { return x * x; }
 
-// a / b. f32: the approximate reciprocal and one Newton step on the quotient
-// (its residual in one fma), within an ulp for the b > 0 of the pair loops.
+// a / b for the b > 0 of the pair loops. f32: the approximate reciprocal (an ulp) and one
+// Newton step on the quotient, its residual in one fma. Before the last rounding the
+// relative error is below 2^-45, so the result is the rounded quotient, or its neighbor
+// where that lies within 2^-20 ulp of a tie.
 __device__ __forceinline__ double quotient(double a, double b) { return a / b; }
 __device__ __forceinline__ float quotient(float a, float b) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
   const float q = a * r;
   return fmaf(fmaf(-b, q, a), r, q);
+}
+
+// Two f32 operations in one instruction (each rounded like the scalar one).
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Both square roots, r0 and r1 > 0: r^2 rsqrt(r^2) and one Heron step, its residual in one
+// fma. Before the last rounding the relative error is below 2^-43 (the approximate
+// reciprocal root's is 2^-22.4 at most): the rounded root, or its neighbor where that lies
+// within 2^-19 ulp of a tie.
+__device__ __forceinline__ unsigned long long roots2(float r0, float r1) {
+  float i0, i1;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i0) : "f"(r0));
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(i1) : "f"(r1));
+  const unsigned long long d = pack2(r0, r1), inv = pack2(i0, i1);
+  const unsigned long long r = mul2(d, inv);
+  return fma2(fma2(mul2(r, pack2(-1.f, -1.f)), r, d), mul2(inv, pack2(0.5f, 0.5f)), r);
 }
 
 // W from the squared distance; zero outside the support.
@@ -104,10 +141,12 @@ __device__ __forceinline__ R kernel_grad_factor(R r2, const KernelConst<R>& k) {
 }
 
 // f32: w'(q) / |r| = 3 ((1-2q)_+^2 - (1-q)_+^2) / |r| from one approximate
-// reciprocal square root (relative error ~1e-7, far inside the f32 state's
-// tolerance); the clamps ride in saturating FMAs, and the squared distance is
-// kept away from 0, where the factor is exactly 0, so that there is no compare
-// and no select. f64 keeps the exact form.
+// reciprocal square root; the clamps ride in saturating FMAs, and the squared
+// distance is kept away from 0, where the factor is exactly 0, so that there is
+// no compare and no select. The difference of squares cancels for close pairs, and
+// (1-q)^2 has its own relative error near the support: relative to the factor, 1e-7
+// (rms) for q in 0.3 to 0.6, 6e-7 at 0.1, 5e-6 at 0.01, 1.4e-6 at 0.9 (the form
+// before, 12 (1/2-q)_+^2 - 3 (1-q)_+^2, cancels more). f64 keeps the exact form.
 __device__ __forceinline__ float grad_third_r2(float r2, float inv_h) {  // -1/3 w'(q) / |r|, r2 > 0
   float inv, t, b;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(r2));
@@ -135,6 +174,26 @@ __device__ __forceinline__ R grad_third(R rx, R ry, R rz, R inv_h) {
 template <>
 __device__ __forceinline__ float grad_third<float>(float rx, float ry, float rz, float inv_h) {
   return grad_third_r2(fmaf(rz, rz, fmaf(ry, ry, fmaf(rx, rx, 1e-30f))), inv_h);
+}
+
+// The same for pass A of the sweeps, whose sums weigh close pairs most (p grows as they
+// approach): for q < 1/3 in f32 the form without cancellation, (2 - 3q) / h, in one FMA on
+// |r| = r^2 rsqrt(r^2) (rms relative error 2e-8 below 0.1, 5e-8 at 0.3); the two forms are
+// equally exact at 1/3.
+template <class R>
+__device__ __forceinline__ R grad_third_close(R rx, R ry, R rz, R inv_h) {
+  return grad_third(rx, ry, rz, inv_h);
+}
+template <>
+__device__ __forceinline__ float grad_third_close<float>(float rx, float ry, float rz, float inv_h) {
+  const float r2 = fmaf(rz, rz, fmaf(ry, ry, fmaf(rx, rx, 1e-30f)));
+  float inv, t, b;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(r2));
+  const float r = r2 * inv;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(t) : "f"(r), "f"(-inv_h), "f"(1.f));  // (1-q)_+
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(b) : "f"(t), "f"(2.f), "f"(-1.f));    // (1-2q)_+
+  const float close = fmaf(r, -3.f * inv_h * inv_h, 2.f * inv_h);
+  return t > 2.f / 3.f ? close : fmaf(-b, b, t * t) * inv;
 }
 
 // Both W and the gradient factor from one square root.

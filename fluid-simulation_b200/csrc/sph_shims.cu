@@ -417,6 +417,21 @@ __global__ void k_static_count(int n, const double* __restrict__ pos, const doub
   counts[i + 1] = c;
 }
 
+// The f32 arithmetic of the pair loops beside CUDA's own, for the tests.
+__global__ void k_pair_math(int op, int n, const float* a, const float* b, float* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float x = a[i], y = b[i];
+  switch (op) {
+    case 0: out[i] = sph::quotient(x, y); break;
+    case 1: out[i] = __fdiv_rn(x, y); break;
+    case 2: out[i] = __uint_as_float((uint32_t)(sph::roots2(y, x) >> 32)); break;
+    case 3: out[i] = __fsqrt_rn(x); break;
+    case 4: out[i] = sph::grad_third<float>(x, 0.f, 0.f, y); break;
+    default: out[i] = sph::grad_third_close<float>(x, 0.f, 0.f, y);
+  }
+}
+
 }  // namespace
 
 extern "C" int sph_spatial_hashing_find_samples_noalloc(double search_range, size_t n, const double* d_positions,
@@ -467,6 +482,19 @@ extern "C" int sph_spatial_hashing_find_samples_noalloc(double search_range, siz
                                   search_range, nullptr, d_offsets, d_indices);
     check(cudaGetLastError(), "find_samples_noalloc");
     check(cudaDeviceSynchronize(), "find_samples_noalloc");
+    return SPH_OK;
+  });
+}
+
+// Not part of the interface (tests only): a, b and out of n floats on the host.
+extern "C" int sph_test_pair_math(int op, size_t n, const float* a, const float* b, float* out, int device) {
+  return run(device, [&]() -> int {
+    Buf<float> da(n), db(n), dout(n);
+    check(cudaMemcpy(da.p, a, n * sizeof(float), cudaMemcpyHostToDevice), "cudaMemcpy");
+    check(cudaMemcpy(db.p, b, n * sizeof(float), cudaMemcpyHostToDevice), "cudaMemcpy");
+    k_pair_math<<<(unsigned)((n + 255) / 256), 256>>>(op, (int)n, da.p, db.p, dout.p);
+    check(cudaGetLastError(), "pair_math");
+    check(cudaMemcpy(out, dout.p, n * sizeof(float), cudaMemcpyDeviceToHost), "cudaMemcpy");
     return SPH_OK;
   });
 }
