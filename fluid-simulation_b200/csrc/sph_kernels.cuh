@@ -782,6 +782,23 @@ struct FoundList {
   }
 };
 
+// Writes a list in whole groups of four 16-bit halo positions, an 8-byte store each; the
+// last group is completed with the particle's own position.
+struct ListWriter {
+  uint2* groups;  // this particle's group 0; group g sits 32 uint2 further
+  int cap;        // list capacity (a multiple of four)
+  uint32_t g0 = 0, g1 = 0;
+  __device__ __forceinline__ void add(int k, uint32_t l) {
+    const int q = k & 3;
+    if (q < 2) g0 = q == 0 ? l : (g0 | (l << 16));
+    else g1 = q == 2 ? l : (g1 | (l << 16));
+    if (q == 3 && k < cap) groups[(size_t)(k >> 2) * 32] = make_uint2(g0, g1);
+  }
+  __device__ __forceinline__ void finish(int cnt, uint32_t self) {
+    for (int k = cnt; (k & 3) != 0; ++k) add(k, self);
+  }
+};
+
 // Bank-aware list order: a particle's entries in one queue per halo position
 // modulo 8 (a full queue passes its entries on to the next); slot k of lane j
 // takes from queue (j + k) mod 8, or the next one that has entries left. A
@@ -832,6 +849,15 @@ struct OrderQueues {
 // inside the guard band by the exact f64 predicate, and a particle that loses
 // one there takes the pass again. The lists then go out in whole groups of
 // four, for the IISPH sweeps (ORDER) in bank-aware order.
+//
+// A halo beyond the staged positions (a compressed scene; f64 at ordinary densities)
+// goes through shared memory in pieces, by the same tests. Its lists are longer than
+// the staged ones, so what a mask finds is summed at once and written group by group
+// (the sweeps do not stage such halos either, so their order is of no use). 195 thousand
+// SESPH particles after 500 steps, 187 to 363 neighbors at most: 273, 371 and 405 us for
+// three stiffnesses; 661, 925 and 1052 us when every candidate was fetched through the
+// halo's index and its list kept two bytes at a time in global memory, 472, 606 and
+// 740 us with the test-and-append loop. f64, 64 thousand: a step's update 1396 -> 1270 us.
 //
 // What bounds it: issue (about 216 candidates per particle; 73 % of the issue
 // slots used, 211 M warp instructions for one million particles at spacing
@@ -1099,39 +1125,26 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
   const bool staged = H <= usable && H <= kStage;
   FoundList found;
   const uint32_t pad = (uint32_t)own_local < usable ? (uint32_t)own_local : 0u;  // the unused slots of a list's last group
-  if (active) {
-    if (miss) atomicMax(&sc->max_halo, 0x7fffffff);  // a bucket beyond 65535 particles
-    found.s = s_list + tid;
-    found.list = nbr + nbr_slot(i, 0, P.K);
-    found.cap = P.K;
-    const RangeTest<R> range(xi, P.range2_out);
-    // (positions beyond a halo table that is too small are skipped: the update is redone with a larger one)
-    auto position = [&](uint32_t l) {
-      return staged ? R4<R>{s_px[l], s_py[l], s_pz[l], R(0)} : pos[hidx[l]];
-    };
+  found.s = s_list + tid;
+  found.list = nbr + (active ? nbr_slot(i, 0, P.K) : 0);
+  found.cap = P.K;
+  const RangeTest<R> range(xi, P.range2_out);
+  if (active && miss) atomicMax(&sc->max_halo, 0x7fffffff);  // a bucket beyond 65535 particles
+  // Candidates of the particle among the staged positions [base, base + count) of the halo:
+  // use(hits, p) with candidate p + c of those positions at bit 31 - c of hits.
+  auto visit = [&](uint32_t base, uint32_t count, auto&& use) {
     auto test_run = [&](uint32_t row) {
-      const uint32_t o = row & 0xffffu, end = o + (row >> 16);
+      const uint32_t first = row & 0xffffu, last = first + (row >> 16);
+      if (last <= base || first >= base + count) return;
+      const uint32_t o = max(first, base) - base, end = min(last - base, count);
       for (uint32_t p = o & ~3u; p < end; p += 32) {
         const int n = min(32, (int)((end - p + 3u) & ~3u));
-        uint32_t hits;  // candidate p + c at bit 31 - c
-        if (staged) {
-          hits = range.run(s_px + p, s_py + p, s_pz + p, n) << (32 - n);
-        } else {
-          hits = 0;
-          for (int c = 0; c < n; ++c) {
-            const uint32_t l = p + c;
-            if (l >= o && l < end && l < usable) {
-              const R4<R> xj = pos[hidx[l]];
-              const R dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-              if (dx * dx + dy * dy + dz * dz < P.range2_out) hits |= 0x80000000u >> c;
-            }
-          }
-        }
+        uint32_t hits = range.run(s_px + p, s_py + p, s_pz + p, n) << (32 - n);
         if (p < o) hits &= 0xffffffffu >> (o - p);
         if (end - p < 32u) hits &= ~(0xffffffffu >> (end - p));
-        const uint32_t self = (uint32_t)own_local - p;
+        const uint32_t self = (uint32_t)own_local - base - p;
         if (self < 32u) hits &= ~(0x80000000u >> self);
-        found.add(hits, p);
+        use(hits, p);
       }
     };
     if (boxed) {
@@ -1142,12 +1155,79 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
 #pragma unroll 1
       for (int q = 0; q < 27; ++q) test_run(span[q]);
     }
+  };
+  if (!staged) {
+    // A larger halo goes through shared memory in pieces. What a particle finds in a mask of
+    // candidates is summed at once, and its list goes out group by group.
+    KernelSum<R> acc(xi, P.k);
+    ListWriter list;
+    list.groups = reinterpret_cast<uint2*>(found.list);
+    list.cap = P.K;
+    for (uint32_t base = 0; base < usable; base += kStage) {
+      const uint32_t count = min(kStage, usable - base);
+      if (base > 0 || !boxed) {  // (the first piece is there where the halo was built from boxes)
+        __syncthreads();
+        for (uint32_t l = tid; l < count; l += kBlock) {
+          const R4<R>* p = &pos[hidx[base + l]];
+          async_copy(&s_px[l], &p->x);
+          async_copy(&s_py[l], &p->y);
+          async_copy(&s_pz[l], &p->z);
+        }
+        stage_done();
+      }
+      if (active)
+        visit(base, count, [&](uint32_t hits, uint32_t p) {
+          auto position = [&](uint32_t l) { return R4<R>{s_px[l], s_py[l], s_pz[l], R(0)}; };
+          for (;;) {
+            KernelSum<R> next = acc;
+            next.farthest = R(0);
+            for (uint32_t left = hits; left;) {
+              R4<R> xj[4];
+              const int n = min(__popc(left), 4);
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                const int hb = left ? __clz(left) : 0;  // (beyond the last: any position)
+                left &= ~(0x80000000u >> hb);
+                xj[u] = position(p + (uint32_t)hb);
+              }
+              next.add(xj, n);
+            }
+            if (next.farthest >= P.range2_lo) {  // some lie inside the guard band
+              uint32_t keep = 0;
+              for (uint32_t left = hits; left;) {
+                const int hb = __clz(left);
+                left ^= 0x80000000u >> hb;
+                if (in_range(xi, position(p + (uint32_t)hb), P.range, P.range2_lo, P.range2_hi)) keep |= 0x80000000u >> hb;
+              }
+              if (keep != hits) {
+                hits = keep;
+                continue;
+              }
+            }
+            acc = next;
+            break;
+          }
+          while (hits) {
+            const int hb = __clz(hits);
+            hits ^= 0x80000000u >> hb;
+            list.add(found.cnt++, base + p + (uint32_t)hb);
+          }
+        });
+    }
+    if (active) {
+      list.finish(found.cnt, pad);
+      xv[i] = R4<R>{xi.x, xi.y, xi.z, acc.s};  // (k_volume puts the volume in its place)
+      ncnt[i] = (uint32_t)found.cnt;
+    }
+  } else if (active) {
+    visit(0, H, [&](uint32_t hits, uint32_t p) { found.add(hits, p); });
+    auto position = [&](uint32_t l) { return R4<R>{s_px[l], s_py[l], s_pz[l], R(0)}; };
     // the kernel sum in list order
     R sum;
     for (;;) {
       const int stored = min(found.cnt, P.K);
       KernelSum<R> acc(xi, P.k);
-      if (staged && !found.global) {
+      if (!found.global) {
         const uint16_t* e = found.s;
         int k = stored;
         for (; k >= 4; k -= 4, e += 4 * kBlock) {
@@ -1193,7 +1273,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
   // the particle's own halo position: the passes over neighbors read whole
   // groups, and the self pair adds zero.
   if (ORDER) __syncthreads();  // the queues take the place of the positions
-  if (active) {
+  if (active && staged) {
     const int stored = min(found.cnt, P.K);
     uint2* groups = reinterpret_cast<uint2*>(found.list);
     OrderQueues queue;

@@ -1,6 +1,6 @@
 """The fluid neighbor search at its limits: candidates in the guard band of a list
-that is longer than its capacity, positions that are not finite, a halo as large as
-16-bit positions allow.
+that is longer than its capacity, positions that are not finite, halos that fill the
+staged positions or go through them in pieces, a halo as large as 16-bit positions allow.
 
 Lists are compared, as sets per particle, with a brute-force f64 search (the
 reference's predicate, sqrt((dx^2 + dy^2) + dz^2) < h).
@@ -87,3 +87,38 @@ def test_halo_beyond_16_bit_positions_only_with_second_copies(far):
         q = np.sqrt((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2]) / h
         w = 16.0 / np.pi / h ** 3 * (np.maximum(1 - q, 0) ** 3 - 4 * np.maximum(0.5 - q, 0) ** 3)
         assert abs(vol[i] * w.sum() - 1.0) < 16 * 2.0 ** -23, i
+
+
+def _check_lists(x, h, spacing, solver, precision):
+    from sphgpu import capi
+    with _system(x, h, spacing, solver, precision) as g:
+        off, idx = g.fluid_neighbors()
+        vol = g.download(capi.FIELD_VOLUME)
+    tol = 16 * 2.0 ** -23 if precision == "f32" else 1e-13  # (as in the search's own test)
+    for i in range(len(x)):
+        near = _near(x, i, h)
+        assert np.array_equal(np.sort(idx[off[i]:off[i + 1]]), near), i
+        d = x[i] - x[near]
+        q = np.sqrt((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2]) / h
+        w = 16.0 / np.pi / h ** 3 * (np.maximum(1 - q, 0) ** 3 - 4 * np.maximum(0.5 - q, 0) ** 3)
+        assert abs(vol[i] * w.sum() - 1.0) < tol, i
+
+
+# All particles of a scene in 2 x 2 x 2 cells are every block's halo: around one, two and
+# four pieces of 1024 (f64) and 2048 (f32) staged positions.
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 2047, 2048, 2049, 4096, 4099])
+@pytest.mark.parametrize("solver,precision", [("SESPH", "f32"), ("IISPH", "f32"), ("SESPH", "f64")])
+def test_halo_in_pieces(n, solver, precision):
+    h = 0.04
+    x = np.random.default_rng(n).uniform(0.01, 1.99, (n, 3)) * h
+    _check_lists(x.astype(np.float32).astype(np.float64), h, 0.5 * h, solver, precision)
+
+
+# 72 pairs of a particle at the support radius, in a halo of some pieces
+@pytest.mark.parametrize("solver", ["SESPH", "IISPH"])
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+def test_shell_at_the_support_radius_in_pieces(solver, precision):
+    spacing = 1.0 / 64
+    c = np.arange(14) * spacing
+    x = np.stack(np.meshgrid(c, c, c, indexing="ij"), -1).reshape(-1, 3)
+    _check_lists(x, np.sqrt(26.0) * spacing, spacing, solver, precision)
