@@ -1796,7 +1796,8 @@ __device__ __forceinline__ void body_accum_flush(double* sh, int nbodies, double
 // kSampleBlock particles, about as many): 27 lanes read the stencil's bucket
 // bounds at once, and a cell without samples around it (most of them) is
 // done. Otherwise its candidates are staged in shared memory, and 4 or 8 lanes
-// share them for every particle of the cell. A lane first tests its
+// share them for every particle of the cell. (A block with fewer cells than warps, as
+// in a compressed scene, hands out its cells' groups of eight particles instead.) A lane first tests its
 // candidates into a mask, then sums over the set bits. The kernel values go
 // through shared memory to one lane, which sums them in sample order (the
 // volume's compensated sum keeps its bits whatever the split).
@@ -1841,8 +1842,18 @@ __global__ void __launch_bounds__(kBlock) k_sample_boundary(
   __syncthreads();
   SampleStage<R>& T = reinterpret_cast<SampleStage<R>*>(dsm)[warp];
   int most = 0;
-  for (int h = warp; h < nheads; h += kBlock / 32) {
+  constexpr int kWarps = kBlock / 32;
+  const bool spread = nheads < kWarps;  // fewer cells than warps: their groups of eight particles one by one
+  for (int h = spread ? 0 : warp, units = 0; h < nheads; h += spread ? 1 : kWarps) {
     const int p0 = s_head[h], np = s_head[h + 1] - p0;
+    const int S = np <= 4 ? 8 : 4;  // lanes per particle
+    int g0 = 0, g_step = 32 / S;
+    if (spread) {
+      g0 = 8 * ((warp - units) & (kWarps - 1));
+      g_step = 8 * kWarps;
+      units += (np + 7) / 8;
+      if (g0 >= np) continue;
+    }
     const uint32_t ck = s_key[p0];
     uint32_t first = 0, len = 0;
     if (lane < 27) {
@@ -1860,9 +1871,8 @@ __global__ void __launch_bounds__(kBlock) k_sample_boundary(
       if (lane >= o) end += y;
     }
     const uint32_t C = __shfl_sync(0xffffffffu, end, 31), begin = end - len;
-    const int S = np <= 4 ? 8 : 4;  // lanes per particle
     const int sub = lane & (S - 1), row = lane / S;
-    for (int g = 0; g < np; g += 32 / S) {
+    for (int g = g0; g < np; g += g_step) {
       const int p = g + row;
       const bool mine = p < np;
       const int ip = i0 + p0 + (mine ? p : 0);
