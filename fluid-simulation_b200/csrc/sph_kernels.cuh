@@ -1054,7 +1054,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
     for (int k = 2; k <= S; k <<= 1)
       for (int j = k >> 1; j > 0; j >>= 1) {
         for (int t = tid; t < (S >> 1); t += kBlock) {
-          const int a = (t / j) * 2 * j + (t % j), b = a + j;
+          const int a = 2 * t - (t & (j - 1)), b = a + j;
           const uint32_t ka = skey[a], kb = skey[b];
           if ((ka > kb) == ((a & k) == 0)) {
             skey[a] = kb;
