@@ -54,6 +54,7 @@ struct Scalars {
   int iterations_eqs1;             // IISPHwOST first solve sweeps
   int max_bnbrs;                   // largest boundary-sample neighbor count seen
   int max_halo;                    // largest block halo (particles) seen
+  int n_wide;                      // blocks whose halo exceeds the staged records
   unsigned int vm_near;            // particles within the support radius of a volume map
   unsigned int n_touch;            // particles with a neighbor on a dynamic body
   unsigned int barrier_count, barrier_gen;  // grid barrier of the cooperative solve

@@ -211,6 +211,7 @@ __device__ __forceinline__ void run_prologue(const Prologue& P) {
   sc->max_nbrs = 0;
   sc->max_bnbrs = 0;
   sc->max_halo = 0;
+  sc->n_wide = 0;
   sc->vm_near = 0;
   sc->n_touch = 0;
   sc->iterations = 0;
@@ -868,7 +869,7 @@ template <class R, bool ORDER>
 __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
     Scalars* sc, const R4<R>* pos, const uint32_t* start,
     R4<R>* xv, uint16_t* nbr, uint32_t* ncnt,
-    uint32_t* halo_idx, uint32_t* halo_n, int hcap, StepParams<R> P) {
+    uint32_t* halo_idx, uint32_t* halo_n, int hcap, int stage, StepParams<R> P) {
   grid_dep_begin();
   extern __shared__ __align__(32) unsigned char dsm[];
   __shared__ int s_own[kSearchCells];        // per cell: own bucket's halo offset - its first particle
@@ -1120,6 +1121,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
   if (tid == 0) {
     halo_n[blockIdx.x] = H;
     atomicMax(&sc->max_halo, (int)min(H, 0x7fffffffu));
+    if (H > (uint32_t)stage) atomicAdd(&sc->n_wide, 1);
   }
   const uint32_t usable = min(H, (uint32_t)hcap);
   const bool staged = H <= usable && H <= kStage;

@@ -869,6 +869,7 @@ class System : public SystemBase {
   // records, and with 1536 the acceleration and source passes of 133 thousand
   // particles took 26 and 27 us, now 19 each)
   int hs_ = sizeof(R) == 4 ? 1792 : 1024;
+  bool unstaged_ = false;  // most blocks' halos are larger (note_halos)
   // the same for the IISPH sweep passes (f32: 1792 x 24 B lets five pass-B
   // blocks share an SM's shared memory)
   int sweep_hs_ = sizeof(R) == 4 ? 1792 : 1024;
@@ -1141,9 +1142,21 @@ class System : public SystemBase {
   void launch(const char* name, Kern kernel, dim3 g, dim3 b, Args... args) {
     launch_s(name, kernel, g, b, 0, args...);
   }
+  // Halo records that the acceleration, source and split passes stage. A block whose halo
+  // is larger gathers from global memory and wants the L1 that staged records would take:
+  // where most blocks of the last update were such (a compressed scene), none are staged
+  // until three in four fit again. The results are the same. 60 thousand crowded particles,
+  // SESPHwSplitting: accelerations and split density 224 + 189 + 126 us with 1792 records
+  // reserved (which leave no L1), 134 + 120 + 86 with 1536, 101 + 94 + 68 with none.
+  int stage() const { return unstaged_ ? 0 : hs_; }
+  void note_halos(const Scalars& s) {
+    const int nb = blocks_for((long long)s.n_active);
+    if (2 * s.n_wide > nb) unstaged_ = true;
+    else if (4 * s.n_wide < nb) unstaged_ = false;
+  }
   // dynamic shared memory of a halo-staging pass: nvec R4 and nscal R arrays
   size_t smem_of(int nvec, int nscal) const {
-    return (size_t)hs_ * ((size_t)nvec * sizeof(R4<R>) + (size_t)nscal * sizeof(R));
+    return (size_t)stage() * ((size_t)nvec * sizeof(R4<R>) + (size_t)nscal * sizeof(R));
   }
   NbrArgs nargs() const {
     NbrArgs N;
@@ -1153,7 +1166,7 @@ class System : public SystemBase {
     N.hn = halo_n_.p;
     N.K = K_;
     N.hcap = hcap_;
-    N.hs = hs_;
+    N.hs = stage();
     return N;
   }
   template <class Kern, class... Args>
@@ -1721,6 +1734,7 @@ class System : public SystemBase {
       update(2);
       return;
     }
+    note_halos(*h_sc_);
     finish_disable();
   }
 
@@ -1764,7 +1778,7 @@ class System : public SystemBase {
     const bool order = sizeof(R) == 4 && (cfg_.pressure_solver == SPH_IISPH || cfg_.pressure_solver == SPH_IISPH_W_OST);
     launch_dep("neighbors_density", order ? k_neighbors_density<R, sizeof(R) == 4> : k_neighbors_density<R, false>,
              dim3(nb), dim3(kBlock), kSearchSmem, d_sc_.p, (const R4<R>*)pos_.p, (const uint32_t*)start_.p, xv_.p,
-             nbr_.p, ncnt_.p, halo_idx_.p, halo_n_.p, hcap_, P_);
+             nbr_.p, ncnt_.p, halo_idx_.p, halo_n_.p, hcap_, hs_, P_);
     join_side();
     launch_impl(dep_launch() && !boundary_kind_, "volume", k_volume<R>, dim3(nb), dim3(kBlock), 0, d_sc_.p, xv_.p, (const R4<R>*)vel_.p, (const R*)bW_.p,
            boundary_kind_ ? 1 : 0, partials_.p, P_);
@@ -1926,6 +1940,7 @@ class System : public SystemBase {
     if ((int)t.gather_batch == nb_ && (int)t.halo_stage == hs_ && (int)t.sweep_stage == sweep_hs_) return;
     nb_ = (int)t.gather_batch;
     hs_ = (int)t.halo_stage;
+    unstaged_ = false;
     sweep_hs_ = (int)t.sweep_stage;
     destroy_graphs();  // the captured launches carry the old parameters
   }
@@ -1980,6 +1995,7 @@ class System : public SystemBase {
       return o;
     }
     *h_sc_ = s;
+    note_halos(s);
     steps_ += c;
     if (cfg_.cfl_time_step) current_time_ = s.time_acc;
     avg_density_ = s.avg_density;
@@ -2001,7 +2017,7 @@ class System : public SystemBase {
   StepGraph graphs_[2];
   uint32_t graph_chunk_ = 0, chunk_steps_ = 0;
   size_t graph_n_ = 0;
-  int graph_K_ = 0, graph_hcap_ = 0;
+  int graph_K_ = 0, graph_hcap_ = 0, graph_stage_ = 0;
   bool capturing_ = false, in_loop_body_ = false;
   uint64_t capture_kernels_ = 0, graph_replays_ = 0;
   cudaStream_t body_stream_ = nullptr;
@@ -2025,7 +2041,7 @@ class System : public SystemBase {
   }
 
   void prepare_graphs() {
-    if (graphs_[0].exec && graph_n_ == n_ && graph_K_ == K_ && graph_hcap_ == hcap_) return;
+    if (graphs_[0].exec && graph_n_ == n_ && graph_K_ == K_ && graph_hcap_ == hcap_ && graph_stage_ == stage()) return;
     destroy_graphs();
     if (!body_stream_) cuda_check(cudaStreamCreateWithFlags(&body_stream_, cudaStreamNonBlocking), "cudaStreamCreate");
     if (!chunk_event_) cuda_check(cudaEventCreateWithFlags(&chunk_event_, cudaEventDisableTiming), "cudaEventCreate");
@@ -2039,6 +2055,7 @@ class System : public SystemBase {
     graph_n_ = n_;
     graph_K_ = K_;
     graph_hcap_ = hcap_;
+    graph_stage_ = stage();
   }
 
   void capture_step(StepGraph& g) {
@@ -3018,7 +3035,7 @@ int sph_autotune(sph_system_t* h, uint32_t steps, sph_tuning* best, double* best
     h->impl->get_tuning(&cur);
     // Small scenes (steps of 110 to 200 us) differ by up to 5 % between two runs of one
     // setting, as much as between most settings: fewer candidates, and the setting in
-    // force is the pick only where it is a tenth faster than all of them.
+    // force is the pick only where it is a twentieth faster than all of them.
     const bool small = h->impl->num_particles() <= 65536;
     std::vector<uint32_t> stages = f32 ? std::vector<uint32_t>{1024, 1536, 2048} : std::vector<uint32_t>{512, 1024, 1536};
     if (f32 && !small) stages.push_back(1792);
@@ -3065,7 +3082,7 @@ int sph_autotune(sph_system_t* h, uint32_t steps, sph_tuning* best, double* best
     const bool timed = std::any_of(cand.begin(), cand.end(), [&](const sph_tuning& c) {
       return c.gather_batch == cur.gather_batch && c.halo_stage == cur.halo_stage;
     });
-    if (!timed) time_candidate(cur, small ? 0.9 : 1.0);
+    if (!timed) time_candidate(cur, small ? 0.95 : 1.0);
     h->impl->set_tuning(pick);
     *best = pick;
     if (best_ms_per_step) *best_ms_per_step = best_t;
