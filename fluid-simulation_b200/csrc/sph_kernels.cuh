@@ -2505,10 +2505,11 @@ __global__ void __launch_bounds__(kBlock, sizeof(R) == 4 ? 5 : 1) k_sweep_accel(
 
 // End of a sweep (one thread): error, sweep count, stop test (iisph.rs:378-393).
 __device__ __forceinline__ void end_sweep(Scalars* sc, double total, int n, int after, double tde, int cap) {
+  const int it = sc->iterations + 1;  // (both loads at once: other blocks wait)
+  const double before = sc->err;
   const double err = n > 0 ? total / (double)n * 100.0 : 0.0;
-  const int it = sc->iterations + 1;
   sc->iterations = it;
-  sc->err_before = sc->err;
+  sc->err_before = before;
   sc->err = err;
   bool stop;
   if (after >= 0) {

@@ -192,8 +192,11 @@ __device__ __forceinline__ float grad_third_close<float>(float rx, float ry, flo
   const float r = r2 * inv;
   asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(t) : "f"(r), "f"(-inv_h), "f"(1.f));  // (1-q)_+
   asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(b) : "f"(t), "f"(2.f), "f"(-1.f));    // (1-2q)_+
-  const float close = fmaf(r, -3.f * inv_h * inv_h, 2.f * inv_h);
-  return t > 2.f / 3.f ? close : fmaf(-b, b, t * t) * inv;
+  float f = fmaf(-b, b, t * t) * inv;
+  // (predicated, which spares the select)
+  asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %1, %2;\n\t@p fma.rn.f32 %0, %3, %4, %5;\n\t}"
+      : "+f"(f) : "f"(t), "f"(2.f / 3.f), "f"(r), "f"(-3.f * inv_h * inv_h), "f"(2.f * inv_h));
+  return f;
 }
 
 // Both W and the gradient factor from one square root.
