@@ -858,13 +858,14 @@ struct OrderQueues {
 // SESPH particles after 500 steps, 187 to 363 neighbors at most: 273, 371 and 405 us for
 // three stiffnesses; 661, 925 and 1052 us when every candidate was fetched through the
 // halo's index and its list kept two bytes at a time in global memory, 472, 606 and
-// 740 us with the test-and-append loop. f64, 64 thousand: a step's update 1396 -> 1270 us.
+// 740 us with the test-and-append loop. f64, three steps of 64 thousand particles in a box:
+// 1396 -> 1270 us.
 //
-// What bounds it: issue (about 216 candidates per particle; 73 % of the issue
+// What bounds it: issue (about 216 candidates per particle; 74 % of the issue
 // slots used, 211 M warp instructions for one million particles at spacing
 // h/2). That scene took 470 us with a test-and-append loop per candidate over
 // 27 hashed buckets, and 78 us more in a kernel of its own for the bank-aware
-// order; in this form 270 us for both.
+// order; in this form 269 us for both.
 template <class R, bool ORDER>
 __global__ void __launch_bounds__(kBlock, 4) k_neighbors_density(
     Scalars* sc, const R4<R>* pos, const uint32_t* start,
